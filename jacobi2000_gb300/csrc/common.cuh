@@ -128,14 +128,19 @@ __device__ __forceinline__ void cp_async_wait_group() {
 // Programmatic dependent launch. A kernel launched with programmatic stream
 // serialization may start (be scheduled, set up shared memory, tensor memory
 // and barriers) while the previous kernel in the stream is still running.
-// JC_PDL_ENTRY lets the next kernel start early, then waits until the previous
-// kernel has completed and its writes are visible; every kernel executes it
+// JC_PDL_ENTRY waits until the previous kernel has completed and its writes
+// are visible, then lets the next kernel start early; every kernel executes it
 // before its first access to memory that other kernels write or read.
 // Without the launch attribute both instructions are no-ops.
+// The wait comes first so that at most one kernel is resident ahead of its
+// turn. Released before the wait, the CTAs of several later kernels sat
+// waiting on the SMs, and a kernel of fewer CTAs than SMs then ran two or
+// three to an SM beside SMs held by idle ones: GEMMs of 128 CTAs back to back
+// took 13.8 us a launch that way and take 6.9 us this way.
 #define JC_PDL_ENTRY                                                      \
     do {                                                                  \
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  \
         asm volatile("griddepcontrol.wait;" ::: "memory");               \
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  \
     } while (0)
 
 // Neumaier compensated accumulator in f64.
