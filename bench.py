@@ -186,7 +186,7 @@ def kernel_work(name: str, B: int, cells: int, D: int, F: int):
     byte = {"bf_attention": R * (3 * D * 2 + D * 2), "bf_embed": N * 12 + R * (4 * D + 2 * D),
             "bf_upsample": R * 32 * 4 + N * (12 + 96), "projection": N * 12 * 4 + N * 12,
             "f32_attention": R * (3 * D * 4 + D * 4), "f32_embed": N * 12 + R * 4 * D,
-            "f32_upsample_concat": R * 32 * 4 + N * (12 + 144), "f32_final_ln": R * D * 8}
+            "f32_upsample_concat": R * 32 * 4 + N * (12 + 144), "f32_ln": R * D * 8, "f32_final_ln": R * D * 8}
     if name in flop:
         return "flop", flop[name]
     if name in byte:

@@ -58,6 +58,15 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// d0 = fma(a0, b0, d0), d1 = fma(a1, b1, d1) in one paired instruction
+// (fma.rn.f32x2: each lane rounds like fmaf).
+__device__ __forceinline__ void fma2_f32(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 d, {%0, %1};\n\t"
+        "fma.rn.f32x2 d, a, b, d;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "+f"(d0), "+f"(d1)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+
 // Index of the instance owning token row r: the last i with inst[i].row0 <= r.
 __device__ __forceinline__ int inst_of_row(const InstDev* inst, int n, int r) {
     int lo = 0, hi = n - 1;

@@ -9,240 +9,313 @@
 namespace jc {
 namespace f32k {
 
-// Per-row context a loader may cache in shared memory in its prologue.
-struct RowCtx {
-    int base;   // first row (token loaders) or cell (cell loaders) of the instance
-    int y, x;   // coordinates inside the instance's grid
-    int w, h;   // grid width and height
-};
-
 // ---------------------------------------------------------------------------
-// A-operand loaders of the tiled GEMM. `prologue` runs once per CTA for its
-// BM rows; `load4(r, k, ctx)` returns A[r][k..k+3] (zeros outside the
-// matrix); K and the loaders' channel counts are multiples of 4.
+// A-operand loaders of the tiled GEMM. `prologue` fills the CTA's shared
+// memory with the rows' places in their grids (kCtx);
+// `src(r, k, i, ctx)` is the address of A[r][k..k+3] (null: zeros), where i is
+// the row's index in the tile; K and the loaders' channel counts are
+// multiples of 4. kAligned = false: `src` may be on a 4-byte boundary only
+// (copied by words).
+
+struct NoCtx {};
+struct GridCtx {
+    int base;  // first row (token loader) or cell (cell loader) of the instance
+    int y, x;  // coordinates inside the instance's grid
+    int w, h;  // grid width and height
+};
 
 struct APlain {
+    using Ctx = NoCtx;
+    static constexpr bool kAligned = true, kCtx = false;
     const float* A;
     int lda, R, K;
-    __device__ void prologue(int, int, float*, RowCtx*) const {}
-    __device__ float4 load4(int r, int k, int, const float*, const RowCtx*) const {
-        if (r >= R || k >= K) return make_float4(0.f, 0.f, 0.f, 0.f);
-        return *reinterpret_cast<const float4*>(A + (size_t)r * lda + k);
+    __device__ void prologue(int, int, Ctx*) const {}
+    __device__ const float* src(int r, int k, int, const Ctx*) const {
+        return r < R && k < K ? A + (size_t)r * lda + k : nullptr;
     }
 };
 
-// LayerNorm of X's rows fused into the load (cpu.rs:49-65: two-pass mean and
-// biased variance, eps 1e-5 before the sqrt). K = D.
-struct ALayerNorm {
-    const float* X;
-    const float* gamma;
-    const float* beta;
-    int R, D;
-    __device__ void prologue(int row0, int bm, float* stats, RowCtx*) const {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-        for (int i = warp; i < bm; i += nw) {
-            int r = row0 + i;
-            float mean = 0.f, rstd = 0.f;
+// Patches of the state (cpu.rs:253-269), P a multiple of 4: feature
+// k = c P P + py P + px of a token is a run of P cells of row py.
+struct PatchCtx {
+    const float* cell0;  // channel 0 of the patch's first cell; null past the last row
+    int nx, inst;
+    long long plane;
+};
+struct APatch {
+    using Ctx = PatchCtx;
+    static constexpr bool kAligned = false, kCtx = true;
+    const InstDev* inst;
+    int n_inst, R, K, P;
+    __device__ void prologue(int row0, int bm, Ctx* ctx) const {
+        for (int i = threadIdx.x; i < bm; i += blockDim.x) {
+            const int r = row0 + i;
+            PatchCtx c{nullptr, 0, 0, 0};
             if (r < R) {
-                const float* x = X + (size_t)r * D;
-                float s = 0.f;
-                for (int d = lane; d < D; d += 32) s += x[d];
-                mean = warp_sum(s) / (float)D;
-                float v = 0.f;
-                for (int d = lane; d < D; d += 32) { float t = x[d] - mean; v += t * t; }
-                rstd = 1.0f / sqrtf(warp_sum(v) / (float)D + 1e-5f);
+                c.inst = inst_of_row(inst, n_inst, r);
+                const InstDev& I = inst[c.inst];
+                const int t = r - I.row0;
+                c.nx = I.nx;
+                c.plane = (long long)I.nx * I.ny;
+                c.cell0 = I.state + (size_t)(t / I.tx) * P * I.nx + (size_t)(t % I.tx) * P;
             }
-            if (lane == 0) { stats[2 * i] = mean; stats[2 * i + 1] = rstd; }
+            ctx[i] = c;
         }
     }
-    __device__ float4 load4(int r, int k, int i, const float* stats, const RowCtx*) const {
-        if (r >= R || k >= D) return make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 x = *reinterpret_cast<const float4*>(X + (size_t)r * D + k);
-        float4 g = *reinterpret_cast<const float4*>(gamma + k);
-        float4 b = *reinterpret_cast<const float4*>(beta + k);
-        const float m = stats[2 * i], s = stats[2 * i + 1];
-        return make_float4((x.x - m) * s * g.x + b.x, (x.y - m) * s * g.y + b.y, (x.z - m) * s * g.z + b.z,
-                           (x.w - m) * s * g.w + b.w);
+    __device__ const float* src(int, int k, int i, const Ctx* ctx) const {
+        const PatchCtx& c = ctx[i];
+        if (!c.cell0 || k >= K) return nullptr;
+        const int ch = k / (P * P), py = (k / P) % P, px = k % P;
+        return c.cell0 + ch * c.plane + (size_t)py * c.nx + px;
     }
 };
 
 // 3x3 zero-padded cross-correlation (cpu.rs:171-205) as an implicit GEMM:
 // A[r][tap*C + c] = X[neighbour(r, tap)][c], or 0 outside the grid; K = 9 C.
-// Token variant: rows are tokens of each instance's token grid.
-struct ATokConv3 {
-    const float* X;  // [rows, C]
-    const InstDev* inst;
-    int n_inst, R, C;
-    __device__ void prologue(int row0, int bm, float*, RowCtx* ctx) const {
-        for (int i = threadIdx.x; i < bm; i += blockDim.x) {
-            int r = row0 + i;
-            RowCtx c{0, -100, -100, 0, 0};
-            if (r < R) {
-                const InstDev& I = inst[inst_of_row(inst, n_inst, r)];
-                int t = r - I.row0;
-                c = RowCtx{I.row0, t / I.tx, t % I.tx, I.tx, I.ty};
-            }
-            ctx[i] = c;
-        }
-    }
-    __device__ float4 load4(int r, int k, int i, const float*, const RowCtx* ctx) const {
-        const RowCtx c = ctx[i];
-        int tap = k / C, ch = k - tap * C;
-        int y = c.y + tap / 3 - 1, x = c.x + tap % 3 - 1;
-        if (r >= R || tap >= 9 || y < 0 || x < 0 || y >= c.h || x >= c.w) return make_float4(0.f, 0.f, 0.f, 0.f);
-        return *reinterpret_cast<const float4*>(X + (size_t)(c.base + y * c.w + x) * C + ch);
-    }
-};
-
-// Cell variant: rows are cells of each instance's cell grid, X [cells, C].
-struct ACellConv3 {
+// CELL: rows are cells of each instance's cell grid, else tokens of its token
+// grid; X is [rows, C].
+template <bool CELL>
+struct AConv3 {
+    using Ctx = GridCtx;
+    static constexpr bool kAligned = true, kCtx = true;
     const float* X;
     const InstDev* inst;
     int n_inst, R, C;
-    __device__ void prologue(int row0, int bm, float*, RowCtx* ctx) const {
+    __device__ void prologue(int row0, int bm, Ctx* ctx) const {
         for (int i = threadIdx.x; i < bm; i += blockDim.x) {
-            int r = row0 + i;
-            RowCtx c{0, -100, -100, 0, 0};
+            const int r = row0 + i;
+            GridCtx c{0, -100, -100, 0, 0};
             if (r < R) {
-                const InstDev& I = inst[inst_of_cell(inst, n_inst, r)];
-                int cl = (int)(r - I.cell0);
-                c = RowCtx{(int)I.cell0, cl / I.nx, cl % I.nx, I.nx, I.ny};
+                const InstDev& I = inst[CELL ? inst_of_cell(inst, n_inst, r) : inst_of_row(inst, n_inst, r)];
+                const int base = CELL ? (int)I.cell0 : I.row0, w = CELL ? I.nx : I.tx, h = CELL ? I.ny : I.ty;
+                c = GridCtx{base, (r - base) / w, (r - base) % w, w, h};
             }
             ctx[i] = c;
         }
     }
-    __device__ float4 load4(int r, int k, int i, const float*, const RowCtx* ctx) const {
-        const RowCtx c = ctx[i];
-        int tap = k / C, ch = k - tap * C;
-        int y = c.y + tap / 3 - 1, x = c.x + tap % 3 - 1;
-        if (r >= R || tap >= 9 || y < 0 || x < 0 || y >= c.h || x >= c.w) return make_float4(0.f, 0.f, 0.f, 0.f);
-        return *reinterpret_cast<const float4*>(X + ((size_t)c.base + (size_t)y * c.w + x) * C + ch);
+    __device__ const float* src(int, int k, int i, const Ctx* ctx) const {
+        const GridCtx& c = ctx[i];
+        const int tap = k / C, ch = k - tap * C;
+        const int y = c.y + tap / 3 - 1, x = c.x + tap % 3 - 1;
+        if (tap >= 9 || y < 0 || x < 0 || y >= c.h || x >= c.w) return nullptr;
+        return X + ((size_t)c.base + (size_t)y * c.w + x) * C + ch;
     }
 };
 
-// Epilogues: v already includes the bias.
+// Epilogues: four consecutive outputs n..n+3 of row r, bias included; i is
+// the row's index in the tile and ctx the loader's row contexts.
 struct EStore {
-    float* out; int ld;
-    __device__ void operator()(int r, int n, float v) const { out[(size_t)r * ld + n] = v; }
+    float* out;
+    int ld;
+    template <class Ctx>
+    __device__ void operator()(int r, int n, float4 v, int, const Ctx*) const {
+        *reinterpret_cast<float4*>(out + (size_t)r * ld + n) = v;
+    }
 };
+__device__ __forceinline__ float4 gelu4(float4 v) {
+    return make_float4(gelu_erf(v.x), gelu_erf(v.y), gelu_erf(v.z), gelu_erf(v.w));
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
 struct EGelu {
-    float* out; int ld;
-    __device__ void operator()(int r, int n, float v) const { out[(size_t)r * ld + n] = gelu_erf(v); }
+    float* out;
+    int ld;
+    template <class Ctx>
+    __device__ void operator()(int r, int n, float4 v, int, const Ctx*) const {
+        *reinterpret_cast<float4*>(out + (size_t)r * ld + n) = gelu4(v);
+    }
 };
 struct EResid {  // x += v (cpu.rs:306,312 add_inplace)
-    float* x; int ld;
-    __device__ void operator()(int r, int n, float v) const { x[(size_t)r * ld + n] += v; }
+    float* x;
+    int ld;
+    template <class Ctx>
+    __device__ void operator()(int r, int n, float4 v, int, const Ctx*) const {
+        float4* p = reinterpret_cast<float4*>(x + (size_t)r * ld + n);
+        *p = add4(*p, v);
+    }
 };
 struct EGeluResidFrom {  // out = src + gelu(v) (cpu.rs:327-328)
-    const float* src; float* out; int ld;
-    __device__ void operator()(int r, int n, float v) const {
-        out[(size_t)r * ld + n] = src[(size_t)r * ld + n] + gelu_erf(v);
+    const float* src;
+    float* out;
+    int ld;
+    template <class Ctx>
+    __device__ void operator()(int r, int n, float4 v, int, const Ctx*) const {
+        const size_t o = (size_t)r * ld + n;
+        *reinterpret_cast<float4*>(out + o) = add4(*reinterpret_cast<const float4*>(src + o), gelu4(v));
+    }
+};
+struct EEmbed {  // x = (v + pos) + meta linear (cpu.rs:270-280)
+    const InstDev* inst;
+    const float* Wm;
+    const float* bm;
+    int meta_dim, D;
+    float* x;
+    __device__ void operator()(int r, int n, float4 v, int i, const PatchCtx* ctx) const {
+        const InstDev& I = inst[ctx[i].inst];
+        float4 m = *reinterpret_cast<const float4*>(bm + n);
+        for (int f = 0; f < meta_dim; f++) {
+            const float4 w = *reinterpret_cast<const float4*>(Wm + (size_t)f * D + n);
+            const float t = I.meta[f];
+            m = make_float4(fmaf(t, w.x, m.x), fmaf(t, w.y, m.y), fmaf(t, w.z, m.z), fmaf(t, w.w, m.w));
+        }
+        const float4 p = *reinterpret_cast<const float4*>(I.pos + (size_t)(r - I.row0) * D + n);
+        *reinterpret_cast<float4*>(x + (size_t)r * D + n) = add4(add4(v, p), m);
     }
 };
 
-// out[r][n] = epi(bias[n] + sum_k A[r][k] W[k][n]). W is [K, N] row-major
-// (the checkpoint's Linear layout). 64 x 64 tile per CTA, 4 x 4 per thread,
-// K in steps of 16 through double-buffered shared memory: the next tile is
-// fetched into registers while the current one is multiplied.
-template <int BN, class AL, class EP>
-__global__ void __launch_bounds__(BN * 4)
-gemm_kernel(AL aload, const float* __restrict__ W, const float* __restrict__ bias, int R, int N, int K, EP epi) {
-    constexpr int BM = 64, BK = 16, TM = 4, TN = 4, NT = BN * 4;
-    static_assert((BM / TM) * (BN / TN) == NT, "thread count");
-    __shared__ __align__(16) float As[2][BK][BM + 4];
-    __shared__ __align__(16) float Bs[2][BK][BN + 4];
-    __shared__ float stats[2 * BM];
-    __shared__ RowCtx ctx[BM];
-    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-    const int tid = threadIdx.x;
-    const int tr = (tid / (BN / TN)) * TM, tc = (tid % (BN / TN)) * TN;
-    aload.prologue(row0, BM, stats, ctx);
-    __syncthreads();
-
-    // the accumulator starts from the bias, as cpu.rs:28 does
-    float acc[TM][TN];
-#pragma unroll
-    for (int j = 0; j < TN; j++) {
-        int n = col0 + tc + j;
-        float b0 = n < N ? bias[n] : 0.0f;
-#pragma unroll
-        for (int i = 0; i < TM; i++) acc[i][j] = b0;
+// out[r][n] = epi(bias[n] + sum_k A[r][k] W[k][n]); W is [K, N] row-major
+// (the checkpoint's Linear layout), N a multiple of 4.
+//
+// Arithmetic, the same for every tile shape, so that a row's result does not
+// depend on how many rows the launch has: chain w (w < 4) is the fmaf chain
+// from 0 over the k of the 16-wide groups w, w + 4, ... in order, and the
+// result is (((bias + T0) + T1) + T2) + T3. The four chains run on separate
+// warps and meet in shared memory: a quarter of the serial chain each.
+//
+// A warp owns 8 TM x 16 TN outputs of one chain: lane (lm = lane / 4, ln =
+// lane % 4) the rows lm + 8 i and the columns 16 c + 4 ln... A rows lie
+// K-contiguous with a pitch of KS + 4 floats, so the eight rows that a warp
+// reads as float4s (4 k at once) fall on different banks; W rows lie as they
+// come. Stages of KS = 64 columns arrive by asynchronous copies, NST - 1 of
+// them in flight.
+//
+// What bounds it is shared-memory reads against FMAs: a thread reads
+// TM / 4 + TN float4s per k for 4 TM TN FMAs (two to three wavefronts a
+// read). ncu at 40 K rows, K = 512, N = 128: 4 x 4 a thread keeps the shared
+// pipe at 77% and the FMA pipe at 56% (38 TFLOP/s).
+//   4 x 4 (4 x 8) a thread, 32 x 16 (32 x 32) tiles: launches of few rows,
+//     which cost the length of a CTA's K loop; more CTAs, a shorter loop body;
+//   8 x 8 a thread, 64 x 32 tiles: large launches, half of the shared and of
+//     the L2 reads per FMA (43-45 TFLOP/s; 8 x 4 a thread: 36-40).
+template <int TM_, int TN_, int WM_, int WN_, int NST_>
+struct Tile {
+    static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, NST = NST_, WK = 4;
+    static constexpr int BM = 8 * TM * WM, BN = 16 * TN * WN, KG = 16, KS = KG * WK, NT = 32 * WM * WN * WK;
+    static constexpr int PITCH = KS + 4;
+    static constexpr int kStage = BM * PITCH + KS * BN;  // floats
+    static size_t smem(int K) {  // as many stages as the K loop has, and room for the partial tiles
+        const int stages = (K + KS - 1) / KS;
+        const size_t a = (size_t)(stages < NST ? stages : NST) * kStage, b = (size_t)WK * BM * BN;
+        return (a > b ? a : b) * 4;
     }
+};
 
-    // A: BM*BK/4 float4 per tile; B: BK*BN/4 float4 per tile
-    constexpr int A4 = BM * BK / 4, B4 = BK * BN / 4;
-    float4 ra[(A4 + NT - 1) / NT], rb[(B4 + NT - 1) / NT];
-    auto fetch = [&](int k0) {
+template <class T, class AL, class EP>
+__global__ void __launch_bounds__(T::NT) gemm_kernel(AL aload, const float* __restrict__ W,
+                                                     const float* __restrict__ bias, int R, int N, int K, EP epi) {
+    constexpr int TM = T::TM, TN = T::TN, WN = T::WN, WK = T::WK, NST = T::NST;
+    constexpr int BM = T::BM, BN = T::BN, KS = T::KS, NT = T::NT, PITCH = T::PITCH;
+    extern __shared__ __align__(16) float gsm[];
+    __shared__ typename AL::Ctx ctx[AL::kCtx ? BM : 1];
+    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nst = (K + KS - 1) / KS;
+    constexpr int A4 = BM * KS / 4, B4 = KS * BN / 4;
+    static_assert(A4 % NT == 0 && B4 % NT == 0, "stage copies");
+    auto load_b = [&](int s) {
+        float* dst = gsm + (size_t)(s % NST) * T::kStage + BM * PITCH;
 #pragma unroll
-        for (int q = 0; q < (A4 + NT - 1) / NT; q++) {
-            int e = tid + q * NT;
-            if (e < A4) {
-                int i = e / (BK / 4), kk = (e % (BK / 4)) * 4;
-                ra[q] = aload.load4(row0 + i, k0 + kk, i, stats, ctx);
-            }
+        for (int q = 0; q < B4 / NT; q++) {
+            const int e = tid + q * NT, kk = e / (BN / 4), j = (e % (BN / 4)) * 4;
+            const bool in = s * KS + kk < K && col0 + j < N;
+            cp_async16(dst + kk * BN + j, in ? W + (size_t)(s * KS + kk) * N + col0 + j : W, in);
         }
+    };
+    auto load_a = [&](int s) {
+        float* dst = gsm + (size_t)(s % NST) * T::kStage;
 #pragma unroll
-        for (int q = 0; q < (B4 + NT - 1) / NT; q++) {
-            int e = tid + q * NT;
-            if (e < B4) {
-                int kk = e / (BN / 4), j = (e % (BN / 4)) * 4;
-                int k = k0 + kk, n = col0 + j;
-                rb[q] = (k < K && n < N) ? *reinterpret_cast<const float4*>(W + (size_t)k * N + n)
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < A4 / NT; u++) {
+            const int e = tid + u * NT, i = e / (KS / 4), kk = (e % (KS / 4)) * 4;
+            const float* p = aload.src(row0 + i, s * KS + kk, i, ctx);
+            float* q = dst + i * PITCH + kk;
+            if (AL::kAligned || (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+                cp_async16(q, p ? p : W, p != nullptr);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++) cp_async4(q + c, p + c, true);
             }
         }
     };
-    auto stash = [&](int buf) {
+    // the weights never change: their first stages start before the previous
+    // kernel has finished
 #pragma unroll
-        for (int q = 0; q < (A4 + NT - 1) / NT; q++) {
-            int e = tid + q * NT;
-            if (e < A4) {
-                int i = e / (BK / 4), kk = (e % (BK / 4)) * 4;
-                As[buf][kk + 0][i] = ra[q].x;
-                As[buf][kk + 1][i] = ra[q].y;
-                As[buf][kk + 2][i] = ra[q].z;
-                As[buf][kk + 3][i] = ra[q].w;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < (B4 + NT - 1) / NT; q++) {
-            int e = tid + q * NT;
-            if (e < B4) {
-                int kk = e / (BN / 4), j = (e % (BN / 4)) * 4;
-                *reinterpret_cast<float4*>(&Bs[buf][kk][j]) = rb[q];
-            }
-        }
-    };
-
-    const int nk = (K + BK - 1) / BK;
-    fetch(0);
-    stash(0);
-    __syncthreads();
-    for (int kt = 0; kt < nk; kt++) {
-        const int buf = kt & 1;
-        if (kt + 1 < nk) fetch((kt + 1) * BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            float4 a = *reinterpret_cast<const float4*>(&As[buf][kk][tr]);
-            float4 b = *reinterpret_cast<const float4*>(&Bs[buf][kk][tc]);
-            float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < TM; i++)
-#pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        if (kt + 1 < nk) stash(buf ^ 1);
+    for (int s = 0; s < NST - 1; s++)
+        if (s < nst) load_b(s);
+    JC_PDL_ENTRY;
+    if (AL::kCtx) {
+        aload.prologue(row0, BM, ctx);
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < TM; i++) {
-        int r = row0 + tr + i;
-        if (r >= R) continue;
+    for (int s = 0; s < NST - 1; s++) {
+        if (s < nst) load_a(s);
+        cp_async_commit();
+    }
+    const int wk = warp % WK, wt = warp / WK, wn = wt % WN, wm = wt / WN;
+    const int lm = lane >> 2, ln = lane & 3;
+    float acc[TM][4 * TN];
 #pragma unroll
-        for (int j = 0; j < TN; j++) {
-            int n = col0 + tc + j;
-            if (n < N) epi(r, n, acc[i][j]);
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int c = 0; c < 4 * TN; c++) acc[i][c] = 0.f;
+    for (int s = 0; s < nst; s++) {
+        cp_async_wait_group<NST - 2>();
+        const float* As = gsm + (size_t)(s % NST) * T::kStage;
+        __syncthreads();
+        if (s + NST - 1 < nst) {
+            load_b(s + NST - 1);
+            load_a(s + NST - 1);
         }
+        cp_async_commit();
+        const float* a = As + (wm * 8 * TM + lm) * PITCH + wk * T::KG;
+        const float* b = As + BM * PITCH + wk * T::KG * BN + wn * 16 * TN + 4 * ln;
+        if (s * KS + wk * T::KG < K) {
+            // unrolled twice only: most launches run the loop a few times, and
+            // its instructions come from memory then (a 128 x 128 rollout's
+            // ticks: 262 us unrolled four times, 245 us twice)
+#pragma unroll 2
+            for (int kk = 0; kk < T::KG; kk += 4) {
+                float4 av[TM];
+#pragma unroll
+                for (int i = 0; i < TM; i++) av[i] = *reinterpret_cast<const float4*>(a + i * 8 * PITCH + kk);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float4 bv[TN];
+#pragma unroll
+                    for (int c = 0; c < TN; c++) bv[c] = *reinterpret_cast<const float4*>(b + (kk + q) * BN + 16 * c);
+#pragma unroll
+                    for (int i = 0; i < TM; i++) {
+                        const float x = q == 0 ? av[i].x : q == 1 ? av[i].y : q == 2 ? av[i].z : av[i].w;
+#pragma unroll
+                        for (int c = 0; c < TN; c++) {
+                            fma2_f32(acc[i][4 * c], acc[i][4 * c + 1], x, x, bv[c].x, bv[c].y);
+                            fma2_f32(acc[i][4 * c + 2], acc[i][4 * c + 3], x, x, bv[c].z, bv[c].w);
+                        }
+                    }
+                }
+            }
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();  // every warp is done with the stages: they take the four partial tiles
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int c = 0; c < TN; c++)
+            *reinterpret_cast<float4*>(gsm + ((size_t)wk * BM + wm * 8 * TM + lm + 8 * i) * BN + wn * 16 * TN + 16 * c +
+                                       4 * ln) =
+                make_float4(acc[i][4 * c], acc[i][4 * c + 1], acc[i][4 * c + 2], acc[i][4 * c + 3]);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < BM * BN / 4 / NT; u++) {
+        const int e = tid + u * NT, i = e / (BN / 4), j = (e % (BN / 4)) * 4, r = row0 + i;
+        if (r >= R || col0 + j >= N) continue;
+        float4 v = *reinterpret_cast<const float4*>(bias + col0 + j);
+#pragma unroll
+        for (int w = 0; w < WK; w++)
+            v = add4(v, *reinterpret_cast<const float4*>(gsm + ((size_t)w * BM + i) * BN + j));
+        epi(r, col0 + j, v, i, ctx);
     }
 }
 

@@ -101,6 +101,7 @@ constexpr int kEmbedTok = 16;
 __global__ void embed_kernel(Dims d, const float* __restrict__ We, const float* __restrict__ be,
                              const float* __restrict__ Wm, const float* __restrict__ bm, const InstDev* inst,
                              int n_inst, int R, float* __restrict__ x) {
+    JC_PDL_ENTRY;
     extern __shared__ float patch[];  // [kEmbedTok][C*P*P]
     __shared__ int rinst[kEmbedTok];
     const int pd = d.C * d.P * d.P;
@@ -152,8 +153,69 @@ __device__ __forceinline__ int candidate_row(const Dims& d, const InstDev& I, in
     return I.row0 + ky * I.tx + kx;
 }
 
+// Radius-1 stencil (any dilation), head widths of 4 LPH floats: LPH lanes per
+// (row, head), each with four of its features, so a warp reads whole
+// key and value rows as float4s and all 18 of a thread's loads are in flight
+// together. The nine scores' lane sums run interleaved (log2 LPH shuffles
+// each, where a warp per (row, head) takes five of a dependent chain).
+// 24 grids of 60-128 (up to 10 K rows, 4 heads of 32): 77 -> 14 us a launch.
+template <int LPH>
+__global__ void __launch_bounds__(256) attention_r1_kernel(Dims d, const float* __restrict__ qkv, const InstDev* inst,
+                                                           int n_inst, int R, float* __restrict__ out) {
+    JC_PDL_ENTRY;
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long unit = gid / LPH;
+    const int l = (int)(gid % LPH);
+    const bool live = unit < (long long)R * d.heads;
+    const int row = live ? (int)(unit / d.heads) : R - 1, head = live ? (int)(unit % d.heads) : 0;
+    const int D3 = 3 * d.D;
+    const InstDev& I = inst[inst_of_row(inst, n_inst, row)];
+    const int tx = I.tx, ty = I.ty, t = row - I.row0, qy = t / tx, qx = t % tx;
+    const float scale = 1.0f / sqrtf((float)(4 * LPH));
+    const float* at = qkv + (size_t)row * D3 + head * 4 * LPH + 4 * l;
+    const float4 q = *reinterpret_cast<const float4*>(at);
+    float4 k[9], v[9];
+    bool in[9];
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+        const int dy = (j / 3 - 1) * d.dilation, dx = (j % 3 - 1) * d.dilation;
+        in[j] = qy + dy >= 0 && qx + dx >= 0 && qy + dy < ty && qx + dx < tx;
+        const float* p = at + (in[j] ? (long long)(dy * tx + dx) * D3 : 0);
+        k[j] = *reinterpret_cast<const float4*>(p + d.D);
+        v[j] = *reinterpret_cast<const float4*>(p + 2 * d.D);
+    }
+    float s[9];
+#pragma unroll
+    for (int j = 0; j < 9; j++) s[j] = fmaf(q.w, k[j].w, fmaf(q.z, k[j].z, fmaf(q.y, k[j].y, q.x * k[j].x)));
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < 9; j++) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    float smax = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+        s[j] *= scale;
+        if (in[j]) smax = fmaxf(smax, s[j]);
+    }
+    float denom = 0.f;
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+        s[j] = in[j] ? expf(s[j] - smax) : 0.f;
+        if (in[j]) denom += s[j];
+    }
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+        if (s[j] == 0.f) continue;
+        const float wn = s[j] / denom;
+        o = make_float4(fmaf(wn, v[j].x, o.x), fmaf(wn, v[j].y, o.y), fmaf(wn, v[j].z, o.z), fmaf(wn, v[j].w, o.w));
+    }
+    if (live) *reinterpret_cast<float4*>(out + (size_t)row * d.D + head * 4 * LPH + 4 * l) = o;
+}
+
 __global__ void attention_kernel(Dims d, const float* __restrict__ qkv, const InstDev* inst, int n_inst, int R,
                                  float* __restrict__ out) {
+    JC_PDL_ENTRY;
     const int lane = threadIdx.x & 31;
     const int wg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int row = wg / d.heads, head = wg % d.heads;
@@ -207,55 +269,110 @@ __global__ void attention_kernel(Dims d, const float* __restrict__ qkv, const In
     if (lane + 32 < hd) o[lane + 32] = o1;
 }
 
-// Row LayerNorm (cpu.rs:49-65), one warp per row.
+// Row LayerNorm (cpu.rs:49-65: two-pass mean and biased variance, eps 1e-5
+// before the sqrt), one warp per row: lane l takes the float4s l, l + 32, ...
+// of the row, held in registers between the passes up to 512 values. Its own
+// kernel, not part of the GEMMs' loads: normalized again by every column tile,
+// the rows cost a 40 K x 512 x 128 GEMM 282 us where it takes 145 us without,
+// and a GEMM of 64 rows 5.8 us against 2.7.
+constexpr int kLnRows = 8;  // rows (warps) per CTA
+
+template <int NV>
+__device__ __forceinline__ void ln_row(const float4* x, const float4* g, const float4* b, int nq, int D, float4* y) {
+    const int lane = threadIdx.x & 31;
+    float4 v[NV];
+#pragma unroll
+    for (int j = 0; j < NV; j++) v[j] = lane + 32 * j < nq ? x[lane + 32 * j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; j++) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+    const float mean = warp_sum(s) / (float)D;
+    s = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; j++)
+        if (lane + 32 * j < nq) {
+            const float a = v[j].x - mean, bb = v[j].y - mean, c = v[j].z - mean, d = v[j].w - mean;
+            s += fmaf(a, a, bb * bb) + fmaf(c, c, d * d);
+        }
+    const float rstd = 1.0f / sqrtf(warp_sum(s) / (float)D + 1e-5f);
+#pragma unroll
+    for (int j = 0; j < NV; j++) {
+        const int q = lane + 32 * j;
+        if (q >= nq) continue;
+        const float4 gg = g[q], be = b[q];
+        y[q] = make_float4(fmaf((v[j].x - mean) * rstd, gg.x, be.x), fmaf((v[j].y - mean) * rstd, gg.y, be.y),
+                           fmaf((v[j].z - mean) * rstd, gg.z, be.z), fmaf((v[j].w - mean) * rstd, gg.w, be.w));
+    }
+}
+
 __global__ void layernorm_kernel(const float* __restrict__ x, const float* __restrict__ g,
                                  const float* __restrict__ b, int R, int D, float* __restrict__ y) {
-    const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    JC_PDL_ENTRY;
+    const int row = blockIdx.x * kLnRows + (threadIdx.x >> 5);
     if (row >= R) return;
-    const float* xr = x + (size_t)row * D;
-    float s = 0.f;
-    for (int i = lane; i < D; i += 32) s += xr[i];
-    float mean = warp_sum(s) / (float)D;
-    float v = 0.f;
-    for (int i = lane; i < D; i += 32) { float t = xr[i] - mean; v += t * t; }
-    float rstd = 1.0f / sqrtf(warp_sum(v) / (float)D + 1e-5f);
-    for (int i = lane; i < D; i += 32) y[(size_t)row * D + i] = (xr[i] - mean) * rstd * g[i] + b[i];
+    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * D);
+    float4* yr = reinterpret_cast<float4*>(y + (size_t)row * D);
+    const float4 *g4 = reinterpret_cast<const float4*>(g), *b4 = reinterpret_cast<const float4*>(b);
+    const int nq = D / 4;
+    if (nq <= 32) ln_row<1>(xr, g4, b4, nq, D, yr);
+    else if (nq <= 128) ln_row<4>(xr, g4, b4, nq, D, yr);
+    else {
+        const int lane = threadIdx.x & 31;
+        float s = 0.f;
+        for (int q = lane; q < nq; q += 32) s += (xr[q].x + xr[q].y) + (xr[q].z + xr[q].w);
+        const float mean = warp_sum(s) / (float)D;
+        s = 0.f;
+        for (int q = lane; q < nq; q += 32) {
+            const float a = xr[q].x - mean, bb = xr[q].y - mean, c = xr[q].z - mean, d = xr[q].w - mean;
+            s += fmaf(a, a, bb * bb) + fmaf(c, c, d * d);
+        }
+        const float rstd = 1.0f / sqrtf(warp_sum(s) / (float)D + 1e-5f);
+        for (int q = lane; q < nq; q += 32) {
+            const float4 v = xr[q], gg = g4[q], be = b4[q];
+            yr[q] = make_float4(fmaf((v.x - mean) * rstd, gg.x, be.x), fmaf((v.y - mean) * rstd, gg.y, be.y),
+                                fmaf((v.z - mean) * rstd, gg.z, be.z), fmaf((v.w - mean) * rstd, gg.w, be.w));
+        }
+    }
 }
 
 // Upsample z0 (token level, [rows, HD]) by P along y then x with edge
 // replicate and weights (i + 0.5)/P (cpu.rs:211-245), and concatenate the
-// state channels (cpu.rs:339-342): zc [cells, kZcStride], one thread per cell.
+// state channels (cpu.rs:339-342): zc [cells, kZcStride]. One thread per four
+// consecutive channels of a cell, so that a warp's stores are one run of
+// memory (a thread per cell wrote 16 bytes every 144).
 __global__ void upsample_concat_kernel(Dims d, const float* __restrict__ z0, const InstDev* inst, int n_inst,
                                        long long NC, float* __restrict__ zc) {
-    long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (cell >= NC) return;
+    JC_PDL_ENTRY;
+    constexpr int kQ = kZcStride / 4;
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long cell = e / kQ;
+    const int q = (int)(e - cell * kQ);
+    if (cell >= NC || q > d.HD / 4) return;
     const InstDev& I = inst[inst_of_cell(inst, n_inst, cell)];
-    long long cl = cell - I.cell0;
-    int y = (int)(cl / I.nx), x = (int)(cl % I.nx);
-    int yt = y / d.P, iy = y % d.P, xt = x / d.P, ix = x % d.P;
-    int yt2 = min(yt + 1, I.ty - 1), xt2 = min(xt + 1, I.tx - 1);
-    float wy = ((float)iy + 0.5f) / (float)d.P, wx = ((float)ix + 0.5f) / (float)d.P;
-    const float4* a = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt * I.tx + xt) * d.HD);
-    const float4* b = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt * I.tx + xt2) * d.HD);
-    const float4* c = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt2 * I.tx + xt) * d.HD);
-    const float4* e = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt2 * I.tx + xt2) * d.HD);
-    float4* o = reinterpret_cast<float4*>(zc + (size_t)cell * kZcStride);
-    const float uy = 1.0f - wy, ux = 1.0f - wx;
-#pragma unroll 4
-    for (int q = 0; q < d.HD / 4; q++) {
-        float4 A = a[q], B = b[q], Cc = c[q], E = e[q], r;
+    const int cl = (int)(cell - I.cell0);
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (q < d.HD / 4) {
+        const int y = cl / I.nx, x = cl % I.nx;
+        const int yt = y / d.P, iy = y % d.P, xt = x / d.P, ix = x % d.P;
+        const int yt2 = min(yt + 1, I.ty - 1), xt2 = min(xt + 1, I.tx - 1);
+        const float wy = ((float)iy + 0.5f) / (float)d.P, wx = ((float)ix + 0.5f) / (float)d.P;
+        const float4 A = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt * I.tx + xt) * d.HD)[q];
+        const float4 B = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt * I.tx + xt2) * d.HD)[q];
+        const float4 C = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt2 * I.tx + xt) * d.HD)[q];
+        const float4 E = reinterpret_cast<const float4*>(z0 + (size_t)(I.row0 + yt2 * I.tx + xt2) * d.HD)[q];
+        const float uy = 1.0f - wy, ux = 1.0f - wx;
         // upsample_y at columns xt and xt2, then upsample_x
-        r.x = (A.x * uy + Cc.x * wy) * ux + (B.x * uy + E.x * wy) * wx;
-        r.y = (A.y * uy + Cc.y * wy) * ux + (B.y * uy + E.y * wy) * wx;
-        r.z = (A.z * uy + Cc.z * wy) * ux + (B.z * uy + E.z * wy) * wx;
-        r.w = (A.w * uy + Cc.w * wy) * ux + (B.w * uy + E.w * wy) * wx;
-        o[q] = r;
+        r.x = (A.x * uy + C.x * wy) * ux + (B.x * uy + E.x * wy) * wx;
+        r.y = (A.y * uy + C.y * wy) * ux + (B.y * uy + E.y * wy) * wx;
+        r.z = (A.z * uy + C.z * wy) * ux + (B.z * uy + E.z * wy) * wx;
+        r.w = (A.w * uy + C.w * wy) * ux + (B.w * uy + E.w * wy) * wx;
+    } else {
+        const size_t plane = (size_t)I.nx * I.ny;
+        float tail[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int ch = 0; ch < d.C; ch++) tail[ch] = I.state[ch * plane + cl];
+        r = make_float4(tail[0], tail[1], tail[2], tail[3]);
     }
-    size_t plane = (size_t)I.nx * I.ny;
-    float tail[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int ch = 0; ch < d.C; ch++) tail[ch] = I.state[ch * plane + cl];
-    o[d.HD / 4] = make_float4(tail[0], tail[1], tail[2], tail[3]);
+    reinterpret_cast<float4*>(zc)[cell * kQ + q] = r;
 }
 
 // head.conv2 (3x3, HD -> C, zero padding; cpu.rs:171-205, 347-348) and the
@@ -653,55 +770,104 @@ projection_kernel(Dims d, const InstDev* inst, ProjSlot* slots, int init, int ca
 
 }  // namespace f32k
 
-template <int BN, class AL, class EP>
+template <class T, class AL, class EP>
+static void gemm_tile(const char* name, const AL& a, const float* W, const float* b, int R, int N, int K, const EP& e,
+                      cudaStream_t s) {
+    static std::atomic<unsigned long long> attr{0};
+    set_smem_per_device(f32k::gemm_kernel<T, AL, EP>, (int)T::smem(1 << 20), attr);
+    const dim3 grid((N + T::BN - 1) / T::BN, (R + T::BM - 1) / T::BM);
+    cuda_check_attr(launch_pdl(f32k::gemm_kernel<T, AL, EP>, grid, dim3(T::NT), T::smem(K), s, 1u, a, W, b, R, N, K, e));
+    check_launch(name);
+}
+
+// The tile by the CTAs it gives: the smallest tiles while they find an SM each
+// (152), the middle ones while there are at most four to an SM, then the large
+// ones. Back to back launches, us (32x16 | 32x32 | 64x32 tiles): R = 256, N =
+// 128, K = 512: 5.0 | 6.9 | 9.7; R = 1024, the same: 6.9 | 7.0 | 9.9; R = 2048,
+// N = 512, K = 128: 10.7 | 9.8 | 10.4; R = 160 K, N = 128, K = 512: 32x32 486,
+// 64x32 461 (45 TFLOP/s).
+template <class AL, class EP>
 static void gemm(const char* name, const AL& a, const float* W, const float* b, int R, int N, int K, const EP& e,
                  cudaStream_t s) {
+    using namespace f32k;
     KScope k(name, s);
-    dim3 grid((N + BN - 1) / BN, (R + 63) / 64);
-    f32k::gemm_kernel<BN, AL, EP><<<grid, BN * 4, 0, s>>>(a, W, b, R, N, K, e);
+    constexpr long long kSms = 152;
+    const long long rows32 = (R + 31) / 32;
+    if (rows32 * ((N + 15) / 16) <= kSms) gemm_tile<Tile<4, 1, 1, 1, 4>>(name, a, W, b, R, N, K, e, s);
+    else if (rows32 * ((N + 31) / 32) <= 4 * kSms) gemm_tile<Tile<4, 2, 1, 1, 3>>(name, a, W, b, R, N, K, e, s);
+    else gemm_tile<Tile<8, 2, 1, 1, 3>>(name, a, W, b, R, N, K, e, s);
+}
+
+static void layernorm(const char* name, const float* x, const float* g, const float* b, int R, int D, float* y,
+                      cudaStream_t s) {
+    KScope k(name, s);
+    cuda_check_attr(launch_pdl(f32k::layernorm_kernel, dim3((unsigned)((R + f32k::kLnRows - 1) / f32k::kLnRows)),
+                               dim3(f32k::kLnRows * 32), 0, s, 1u, x, g, b, R, D, y));
     check_launch(name);
+}
+
+static void attention(const Dims& d, const float* qkv, const InstDev* inst, int n, int R, float* out, cudaStream_t s) {
+    using namespace f32k;
+    KScope k("f32_attention", s);
+    const int hd = d.D / d.heads;
+    const bool r1 = d.mask_kind == 1 && d.radius == 1;
+    auto r1_launch = [&](auto kernel) {
+        const long long threads = (long long)R * d.D / 4;
+        cuda_check_attr(launch_pdl(kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, s, 1u, d, qkv, inst, n,
+                                   R, out));
+    };
+    if (r1 && hd == 8) r1_launch(attention_r1_kernel<2>);
+    else if (r1 && hd == 16) r1_launch(attention_r1_kernel<4>);
+    else if (r1 && hd == 32) r1_launch(attention_r1_kernel<8>);
+    else if (r1 && hd == 64) r1_launch(attention_r1_kernel<16>);
+    else {
+        const long long warps = (long long)R * d.heads;
+        cuda_check_attr(launch_pdl(attention_kernel, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, s, 1u, d, qkv, inst,
+                                   n, R, out));
+    }
+    check_launch("attention");
 }
 
 void forward_f32(const Dims& d, const WeightsF32& w, const Pack& p, int mode, cudaStream_t s) {
     using namespace f32k;
     const int R = p.R, D = d.D, n = p.n_inst;
-    {
+    const InstDev* inst = p.inst;
+    if (R == 0) return;
+    const int pd = d.C * d.P * d.P;
+    if (d.P % 4 == 0) {
+        gemm("f32_embed", APatch{inst, n, R, pd, d.P}, w.embed_w, w.embed_b, R, D, pd,
+             EEmbed{inst, w.meta_w, w.meta_b, d.meta_dim, D, p.x}, s);
+    } else {
         KScope k("f32_embed", s);
-        int pd = d.C * d.P * d.P;
-        embed_kernel<<<(R + kEmbedTok - 1) / kEmbedTok, 128, kEmbedTok * pd * sizeof(float), s>>>(
-            d, w.embed_w, w.embed_b, w.meta_w, w.meta_b, p.inst, n, R, p.x);
+        cuda_check_attr(launch_pdl(embed_kernel, dim3((R + kEmbedTok - 1) / kEmbedTok), dim3(128),
+                                   kEmbedTok * pd * sizeof(float), s, 1u, d, w.embed_w, w.embed_b, w.meta_w, w.meta_b, inst,
+                                   n, R, p.x));
         check_launch("embed");
     }
     for (int l = 0; l < d.L; l++) {
         const auto& B = w.blk[l];
-        gemm<64>("f32_ln_qkv", ALayerNorm{p.x, B.n1g, B.n1b, R, D}, B.wqkv, B.bqkv, R, 3 * D, D,
-                 EStore{p.qkv, 3 * D}, s);
-        {
-            KScope k("f32_attention", s);
-            long long warps = (long long)R * d.heads;
-            attention_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(d, p.qkv, p.inst, n, R, p.attn);
-            check_launch("attention");
-        }
-        gemm<64>("f32_proj", APlain{p.attn, D, R, D}, B.wp, B.bp, R, D, D, EResid{p.x, D}, s);
-        gemm<64>("f32_ln_ff1", ALayerNorm{p.x, B.n2g, B.n2b, R, D}, B.w1, B.b1, R, d.F, D, EGelu{p.ff1, d.F}, s);
-        gemm<64>("f32_ff2", APlain{p.ff1, d.F, R, d.F}, B.w2, B.b2, R, D, d.F, EResid{p.x, D}, s);
+        layernorm("f32_ln", p.x, B.n1g, B.n1b, R, D, p.xn, s);
+        gemm("f32_ln_qkv", APlain{p.xn, D, R, D}, B.wqkv, B.bqkv, R, 3 * D, D, EStore{p.qkv, 3 * D}, s);
+        attention(d, p.qkv, inst, n, R, p.attn, s);
+        gemm("f32_proj", APlain{p.attn, D, R, D}, B.wp, B.bp, R, D, D, EResid{p.x, D}, s);
+        layernorm("f32_ln", p.x, B.n2g, B.n2b, R, D, p.xn, s);
+        gemm("f32_ln_ff1", APlain{p.xn, D, R, D}, B.w1, B.b1, R, d.F, D, EGelu{p.ff1, d.F}, s);
+        gemm("f32_ff2", APlain{p.ff1, d.F, R, d.F}, B.w2, B.b2, R, D, d.F, EResid{p.x, D}, s);
     }
-    {
-        KScope k("f32_final_ln", s);
-        layernorm_kernel<<<(R + 7) / 8, 256, 0, s>>>(p.x, w.norm_g, w.norm_b, R, D, p.xn);
-        check_launch("layernorm");
-    }
-    gemm<64>("f32_token_mix", ATokConv3{p.xn, p.inst, n, R, D}, w.tm_w, w.tm_b, R, D, 9 * D,
-             EGeluResidFrom{p.xn, p.t1, D}, s);
-    gemm<32>("f32_to_cells", APlain{p.t1, D, R, D}, w.tc_w, w.tc_b, R, d.HD, D, EStore{p.z0, d.HD}, s);
+    layernorm("f32_final_ln", p.x, w.norm_g, w.norm_b, R, D, p.xn, s);
+    gemm("f32_token_mix", AConv3<false>{p.xn, inst, n, R, D}, w.tm_w, w.tm_b, R, D, 9 * D, EGeluResidFrom{p.xn, p.t1, D},
+         s);
+    gemm("f32_to_cells", APlain{p.t1, D, R, D}, w.tc_w, w.tc_b, R, d.HD, D, EStore{p.z0, d.HD}, s);
     const long long NC = p.NC;
     {
         KScope k("f32_upsample_concat", s);
-        upsample_concat_kernel<<<(unsigned)((NC + 255) / 256), 256, 0, s>>>(d, p.z0, p.inst, n, NC, p.zc);
+        const long long chunks = NC * (kZcStride / 4);
+        cuda_check_attr(launch_pdl(upsample_concat_kernel, dim3((unsigned)((chunks + 255) / 256)), dim3(256), 0, s, 1u, d,
+                                   (const float*)p.z0, inst, n, NC, p.zc));
         check_launch("upsample_concat");
     }
-    gemm<32>("f32_conv1", ACellConv3{p.zc, p.inst, n, (int)NC, kZcStride}, w.c1_w, w.c1_b, (int)NC, d.HD,
-             9 * kZcStride, EGelu{p.c1, d.HD}, s);
+    gemm("f32_conv1", AConv3<true>{p.zc, inst, n, (int)NC, kZcStride}, w.c1_w, w.c1_b, (int)NC, d.HD, 9 * kZcStride,
+         EGelu{p.c1, d.HD}, s);
     conv2_step(d, p.c1, w, p, mode, "f32_conv2_step", s);
 }
 
