@@ -119,6 +119,14 @@ static CUtensorMap store_map(const void* base, int cols, int rows, int ld, bool 
                     CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// Rows of a [rows, cols] f32 matrix, moved as 16-column x 128-row boxes.
+static CUtensorMap resid_map(const void* base, int cols, int rows) {
+    uint64_t dims[2] = {(uint64_t)cols, (uint64_t)(rows > 0 ? rows : 1)};
+    uint64_t strides[1] = {(uint64_t)cols * 4};
+    uint32_t box[2] = {16, 128};
+    return make_map(base, 2, dims, strides, box, CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
+}
+
 // One instance's [ny, nx, C] channel-last grid (bf16, or f32 when f32),
 // stored as 128-byte x 8 x 16 boxes (one 8 x 16 conv tile, 128 bytes of
 // channels) from 128-byte swizzled shared memory; positions outside the grid
@@ -988,7 +996,7 @@ __device__ __forceinline__ void load_xrows(const float* __restrict__ x, int m0, 
     }
 }
 
-template <int SPL, bool FULL, bool PRE = false, bool LNS = false>  // FULL: every lane owns SPL slots (D = 128 SPL)
+template <int SPL, bool FULL, bool PRE = false>  // FULL: every lane owns SPL slots (D = 128 SPL)
 __device__ __forceinline__ void rows_resid_ln_t(const float* tile, int D, int m0, int R, const float* __restrict__ bias,
                                 float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ b,
                                 bf16* __restrict__ ln, int warp, int nwarps, int nrows, const XRows* xin = nullptr) {
@@ -1091,25 +1099,16 @@ __device__ __forceinline__ void rows_resid_ln_t(const float* tile, int D, int m0
                               ln1(v[k][j].y, mean[k], rstd, gg[j].y, be[j].y),
                               ln1(v[k][j].z, mean[k], rstd, gg[j].z, be[j].z),
                               ln1(v[k][j].w, mean[k], rstd, gg[j].w, be[j].w)};
-                if (LNS)  // the MMA A tile in shared memory: [D/8][128][8] core matrices
-                    BfVec<4>::store(reinterpret_cast<bf16*>(reinterpret_cast<uint8_t*>(ln) + (size_t)(q >> 1) * 2048 +
-                                                            (size_t)(r0 + k) * 16 + (q & 1) * 8), o);
-                else
-                    BfVec<4>::store(ln + (size_t)row * D + 4 * q, o);
+                BfVec<4>::store(ln + (size_t)row * D + 4 * q, o);
             }
         }
     }
 }
 
-// LNS: `ln` is the shared-memory A tile of an MMA (D = 128 only).
-template <bool PRE = false, bool LNS = false>
+template <bool PRE = false>
 __device__ __forceinline__ void rows_resid_ln_any(const float* tile, int D, int m0, int R, const float* bias, float* x,
                                   const float* g, const float* b, bf16* ln, int warp, int nwarps, int nrows = 128,
                                   const XRows* xin = nullptr) {
-    if (LNS) {
-        if (D == 128) rows_resid_ln_t<1, true, PRE, true>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows, xin);
-        return;
-    }
     if (D == 256) rows_resid_ln_t<2, true>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows);
     else if (D == 128) rows_resid_ln_t<1, true, PRE>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows, xin);
     else if (D > 128) rows_resid_ln_t<2, false>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows);
@@ -1308,35 +1307,22 @@ constexpr int kLnMaxD = 128;  // widest row the row-per-thread LayerNorm serves
 // NC-independent K slices of 16, so every chunk width gives the same bits.
 // The residual + LayerNorm epilogue stages O through shared memory and runs
 // one warp per row.
-//
-// PROJ: the block's output projection first (cpu.rs:300-305: x += attn @ Wp
-// + bp, then LayerNorm2): the tile's attention rows (TMA, tmP) and Wp (one
-// bulk copy into the weight buffers, which need D * D * 2 bytes: dim 128
-// with 64-column chunks) give P in the O accumulator; its residual +
-// LayerNorm epilogue is the one above (the arithmetic every residual +
-// LayerNorm here shares, so the result equals the separate projection
-// kernel's bit for bit), with P staged behind sA and the LN2 rows written
-// straight into sA as the MLP's A operand (no global round trip). The
-// tile's rows of x and ln are only touched by this CTA.
 constexpr int kMlpSerialThreads = 256;
 
-template <bool PROJ>
 __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(const __grid_constant__ CUtensorMap tmA,
                                                              const bf16* __restrict__ W1, const bf16* __restrict__ W2,
                                                              const float* __restrict__ b1,
                                                              const float* __restrict__ b2, int D, int F, int NC, int R,
                                                              float* __restrict__ x, const float* __restrict__ g,
                                                              const float* __restrict__ b, bf16* __restrict__ ln,
-                                                             int* err, const __grid_constant__ CUtensorMap tmP,
-                                                             const bf16* __restrict__ Wp, const float* __restrict__ bp,
-                                                             const float* __restrict__ g2, const float* __restrict__ be2) {
+                                                             int* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sA = smem;                           // [D/8][128][8]
     uint8_t* sB1 = sA + (size_t)D * 256;          // [D/8][NC][8]
     uint8_t* sB2 = sB1 + (size_t)D * NC * 2;      // [NC/8][D][8]
     uint8_t* sH = sB2 + (size_t)D * NC * 2;       // [NC/8][128][8]
     __shared__ __align__(16) float sb1[1024];
-    __shared__ uint64_t bar_a, bar_w1, bar_w2, bar_s, bar_o, bar_p, bar_pm;
+    __shared__ uint64_t bar_a, bar_w1, bar_w2, bar_s, bar_o;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1345,8 +1331,6 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
     const uint32_t ncols = D <= 128 ? 256 : 512;
     const uint32_t s_col = D <= 128 ? 128 : 256;  // O in [0, D), S in [s_col, s_col + NC)
     if (threadIdx.x == 0) {
-        tc::mbar_init(&bar_p, 1);
-        tc::mbar_init(&bar_pm, 1);
         tc::mbar_init(&bar_a, 1);
         tc::mbar_init(&bar_w1, 1);
         tc::mbar_init(&bar_w2, 1);
@@ -1367,41 +1351,6 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
     tc::tc_fence_after();
     const uint32_t tO = tmem_base, tS = tmem_base + s_col;
     const uint32_t a0 = tc::smem_u32(sA), w1s = tc::smem_u32(sB1), w2s = tc::smem_u32(sB2), hs = tc::smem_u32(sH);
-    if constexpr (PROJ) {
-        // P = attn @ Wp into the O accumulator, then x += P + bp, ln = LN2(x)
-        if (threadIdx.x == 0 && !failed) {
-            tc::mbar_expect_tx(&bar_p, (uint32_t)D * 256 + (uint32_t)D * D * 2);
-            for (int kc = 0; kc < D / 8; kc++) tc::tma_load_2d(sA + kc * 2048, &tmP, kc * 8, m0, &bar_p);
-            tc::bulk_load(sB1, Wp, (uint32_t)D * D * 2, &bar_p);
-            if (tc::mbar_wait(&bar_p, 0, err, &failed)) {
-                tc::tc_fence_after();
-                const uint32_t idesc = tc::idesc_bf16(128, D);
-                for (int k = 0; k < D / 16; k++)
-                    tc::mma_bf16(tO, tc::sdesc(a0 + k * 4096, 2048, 128), tc::sdesc(w1s + k * 2 * D * 16, D * 16, 128),
-                                 idesc, k > 0 ? 1u : 0u);
-                tc::mma_commit(&bar_pm);
-            }
-        }
-        __syncwarp();
-        XRows xr;  // the residual rows, loaded while P is computed
-        if (D == 128) load_xrows(x, m0, R, warp, kMlpSerialThreads / 32, 128, xr);
-        const bool pok = __syncthreads_and(tc::mbar_wait(&bar_pm, 0, err, &failed) ? 1 : 0) != 0;
-        tc::tc_fence_after();
-        if (pok) {
-            // Wp is consumed: the f32 P tile is staged behind sA, and the LN2
-            // rows go straight into sA as the MLP's A operand
-            float* tile = reinterpret_cast<float*>(smem + (size_t)D * 256);
-            stage_rows(lane_addr(tO), quarter * 32 + lane, D, half * (D / 2), (half + 1) * (D / 2), tile);
-            __syncthreads();
-            rows_resid_ln_any<true, true>(tile, D, m0, R, bp, x, g2, be2, reinterpret_cast<bf16*>(sA), warp,
-                                          kMlpSerialThreads / 32, 128, &xr);
-        }
-        // the A tile written above is read by the MMAs (async proxy)
-        tc::fence_async_shared();
-        tc::tc_fence_before();
-        __syncthreads();
-        tc::tc_fence_after();
-    }
     const int nchunks = F / NC;
     const uint32_t wbytes = (uint32_t)D * NC * 2;
     auto issue_s = [&]() {  // S = A @ W1_chunk into tS
@@ -1416,15 +1365,13 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
     // S_{j+1} is issued right after GELU_j, ahead of O_j. The MMAs and their
     // accumulation order are those of one chunk after another.
     if (threadIdx.x == 0 && !failed) {
-        if (!PROJ) {
-            tc::mbar_expect_tx(&bar_a, (uint32_t)D * 256);
-            for (int kc = 0; kc < D / 8; kc++) tc::tma_load_2d(sA + kc * 2048, &tmA, kc * 8, m0, &bar_a);
-        }
+        tc::mbar_expect_tx(&bar_a, (uint32_t)D * 256);
+        for (int kc = 0; kc < D / 8; kc++) tc::tma_load_2d(sA + kc * 2048, &tmA, kc * 8, m0, &bar_a);
         tc::mbar_expect_tx(&bar_w1, wbytes);
         tc::bulk_load(sB1, W1, wbytes, &bar_w1);
         tc::mbar_expect_tx(&bar_w2, wbytes);
         tc::bulk_load(sB2, W2, wbytes, &bar_w2);
-        if ((PROJ || tc::mbar_wait(&bar_a, 0, err, &failed)) && tc::mbar_wait(&bar_w1, 0, err, &failed)) {
+        if (tc::mbar_wait(&bar_a, 0, err, &failed) && tc::mbar_wait(&bar_w1, 0, err, &failed)) {
             tc::tc_fence_after();
             issue_s();
         }
@@ -1483,7 +1430,7 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
         }
         __syncwarp();
     }
-    XRows xr2;  // the residual rows (this CTA wrote them above, or an earlier kernel), loaded while the last O runs
+    XRows xr2;  // the residual rows, loaded while the last O runs
     if (D == 128) load_xrows(x, m0, R, warp, kMlpSerialThreads / 32, 128, xr2);
     if (ok) {  // the last O
         ok = __syncthreads_and(tc::mbar_wait(&bar_o, (nchunks - 1) & 1, err, &failed) ? 1 : 0) != 0;
@@ -1514,6 +1461,485 @@ __device__ __forceinline__ bool all_of(bool v, int bar, int n) {
     return r != 0;
 }
 
+// Output projection + MLP of one block at dim 128 (cpu.rs:300-313): x += attn @
+// Wp + bp, A = LN2(x), x += gelu(A @ W1 + b1) @ W2 + b2, ln = LN(x) for the next
+// step. Persistent: one CTA per SM walks 128-row tiles, its stages on separate
+// warps:
+//   0-7  the row work: both residual + LayerNorms and the GELUs;
+//   8    (one lane) loads the weights in 16 KB blocks, in the order the MMAs
+//        take them, into a ring of kPMSlots slots, tiles ahead included;
+//   9    (one lane) issues every MMA;
+//   10   (one lane) loads the attention and residual rows, a tile ahead, and
+//        stores each tile's rows.
+// The hidden columns go through in chunks of 128: S_c = A @ W1_c into one of two
+// TMEM accumulators, h_c = gelu(S_c + b1_c) rounded to bf16 back over S_c's own
+// columns (a thread holds all it reads before it writes), O += h_c @ W2_c with
+// h_c as the MMA's A operand straight from TMEM. S_{c+1} runs while the row
+// warps work on S_c, and the next tile's projection P, in the accumulator that
+// chunk n - 2 has left, while they work on the last chunk: they wait for an MMA
+// only at the two ends of a tile. A (packed bf16) lies in TMEM too. The residual
+// rows stay in the row warps' registers from one LayerNorm to the other (64 of
+// 168); they come and go through two shared-memory buffers, tiles alternating
+// (an SM writes about 30 bytes a cycle: stored by the row warps themselves the
+// 64 KB held them 2500 cycles a tile).
+// The residual + LayerNorm rows are read from TMEM as 16 x 8 fragments: a warp
+// owns 16 rows and a row lies in four lanes. Wp's and W2's output columns are
+// stored in the order (pm_column) that gives lane j of the four the columns 16 m
+// + 4 j .. + 3: it moves its part of a row as float4s, and a row's sum takes two
+// shuffles, where a row spread over a warp takes five (and the fragments'
+// own column order 17). The arithmetic and its order are those of
+// rows_resid_ln_t (D = 128), so every form gives the same bits. The MMAs' K
+// order is that of tc_mlp_serial_kernel.
+// What bounds it: the GELUs' MUFU operations (two for each of 65,536 hidden
+// values a tile, 8192 cycles) and the row work around them. At 64 K rows:
+// 76 us a launch for the form before it (two CTAs per SM, one accumulator, the
+// chunk through shared memory, CTA barriers around every step), 51 for this one;
+// a tile alone on its SM: 28 and 16 us. A tile's 19.4 K cycles: the four chunks'
+// GELUs 9.8 K, S_0 1.4 K, the last O 1.5 K, the LayerNorms 2.3 K and 2.8 K.
+constexpr int kPMThreads = 11 * 32;
+constexpr int kPMD = 128, kPMNC = 128;       // width; hidden columns per chunk
+constexpr int kPMBlock = 64 * kPMD * 2;      // bytes of a weight block: 64 hidden columns (or half of Wp's K)
+constexpr int kPMSlots = 3;
+constexpr int kPMX = kPMD * 512;             // bytes of a tile's residual rows
+constexpr int kPMOffX = kPMD * 256, kPMOffW = kPMOffX + 2 * kPMX;
+constexpr int kPMSmem = kPMOffW + kPMSlots * kPMBlock;
+
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a.x), "+f"(a.y)
+        : "f"(b.x), "f"(b.y));
+    return a;
+}
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tmul.rn.f32x2 a, a, b;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a.x), "+f"(a.y)
+        : "f"(b.x), "f"(b.y));
+    return a;
+}
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+    fma2_f32(c.x, c.y, a.x, a.y, b.x, b.y);
+    return c;
+}
+
+// The logical output column in column p of the weights arranged for
+// tc_proj_mlp_kernel (fragment groups 2 m and 2 m + 1 give a thread columns 2 j,
+// 2 j + 1 of each).
+__host__ __device__ constexpr int pm_column(int p) {
+    return (p & ~15) + 4 * ((p >> 1) & 3) + 2 * ((p >> 3) & 1) + (p & 1);
+}
+
+// A layer's weights as tc_proj_mlp_kernel reads them, from the arrangements the
+// other kernels read, in 16-byte pieces (8 K elements of a column): Wp and W2
+// with their columns in pm_column's order, W1 in blocks of 64 K x 128 columns
+// (its last 64 columns, if F is an odd multiple of 64, as they were).
+__global__ void pm_arrange_kernel(const uint4* __restrict__ wp, const uint4* __restrict__ w1,
+                                  const uint4* __restrict__ w2, int F, uint4* __restrict__ dst) {
+    constexpr int D = kPMD, KC = D / 8;
+    const int n_p = KC * D, n_1 = F * KC, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_p) {
+        dst[i] = wp[(i & ~(D - 1)) + pm_column(i % D)];
+    } else if (i < n_p + n_1) {
+        const int e = i - n_p, c = e / (KC * 128);
+        if ((c + 1) * 128 > F) {
+            dst[i] = w1[e];
+        } else {
+            const int kc = e / 128 % KC, col = e % 128;
+            dst[i] = w1[((2 * c + col / 64) * KC + kc) * 64 + col % 64];
+        }
+    } else if (i < n_p + 2 * n_1) {
+        const int e = i - n_p - n_1;
+        dst[i] = w2[(e & ~(D - 1)) + pm_column(e % D)];
+    }
+}
+
+// The sum of a row that lies in four lanes (p[m] = slot 4 m + lane % 4) in
+// tree32's order.
+__device__ __forceinline__ float frag_row_sum(float (&p)[8]) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; i++) p[i] = __fadd_rn(p[i], p[i + o]);
+    p[0] = __fadd_rn(p[0], __shfl_xor_sync(0xffffffffu, p[0], 2));
+    return __fadd_rn(p[0], __shfl_xor_sync(0xffffffffu, p[0], 1));
+}
+
+// x[2 m + k] holds columns 16 m + 4 (lane % 4) .. + 3 of row k (rows lane / 4 and
+// lane / 4 + 8 of the warp's 16): x += acc + bias (acc: the warp's 16 TMEM lanes at
+// tacc), and the rows' mean and 1 / sqrt(variance + eps).
+__device__ __forceinline__ void frag_resid(float4 (&x)[16], uint32_t tacc, const float* bias, float (&mean)[2],
+                                           float (&rstd)[2]) {
+    const float4* b4 = reinterpret_cast<const float4*>(bias) + (threadIdx.x & 3);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float a[16];
+        tc::tmem_ld_frag32(tacc + 32 * q, a);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float4 bb = b4[4 * (2 * q + i)];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                float4& v = x[2 * (2 * q + i) + k];
+                const float2 lo = add_f32x2(make_float2(v.x, v.y), add_f32x2(make_float2(a[8 * i + 2 * k], a[8 * i + 2 * k + 1]),
+                                                                             make_float2(bb.x, bb.y)));
+                const float2 hi = add_f32x2(make_float2(v.z, v.w),
+                                            add_f32x2(make_float2(a[8 * i + 4 + 2 * k], a[8 * i + 5 + 2 * k]),
+                                                      make_float2(bb.z, bb.w)));
+                v = make_float4(lo.x, lo.y, hi.x, hi.y);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        float p[8];
+#pragma unroll
+        for (int m = 0; m < 8; m++) p[m] = sum4(x[2 * m + k]);
+        mean[k] = frag_row_sum(p) / (float)kPMD;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float2 nm = make_float2(-mean[k], -mean[k]);
+        float p[8];
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            const float4 v = x[2 * m + k];
+            const float2 e = add_f32x2(make_float2(v.x, v.y), nm), f = add_f32x2(make_float2(v.z, v.w), nm);
+            p[m] = __fadd_rn(__fmaf_rn(e.x, e.x, __fmul_rn(e.y, e.y)), __fmaf_rn(f.x, f.x, __fmul_rn(f.y, f.y)));
+        }
+        rstd[k] = ln_rstd(frag_row_sum(p), kPMD);
+    }
+}
+
+// LayerNorm(x) of columns 16 m + 4 (lane % 4) .. + 3 of row k, as two bf16 pairs.
+__device__ __forceinline__ uint2 frag_ln4(const float4 v, float mean, float rstd, const float4 g, const float4 b) {
+    const float2 nm = make_float2(-mean, -mean), rs = make_float2(rstd, rstd);
+    const float2 lo = fma_f32x2(mul_f32x2(add_f32x2(make_float2(v.x, v.y), nm), rs), make_float2(g.x, g.y),
+                                make_float2(b.x, b.y));
+    const float2 hi = fma_f32x2(mul_f32x2(add_f32x2(make_float2(v.z, v.w), nm), rs), make_float2(g.z, g.w),
+                                make_float2(b.z, b.w));
+    const __nv_bfloat162 l = __floats2bfloat162_rn(lo.x, lo.y), h = __floats2bfloat162_rn(hi.x, hi.y);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
+}
+// Into TMEM as an MMA's A operand: the 64 packed columns at tA.
+__device__ __forceinline__ void frag_ln_tmem(const float4 (&x)[16], const float (&mean)[2], const float (&rstd)[2],
+                                             const float* g, const float* b, uint32_t tA) {
+    const float4 *g4 = reinterpret_cast<const float4*>(g) + (threadIdx.x & 3),
+                 *b4 = reinterpret_cast<const float4*>(b) + (threadIdx.x & 3);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        uint32_t r[16];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int m = 4 * q + i;
+            const float4 gg = g4[4 * m], be = b4[4 * m];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const uint2 u = frag_ln4(x[2 * m + k], mean[k], rstd[k], gg, be);
+                r[4 * i + 2 * k] = u.x;
+                r[4 * i + 2 * k + 1] = u.y;
+            }
+        }
+        tc::tmem_st_frag32(tA + 32 * q, r);
+    }
+}
+// Into the swizzled tile sOut (boxes of 64 columns x 128 rows; tr = the tile row
+// that lane / 4 falls on).
+__device__ __forceinline__ void frag_ln_smem(const float4 (&x)[16], const float (&mean)[2], const float (&rstd)[2],
+                                             const float* g, const float* b, uint8_t* sOut, int tr) {
+    const int j = threadIdx.x & 3, sw = tr & 7;
+    const float4 *g4 = reinterpret_cast<const float4*>(g) + j, *b4 = reinterpret_cast<const float4*>(b) + j;
+    uint8_t* row = sOut + (size_t)tr * 128 + (j & 1) * 8;
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+        const float4 gg = g4[4 * m], be = b4[4 * m];
+        uint8_t* at = row + (m >> 2) * 16384 + (((2 * (m & 3) + (j >> 1)) ^ sw) << 4);
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+            *reinterpret_cast<uint2*>(at + k * 8 * 128) = frag_ln4(x[2 * m + k], mean[k], rstd[k], gg, be);
+    }
+}
+
+__global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
+    const __grid_constant__ CUtensorMap tmAttn, const __grid_constant__ CUtensorMap tmLn,
+    const __grid_constant__ CUtensorMap tmX, const bf16* __restrict__ Wp,
+    const bf16* __restrict__ W1, const bf16* __restrict__ W2, const float* __restrict__ bp, const float* __restrict__ g2,
+    const float* __restrict__ be2, const float* __restrict__ b1, const float* __restrict__ b2,
+    const float* __restrict__ g, const float* __restrict__ b, int F, int R, float* __restrict__ xg, int* err) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    constexpr int D = kPMD, NC = kPMNC, NS = kPMSlots;
+    constexpr uint32_t kB = kPMBlock;
+    uint8_t* sAT = smem;            // attention rows, then the tile's LayerNorm rows: 2 x [128][64] swizzled
+    uint8_t* sX = smem + kPMOffX;   // residual rows, tiles alternating: 2 x (8 x [128][16] f32)
+    uint8_t* sW = smem + kPMOffW;   // weight ring
+    __shared__ __align__(16) float sb1[1024], sv[6][D];          // bp, g2, be2, b2, g, b
+    __shared__ uint64_t w_full[NS], w_empty[NS], at_full, at_empty, x_full[2], p_full, a_full, s_full[2], h_full[2],
+        o_full, out_full;
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int failed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_tiles = (R + 127) / 128;
+    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int n = (F + NC - 1) / NC;  // chunks; the last may have 64 columns
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NS; i++) {
+            tc::mbar_init(&w_full[i], 1);
+            tc::mbar_init(&w_empty[i], 1);
+        }
+        for (uint64_t* q : {&at_full, &at_empty, &x_full[0], &x_full[1], &p_full, &s_full[0], &s_full[1], &o_full}) tc::mbar_init(q, 1);
+        for (uint64_t* q : {&a_full, &h_full[0], &h_full[1], &out_full}) tc::mbar_init(q, 8);  // one arrival per row warp
+        tc::fence_barrier_init();
+        failed = 0;
+        if (tc::smem_u32(smem) & 1023u) {  // operand tiles need aligned shared memory
+            failed = 1;
+            atomicExch(err, 2);
+        }
+    }
+    for (int i = threadIdx.x; i < F; i += kPMThreads) sb1[i] = b1[i];
+    for (int i = threadIdx.x; i < 6 * D; i += kPMThreads) {
+        const float* src = i < D ? bp : i < 2 * D ? g2 : i < 3 * D ? be2 : i < 4 * D ? b2 : i < 5 * D ? g : b;
+        sv[i / D][i % D] = src[i % D];
+    }
+    if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tO = tmem_base, tS = tmem_base + 128, tA = tmem_base + 384;  // O | S_0 | S_1 | A (64 columns)
+    const uint32_t tP = tS + (n & 1) * NC;                // P: the accumulator that chunk n - 2 used
+    auto blocks_of = [&](int c) { return min(NC, F - c * NC) / 64; };
+    if (warp == 8) {
+        // the weights never change: their loads do not wait for the previous kernel
+        if (tc::elect_one() && !failed) {
+            int cnt = 0;
+            bool ok = true;
+            auto put = [&](const bf16* src) {
+                const int sl = cnt % NS;
+                if (cnt >= NS) ok = ok && tc::mbar_wait(&w_empty[sl], (uint32_t)(cnt / NS - 1) & 1u, err, &failed);
+                if (!ok) return;
+                tc::mbar_expect_tx(&w_full[sl], kB);
+                tc::bulk_load(sW + sl * kB, src, kB, &w_full[sl]);
+                cnt++;
+            };
+            auto put_chunk = [&](const bf16* W, int c) {
+                for (int q = 0; q < blocks_of(c); q++) put(W + (size_t)(2 * c + q) * 64 * D);
+            };
+            auto put_p = [&]() {
+                put(Wp);
+                put(Wp + 64 * D);
+            };
+            if (my_tiles > 0) put_p();
+            for (int it = 0; it < my_tiles && ok; it++) {
+                for (int c = 0; c < 2 && c < n; c++) put_chunk(W1, c);
+                for (int c = 0; c < n && ok; c++) {
+                    if (c == n - 1 && it + 1 < my_tiles) put_p();
+                    put_chunk(W2, c);
+                    if (c + 2 < n) put_chunk(W1, c + 2);
+                }
+            }
+        }
+        __syncwarp();
+        JC_PDL_ENTRY;
+    } else if (warp == 9) {
+        JC_PDL_ENTRY;
+        if (tc::elect_one() && !failed) {
+            constexpr uint32_t id128 = tc::idesc_bf16(128, D), id64 = tc::idesc_bf16(128, 64);
+            const uint64_t dAT = tc::sdesc_sw128(tc::smem_u32(sAT));
+            const uint64_t dW128 = tc::sdesc(tc::smem_u32(sW), D * 16, 128), dW64 = tc::sdesc(tc::smem_u32(sW), 64 * 16, 128);
+            int sl = 0;
+            uint32_t ph_w = 0;
+            bool ok = true;
+            auto take = [&]() {  // the next weight block has arrived
+                ok = ok && tc::mbar_wait(&w_full[sl], ph_w, err, &failed);
+                tc::tc_fence_after();
+                return ok;
+            };
+            auto done = [&]() {
+                tc::mma_commit(&w_empty[sl]);
+                if (++sl == NS) {
+                    sl = 0;
+                    ph_w ^= 1u;
+                }
+            };
+            auto issue_p = [&](int it) {  // P = attn @ Wp
+                ok = ok && tc::mbar_wait(&at_full, (uint32_t)it & 1u, err, &failed);
+                for (int q = 0; q < 2; q++) {
+                    if (!take()) return;
+                    const uint64_t w = tc::sdesc_at(dW128, sl * kB), a = tc::sdesc_at(dAT, q * 16384);
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        tc::mma_bf16(tP, tc::sdesc_at(a, k * 32), tc::sdesc_at(w, k * 2 * D * 16), id128,
+                                     k > 0 ? 1u : (uint32_t)q);
+                    done();
+                }
+                tc::mma_commit(&at_empty);
+                tc::mma_commit(&p_full);
+            };
+            auto issue_s = [&](int c) {  // S_c = A @ W1_c: 128 columns in two K halves, or 64 in one block
+                const int nb = blocks_of(c);
+                const uint32_t t = tS + (c & 1) * NC;
+                for (int q = 0; q < nb; q++) {
+                    if (!take()) return;
+                    if (nb == 2) {
+                        const uint64_t w = tc::sdesc_at(dW128, sl * kB);
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            tc::mma_bf16_ta(t, tA + q * 32 + k * 8, tc::sdesc_at(w, k * 2 * 128 * 16), id128,
+                                            k > 0 ? 1u : (uint32_t)q);
+                    } else {
+                        const uint64_t w = tc::sdesc_at(dW64, sl * kB);
+#pragma unroll
+                        for (int k = 0; k < D / 16; k++)
+                            tc::mma_bf16_ta(t, tA + k * 8, tc::sdesc_at(w, k * 2 * 64 * 16), id64, k > 0 ? 1u : 0u);
+                    }
+                    done();
+                }
+                tc::mma_commit(&s_full[c & 1]);
+            };
+            auto issue_o = [&](int c) {  // O += h_c @ W2_c; 32 columns of h lie packed in the first 16 of their own
+                const int nb = blocks_of(c);
+                for (int q = 0; q < nb; q++) {
+                    if (!take()) return;
+                    const uint64_t w = tc::sdesc_at(dW128, sl * kB);
+                    const uint32_t t = tS + (c & 1) * NC + q * 64;
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        tc::mma_bf16_ta(tO, t + (k >> 1) * 32 + (k & 1) * 8, tc::sdesc_at(w, k * 2 * D * 16), id128,
+                                        k > 0 ? 1u : (uint32_t)(c + q > 0));
+                    done();
+                }
+                if (c == n - 1) tc::mma_commit(&o_full);
+            };
+            uint32_t ph_h[2] = {0u, 0u};
+            if (my_tiles > 0) issue_p(0);
+            for (int it = 0; it < my_tiles && ok; it++) {
+                ok = tc::mbar_wait(&a_full, (uint32_t)it & 1u, err, &failed);
+                tc::tc_fence_after();
+                for (int c = 0; c < 2 && c < n && ok; c++) issue_s(c);
+                for (int c = 0; c < n && ok; c++) {
+                    if (c == n - 1 && it + 1 < my_tiles) issue_p(it + 1);  // after O_{n-2}, which reads tP's columns
+                    ok = ok && tc::mbar_wait(&h_full[c & 1], ph_h[c & 1], err, &failed);
+                    ph_h[c & 1] ^= 1u;
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    issue_o(c);
+                    if (c + 2 < n && ok) issue_s(c + 2);  // after O_c, which reads h_c from its columns
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 10) {
+        JC_PDL_ENTRY;
+        if (tc::elect_one() && !failed) {
+            auto m0_of = [&](int it) { return ((int)blockIdx.x + it * (int)gridDim.x) * 128; };
+            auto load_attn = [&](int it) {
+                tc::mbar_expect_tx(&at_full, D * 256);
+                for (int c = 0; c < 2; c++) tc::tma_load_2d(sAT + c * 16384, &tmAttn, 64 * c, m0_of(it), &at_full);
+            };
+            auto load_x = [&](int it) {
+                tc::mbar_expect_tx(&x_full[it & 1], kPMX);
+                for (int m = 0; m < 8; m++)
+                    tc::tma_load_2d(sX + (it & 1) * kPMX + m * 8192, &tmX, 16 * m, m0_of(it), &x_full[it & 1]);
+            };
+            bool ok = true;
+            if (my_tiles > 0) {
+                load_attn(0);
+                load_x(0);
+            }
+            if (my_tiles > 1) {
+                load_x(1);
+                ok = tc::mbar_wait(&at_empty, 0, err, &failed);
+                if (ok) load_attn(1);
+            }
+            for (int it = 0; it < my_tiles && ok; it++) {
+                ok = tc::mbar_wait(&out_full, (uint32_t)it & 1u, err, &failed);
+                if (!ok) break;
+                for (int c = 0; c < 2; c++) tc::tma_store_2d(&tmLn, sAT + c * 16384, 64 * c, m0_of(it));
+                for (int m = 0; m < 8; m++) tc::tma_store_2d(&tmX, sX + (it & 1) * kPMX + m * 8192, 16 * m, m0_of(it));
+                tc::bulk_commit();
+                tc::bulk_wait_read();
+                if (it + 2 < my_tiles) {
+                    load_attn(it + 2);
+                    load_x(it + 2);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        JC_PDL_ENTRY;
+        const int quarter = warp & 3, half = warp >> 2;
+        const int tr = 32 * quarter + 16 * half + (lane >> 2);  // tile row of this thread's first row
+        const uint32_t trow = (uint32_t)(32 * quarter + 16 * half) << 16;
+        const uint32_t lane_s = ((uint32_t)(32 * quarter) << 16) + half * 64;
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
+            const bool good = __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, err, &failed) ? 1 : 0) != 0;
+            tc::tc_fence_after();
+            return good;
+        };
+        auto warp_arrive = [&](uint64_t* bar) {
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bar);
+        };
+        uint32_t ph_s[2] = {0u, 0u};
+        for (int it = 0; it < my_tiles; it++) {
+            float4 x[16];
+            float mean[2], rstd[2];
+            uint8_t* xs = sX + (it & 1) * kPMX + tr * 64 + (lane & 3) * 16;  // this thread's part of its rows
+            bool ok = warp_wait(&x_full[it & 1], (uint32_t)(it >> 1) & 1u);
+            if (!ok) break;
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                x[2 * m] = *reinterpret_cast<const float4*>(xs + m * 8192);
+                x[2 * m + 1] = *reinterpret_cast<const float4*>(xs + m * 8192 + 8 * 64);
+            }
+            if (!warp_wait(&p_full, (uint32_t)it & 1u)) break;
+            frag_resid(x, tP + trow, sv[0], mean, rstd);
+            frag_ln_tmem(x, mean, rstd, sv[1], sv[2], tA + trow);
+            warp_arrive(&a_full);
+            for (int c = 0; c < n; c++) {
+                ok = warp_wait(&s_full[c & 1], ph_s[c & 1]);
+                ph_s[c & 1] ^= 1u;
+                if (!ok) break;
+                if (half < blocks_of(c)) {
+                    const float* bj = sb1 + c * NC + half * 64;
+#pragma unroll 1
+                    for (int q = 0; q < 2; q++) {
+                        const uint32_t ts = tS + (c & 1) * NC + lane_s + 32 * q;
+                        float a[32];
+                        tc::tmem_ld32(ts, a);
+                        uint32_t h[16];
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) {
+                            const float4 bb = *reinterpret_cast<const float4*>(bj + 32 * q + i);
+                            gelu_fast_pair(a[i], a[i + 1], bb.x, bb.y);
+                            gelu_fast_pair(a[i + 2], a[i + 3], bb.z, bb.w);
+                            __nv_bfloat162 lo = __floats2bfloat162_rn(a[i], a[i + 1]);
+                            __nv_bfloat162 hi = __floats2bfloat162_rn(a[i + 2], a[i + 3]);
+                            h[i / 2] = *reinterpret_cast<uint32_t*>(&lo);
+                            h[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
+                        }
+                        tc::tmem_st16(ts, h);
+                    }
+                }
+                warp_arrive(&h_full[c & 1]);
+            }
+            if (!ok || !warp_wait(&o_full, (uint32_t)it & 1u)) break;
+            frag_resid(x, tO + trow, sv[3], mean, rstd);
+            // P of the next tile has been computed (before the last O): its attention rows are no longer read
+            frag_ln_smem(x, mean, rstd, sv[4], sv[5], sAT, tr);
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                *reinterpret_cast<float4*>(xs + m * 8192) = x[2 * m];
+                *reinterpret_cast<float4*>(xs + m * 8192 + 8 * 64) = x[2 * m + 1];
+            }
+            tc::fence_async_shared();
+            warp_arrive(&out_full);
+        }
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+}
 
 // Persistent output projection + residual + LayerNorm (cpu.rs:300-313) for
 // dims up to 128: x += attn @ Wp + bp, ln = LayerNorm2(x). One CTA per SM
@@ -2412,8 +2838,8 @@ void BF16Path::set_kernel_attributes() {
     set_smem(tc_gemm_kernel<EPI_BF16>, 200 * 1024);
     set_smem(tc_gemm_kernel<EPI_F32>, 200 * 1024);
     set_smem(tc_gemm_kernel<EPI_RESID_LN>, 200 * 1024);
-    set_smem(tc_mlp_serial_kernel<false>, kMlpSmemMax);
-    set_smem(tc_mlp_serial_kernel<true>, kMlpSmemMax);
+    set_smem(tc_mlp_serial_kernel, kMlpSmemMax);
+    set_smem(tc_proj_mlp_kernel, kPMSmem);
     set_smem(tc_projln_persistent_kernel, 225 * 1024);  // 227 KB per CTA less the static shared memory
     set_smem(tc_qkv_persistent_kernel, 225 * 1024);
     set_smem(tc_cellconv_kernel<kCellConv1>, 200 * 1024);
@@ -2429,6 +2855,19 @@ void BF16Path::set_kernel_attributes() {
     set_smem(bf_embed_kernel<6>, 100 * 1024);
     set_smem(bf_embed_kernel<7>, 100 * 1024);
     set_smem(bf_embed_kernel<8>, 100 * 1024);
+}
+
+void BF16Path::arrange(DeviceArena& arena, cudaStream_t s) {
+    if (dims_D_ != kPMD) return;
+    const size_t pieces = (size_t)(kPMD + 2 * dims_F_) * kPMD / 8;  // 16 bytes each
+    for (int l = 0; l < dims_.L; l++) {
+        bf16* dst = static_cast<bf16*>(arena.alloc(pieces * 16));
+        pm_arrange_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, s>>>(
+            reinterpret_cast<const uint4*>(wp[l]), reinterpret_cast<const uint4*>(w1v[1][l]),
+            reinterpret_cast<const uint4*>(w2v[1][l]), dims_F_, reinterpret_cast<uint4*>(dst));
+        check_launch("pm_arrange");
+        pm_w_[l] = dst;
+    }
 }
 
 // One thread per (token row, head) in CTAs of `threads` threads (64, 128 or
@@ -2489,21 +2928,19 @@ Tuning BF16Path::tuning_for(int rows) const {
     return def_tuning_;
 }
 
-// Shared memory of the MLP kernel (one stage, one h buffer; with the fused
-// projection, the f32 P tile behind the A tile).
-static size_t mlp_serial_smem(int D, int NC, bool proj = false) {
-    return std::max({(size_t)D * 256 + 2 * (size_t)D * NC * 2 + (size_t)NC * 256, (size_t)128 * D * 4,
-                     proj ? (size_t)D * 256 + (size_t)128 * D * 4 : (size_t)0});
+// Shared memory of the serial MLP kernel (one stage, one h buffer).
+static size_t mlp_serial_smem(int D, int NC) {
+    return std::max((size_t)D * 256 + 2 * (size_t)D * NC * 2 + (size_t)NC * 256, (size_t)128 * D * 4);
 }
 
 bool BF16Path::mlp_fits(int nc) const {
     return (nc == 32 || nc == 64) && dims_F_ % nc == 0 && mlp_serial_smem(dims_D_, nc) <= kMlpSmemMax;
 }
 
-bool BF16Path::proj_fuses(const Tuning& tu) const { return dims_D_ == 128 && tu.nc == 64; }
+bool BF16Path::proj_fuses(const Tuning& tu) const { return dims_D_ == kPMD && tu.nc == 64; }
 
 void BF16Path::launch_mlp(const Dims& d, const WeightsF32& w, int l, const Tuning& tu, const CUtensorMap& m_ln,
-                          const Pack& p, cudaStream_t s, const CUtensorMap* m_attn) const {
+                          const Pack& p, cudaStream_t s, const CUtensorMap* m_attn, const CUtensorMap* m_x) const {
     const int D = d.D, R = p.R;
     const int v = tu.nc == 64 ? 1 : 0;
     const float* ng = l + 1 < d.L ? w.blk[l + 1].n1g : w.norm_g;
@@ -2512,15 +2949,14 @@ void BF16Path::launch_mlp(const Dims& d, const WeightsF32& w, int l, const Tunin
     bf16* ln = reinterpret_cast<bf16*>(p.bt[0]);
     if (m_attn) {
         if (!proj_fuses(tu)) throw Error(JC_LIMIT, "the fused projection needs dim 128 and 64-column MLP chunks");
-        cuda_check(launch_pdl(tc_mlp_serial_kernel<true>, (unsigned)((R + 127) / 128), kMlpSerialThreads,
-                              mlp_serial_smem(D, tu.nc, true), s, 1u, m_ln, w1v[v][l], w2v[v][l], B.b1, B.b2, D, d.F, tu.nc, R,
-                              p.x, ng, nbeta, ln, p.err, *m_attn, wp[l], B.bp, B.n2g, B.n2b),
+        cuda_check(launch_pdl(tc_proj_mlp_kernel, (unsigned)std::min((R + 127) / 128, n_sms_), kPMThreads, kPMSmem, s, 1u, *m_attn, m_ln,
+                              *m_x, pm_w_[l], pm_w_[l] + D * D, pm_w_[l] + D * D + (size_t)d.F * D, B.bp, B.n2g, B.n2b, B.b1, B.b2, ng, nbeta, d.F, R, p.x, p.err),
                    "launch");
         return;
     }
-    cuda_check(launch_pdl(tc_mlp_serial_kernel<false>, (unsigned)((R + 127) / 128), kMlpSerialThreads,
+    cuda_check(launch_pdl(tc_mlp_serial_kernel, (unsigned)((R + 127) / 128), kMlpSerialThreads,
                           mlp_serial_smem(D, tu.nc), s, 1u, m_ln, w1v[v][l], w2v[v][l], B.b1, B.b2, D, d.F, tu.nc, R,
-                          p.x, ng, nbeta, ln, p.err, m_ln, wp[l], B.bp, B.n2g, B.n2b),
+                          p.x, ng, nbeta, ln, p.err),
                "launch");
 }
 
@@ -2569,7 +3005,7 @@ void BF16Path::tune(const Dims& d, const WeightsF32& w, const Pack& p, cudaStrea
     for (int nc : {def_tuning_.nc, 96 - def_tuning_.nc}) {  // the default width first, then the other
         // where the default width carries the fused output projection, the
         // MLP alone is not the comparison: keep it
-        if (!mlp_fits(nc) || (nc != def_tuning_.nc && proj_fuses(def_tuning_))) continue;
+        if (!mlp_fits(nc) || proj_fuses(def_tuning_)) continue;
         Tuning t = best;
         t.nc = nc;
         const float ms = time_launches([&] { launch_mlp(d, w, 0, t, m_ln, p, s); }, kTuneReps, s);
@@ -2588,7 +3024,7 @@ void BF16Path::tune(const Dims& d, const WeightsF32& w, const Pack& p, cudaStrea
     for (int threads : forms) {
         const float ms = time_launches([&] { launch_attention(d, qkv, p.inst, p.n_inst, R, attn, threads, s, &p); },
                                        kTuneReps, s);
-        log += ", \"attn_" + std::to_string(threads) + "_ms\": " + std::to_string(ms);
+        log += (log.empty() ? "\"attn_" : ", \"attn_") + std::to_string(threads) + "_ms\": " + std::to_string(ms);
         if (threads == def_attn) {
             def_ms = best_ms = ms;
         } else if (ms < kTuneMargin * def_ms && ms < best_ms) {
@@ -2688,6 +3124,9 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
     const CUtensorMap m_ln = rows_map(ln, D, R), m_attn = rows_map(attn, D, R), m_t1 = rows_map(t1, D, R);
     const CUtensorMap m_qkv_out = store_map(qkv, 3 * D, R, 3 * D, false), m_z0_out = store_map(p.z0, d.HD, R, d.HD, true);
     const CUtensorMap m_x = store_map(p.x, D, R, D, true);
+    // 64-column swizzled boxes (loads and stores of the fused projection + MLP)
+    const CUtensorMap m_attn_box = store_map(attn, D, R, D, false), m_ln_box = store_map(ln, D, R, D, false);
+    const CUtensorMap m_x_box = resid_map(p.x, D, R);
     const unsigned gm = (unsigned)((R + 127) / 128);
     const Tuning tu = tuning_for(R);
     {
@@ -2740,7 +3179,7 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
         if (proj_fuses(tu)) {
             // output projection + LayerNorm2 inside the MLP kernel
             KScope k("tc_proj_mlp", s);
-            launch_mlp(d, w, l, tu, m_ln, p, s, &m_attn);
+            launch_mlp(d, w, l, tu, m_ln_box, p, s, &m_attn_box, &m_x_box);
             check_launch("tc_proj_mlp");
             continue;
         }

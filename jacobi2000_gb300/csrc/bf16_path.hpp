@@ -36,6 +36,10 @@ class BF16Path {
     BF16Path(const Dims& d, const TensorMap* t, DeviceArena* arena);
     // Addresses of every weight pointer, in a fixed order.
     void weight_slots(std::vector<const void**>& out) const;
+    // Arranges the weights on the device for the kernels that read them in
+    // another order than the packed image holds (dim 128); once, after the
+    // weight pointers are set.
+    void arrange(DeviceArena& a, cudaStream_t s);
     // Allocates this path's token- and cell-level buffers into p.bt / p.bc
     // and its per-instance tensor-map array into p.tmaps.
     void alloc_workspace(DeviceArena& a, const Dims& d, Pack& p, int rows, long long cells, int max_inst) const;
@@ -72,8 +76,9 @@ class BF16Path {
     // The fused MLP of layer l; with m_attn (attention rows) the layer's output
     // projection + LayerNorm2 runs first in the same kernel (proj_fuses).
     void launch_mlp(const Dims& d, const WeightsF32& w, int l, const Tuning& tu, const CUtensorMap& m_ln, const Pack& p,
-                    cudaStream_t s, const CUtensorMap* m_attn = nullptr) const;
+                    cudaStream_t s, const CUtensorMap* m_attn = nullptr, const CUtensorMap* m_x = nullptr) const;
     bool proj_fuses(const Tuning& tu) const;
+    const __nv_bfloat16* pm_w_[kMaxLayers] = {};  // Wp | W1 | W2 of a layer for the fused projection + MLP
     mutable std::mutex tune_mu_;
     mutable std::map<int, Tuning> tuned_;  // row-count bucket -> schedule
     std::string cache_key_;

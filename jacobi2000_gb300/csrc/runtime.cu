@@ -670,7 +670,10 @@ void Model::finish_init() {
     inst_.tile0 = 0;
     inst_.tt0 = 0;
     inst_.ct0 = 0;
-    if (w.bf16) w.bf16->prepare(dims, pack_, &inst_, stream);
+    if (w.bf16) {
+        w.bf16->arrange(arena, stream);
+        w.bf16->prepare(dims, pack_, &inst_, stream);  // waits for the stream: the arranged weights are ready
+    }
     d_inc_ = arena.alloc_n<float>(state_len);
     cuda_check(cudaMallocHost(&h_pinned_, (2 * state_len + 64) * sizeof(float)), "cudaMallocHost", JC_OVER_BUDGET);
 }

@@ -27,6 +27,21 @@ __device__ __forceinline__ unsigned long long globaltimer() {
     return t;
 }
 
+// True in one lane of a converged warp. A branch on this, not on the lane
+// number, tells the compiler that one thread runs what follows: MMAs, commits
+// and bulk copies take their operands from uniform registers, and in code that
+// several lanes might run each of them costs a loop over the lanes (an MMA
+// issued under `lane == 0` took 130 to 250 cycles).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred = 0;
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\t.reg .pred p;\n\t"
+        "elect.sync r|p, 0xffffffff;\n\t"
+        "@p mov.s32 %0, 1;\n\t}"
+        : "+r"(pred));
+    return pred != 0;
+}
+
 // ---- mbarrier --------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -157,6 +172,30 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
     return d;                // base offset 0, layout type 0 (no swizzle)
 }
 
+// Shared-memory matrix descriptor: K-major, 128-byte swizzle (rows of 64 16-bit
+// elements, 16-byte chunk c of row r at chunk c ^ (r % 8); the operand starts
+// on a 1024-byte boundary, K step k of 16 elements 32 k bytes further).
+__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;                // leading offset: not used by this layout
+    d |= (uint64_t)(1024 >> 4) << 32;      // 8 rows x 128 bytes
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;                // 128-byte swizzle
+    return d;
+}
+
+// The descriptor of an operand `bytes` further on (the address field alone
+// changes: one addition, where a descriptor made anew costs a dozen dependent
+// instructions on the one thread that issues the MMAs).
+__device__ __forceinline__ uint64_t sdesc_at(uint64_t d, uint32_t bytes) {
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(d));
+    lo += bytes >> 4;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+    return d;
+}
+
 // Instruction descriptor of kind::f16: A = B = bf16, D = f32, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -175,6 +214,18 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// D[tmem] (+)= A[tmem] * B[smem]^T: A holds row r in lane r, two K elements per
+// 32-bit column.
+__device__ __forceinline__ void mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
@@ -218,6 +269,47 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 lanes x 32 columns as four 16x8 fragments: thread t holds row t / 4 (v[4 i],
+// v[4 i + 1]) and row t / 4 + 8 (v[4 i + 2], v[4 i + 3]) of columns 8 i + 2 (t % 4)
+// and the next (warp-collective; the lane field of taddr is the first of the 16).
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, float* v) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// The store of tmem_ld_frag32's layout: 16 lanes x 32 32-bit columns, complete
+// on return.
+__device__ __forceinline__ void tmem_st_frag32(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+        "%14, %15};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(taddr)
+        : "memory");
+}
+
+// 16 32-bit columns of this thread's TMEM lane, complete on return
+// (warp-collective).
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+        "%14, %15};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(taddr)
+        : "memory");
 }
 
 // Makes tensor maps written to global memory by ordinary copies visible to
