@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(64 * (64 / HD), 5) bf_attn_tile_kernel(Dims d,
     __syncthreads();
     JC_PDL_ENTRY;
     if (y0 >= Ity) return;  // the lower half of a tile that overhangs the grid (uniform per CTA)
-    if (threadIdx.x == 0 && !failed) {
+    if (threadIdx.x < 32 && tc::elect_one() && !failed) {
         tc::tensormap_acquire(mkv);
         tc::tensormap_acquire(mq);
         tc::mbar_expect_tx(&bar, (uint32_t)(2 * kAttBoxKV + kAttBoxQ));
@@ -1164,7 +1164,7 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const __grid_constant__ CU
     JC_PDL_ENTRY;
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
-    if (threadIdx.x == 0 && !failed) {
+    if (warp == 0 && tc::elect_one() && !failed) {
         const uint32_t bytes_b = (uint32_t)K * BN * 2;
         tc::mbar_expect_tx(&bar_load, (uint32_t)K * 256 + bytes_b);
         for (int kc = 0; kc < K / 8; kc++) tc::tma_load_2d(sA + kc * 2048, &tmA, kc * 8, m0, &bar_load);
@@ -1172,12 +1172,9 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const __grid_constant__ CU
         if (tc::mbar_wait(&bar_load, 0, err, &failed)) {
             tc::tc_fence_after();
             const uint32_t idesc = tc::idesc_bf16(128, BN);
-            const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB);
-            for (int k = 0; k < K / 16; k++) {
-                uint64_t ad = tc::sdesc(a0 + k * 4096, 2048, 128);
-                uint64_t bd = tc::sdesc(b0 + k * 2 * BN * 16, BN * 16, 128);
-                tc::mma_bf16(tmem, ad, bd, idesc, k > 0 ? 1u : 0u);
-            }
+            const uint64_t ad = tc::sdesc(tc::smem_u32(sA), 2048, 128), bd = tc::sdesc(tc::smem_u32(sB), BN * 16, 128);
+            for (int k = 0; k < K / 16; k++)
+                tc::mma_bf16(tmem, tc::sdesc_at(ad, k * 4096), tc::sdesc_at(bd, k * 2 * BN * 16), idesc, k > 0 ? 1u : 0u);
             tc::mma_commit(&bar_mma);
         }
     }
@@ -1225,7 +1222,7 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const __grid_constant__ CU
             }
             tc::fence_async_shared();
             __syncthreads();
-            if (threadIdx.x == 0) {
+            if (warp == 0 && tc::elect_one()) {
                 for (int c = 0; c < BN; c += PB) tc::tma_store_2d(&tmO, smem + (size_t)(c / PB) * 16384, n0 + c, m0);
                 tc::bulk_commit();
                 tc::bulk_wait_read();
@@ -1350,21 +1347,21 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
     JC_PDL_ENTRY;
     tc::tc_fence_after();
     const uint32_t tO = tmem_base, tS = tmem_base + s_col;
-    const uint32_t a0 = tc::smem_u32(sA), w1s = tc::smem_u32(sB1), w2s = tc::smem_u32(sB2), hs = tc::smem_u32(sH);
+    const uint64_t dA = tc::sdesc(tc::smem_u32(sA), 2048, 128), dW1 = tc::sdesc(tc::smem_u32(sB1), NC * 16, 128),
+                   dW2 = tc::sdesc(tc::smem_u32(sB2), D * 16, 128), dH = tc::sdesc(tc::smem_u32(sH), 2048, 128);
     const int nchunks = F / NC;
     const uint32_t wbytes = (uint32_t)D * NC * 2;
     auto issue_s = [&]() {  // S = A @ W1_chunk into tS
         const uint32_t idesc = tc::idesc_bf16(128, NC);
         for (int k = 0; k < D / 16; k++)
-            tc::mma_bf16(tS, tc::sdesc(a0 + k * 4096, 2048, 128), tc::sdesc(w1s + k * 2 * NC * 16, NC * 16, 128), idesc,
-                         k > 0 ? 1u : 0u);
+            tc::mma_bf16(tS, tc::sdesc_at(dA, k * 4096), tc::sdesc_at(dW1, k * 2 * NC * 16), idesc, k > 0 ? 1u : 0u);
         tc::mma_commit(&bar_s);
     };
     // Chunk j's critical path is GELU_j then S_{j+1}: W1_{j+1} is loaded as
     // soon as S_j has read W1_j, W2_j once O_{j-1} has read W2_{j-1}, and
     // S_{j+1} is issued right after GELU_j, ahead of O_j. The MMAs and their
     // accumulation order are those of one chunk after another.
-    if (threadIdx.x == 0 && !failed) {
+    if (warp == 0 && tc::elect_one() && !failed) {
         tc::mbar_expect_tx(&bar_a, (uint32_t)D * 256);
         for (int kc = 0; kc < D / 8; kc++) tc::tma_load_2d(sA + kc * 2048, &tmA, kc * 8, m0, &bar_a);
         tc::mbar_expect_tx(&bar_w1, wbytes);
@@ -1382,7 +1379,7 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
         ok = __syncthreads_and(tc::mbar_wait(&bar_s, j & 1, err, &failed) ? 1 : 0) != 0;
         tc::tc_fence_after();
         if (!ok) break;
-        if (threadIdx.x == 0 && !failed && j + 1 < nchunks) {  // S_j has read W1_j
+        if (warp == 0 && tc::elect_one() && !failed && j + 1 < nchunks) {  // S_j has read W1_j
             tc::mbar_expect_tx(&bar_w1, wbytes);
             tc::bulk_load(sB1, W1 + (size_t)(j + 1) * D * NC, wbytes, &bar_w1);
         }
@@ -1390,7 +1387,7 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
             ok = __syncthreads_and(tc::mbar_wait(&bar_o, (j - 1) & 1, err, &failed) ? 1 : 0) != 0;
             tc::tc_fence_after();
             if (!ok) break;
-            if (threadIdx.x == 0 && !failed) {
+            if (warp == 0 && tc::elect_one() && !failed) {
                 tc::mbar_expect_tx(&bar_w2, wbytes);
                 tc::bulk_load(sB2, W2 + (size_t)j * D * NC, wbytes, &bar_w2);
             }
@@ -1413,7 +1410,7 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
         tc::tc_fence_before();
         __syncthreads();
         tc::tc_fence_after();
-        if (threadIdx.x == 0 && !failed) {
+        if (warp == 0 && tc::elect_one() && !failed) {
             // S_{j+1} first (tS was read by every GELU thread), then O_j
             if (j + 1 < nchunks && tc::mbar_wait(&bar_w1, (j + 1) & 1, err, &failed)) {
                 tc::tc_fence_after();
@@ -1423,8 +1420,8 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
                 tc::tc_fence_after();
                 const uint32_t idesc = tc::idesc_bf16(128, D);
                 for (int k = 0; k < NC / 16; k++)
-                    tc::mma_bf16(tO, tc::sdesc(hs + k * 4096, 2048, 128), tc::sdesc(w2s + k * 2 * D * 16, D * 16, 128),
-                                 idesc, (j > 0 || k > 0) ? 1u : 0u);
+                    tc::mma_bf16(tO, tc::sdesc_at(dH, k * 4096), tc::sdesc_at(dW2, k * 2 * D * 16), idesc,
+                                 (j > 0 || k > 0) ? 1u : 0u);
                 tc::mma_commit(&bar_o);
             }
         }
@@ -2009,7 +2006,7 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
     const uint32_t tmem = tmem_base;
     const size_t a_bytes = (size_t)D * 256, x_bytes = (size_t)D * 512;
     if (warp == 0) {
-        if (lane == 0 && !failed) {
+        if (tc::elect_one() && !failed) {
             for (int it = 0; it < my_tiles; it++) {
                 const int s = it & 1;
                 if (it >= 2 && !tc::mbar_wait(&in_empty[s], (uint32_t)((it - 2) >> 1) & 1u, err, &failed)) break;
@@ -2023,23 +2020,22 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && !failed) {
+        if (tc::elect_one() && !failed) {
             tc::mbar_expect_tx(&b_full, (uint32_t)D * D * 2);
             tc::bulk_load(sB, Wp, (uint32_t)D * D * 2, &b_full);
             bool good = tc::mbar_wait(&b_full, 0, err, &failed);
             const uint32_t idesc = tc::idesc_bf16(128, D);
-            const uint32_t b0 = tc::smem_u32(sB);
+            const uint64_t dA = tc::sdesc(tc::smem_u32(sA), 2048, 128), dB = tc::sdesc(tc::smem_u32(sB), D * 16, 128);
             for (int it = 0; it < my_tiles && good; it++) {
                 const int s = it & 1;
                 good = tc::mbar_wait(&in_full[s], (uint32_t)(it >> 1) & 1u, err, &failed) &&
                        (it < 2 || tc::mbar_wait(&acc_empty[s], (uint32_t)((it - 2) >> 1) & 1u, err, &failed));
                 if (!good) break;
                 tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(sA + s * a_bytes);
+                const uint64_t da = tc::sdesc_at(dA, s * (uint32_t)a_bytes);
                 const uint32_t acc = tmem + (uint32_t)s * D;
                 for (int k = 0; k < D / 16; k++)
-                    tc::mma_bf16(acc, tc::sdesc(a0 + k * 4096, 2048, 128), tc::sdesc(b0 + k * 2 * D * 16, D * 16, 128),
-                                 idesc, k > 0 ? 1u : 0u);
+                    tc::mma_bf16(acc, tc::sdesc_at(da, k * 4096), tc::sdesc_at(dB, k * 2 * D * 16), idesc, k > 0 ? 1u : 0u);
                 tc::mma_commit(&in_empty[s]);
                 tc::mma_commit(&acc_full[s]);
             }
@@ -2047,7 +2043,6 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
         __syncwarp();
     } else {
         const int r = (warp & 3) * 32 + lane;
-        const bool leader = warp == 2 && lane == 0;
         for (int it = 0; it < my_tiles; it++) {
             const int s = it & 1;
             const bool ready = tc::mbar_wait(&acc_full[s], (uint32_t)(it >> 1) & 1u, err, &failed) &&
@@ -2062,7 +2057,7 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
             tc::mbar_arrive(&acc_empty[s]);
             tc::fence_async_shared();
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (leader) {
+            if (warp == 2 && tc::elect_one()) {
                 for (int bx = 0; bx < D / 32; bx++) tc::tma_store_2d(&tmX, sX + s * x_bytes + bx * 16384, bx * 32, m0);
                 tc::bulk_commit();
                 tc::bulk_wait_read();
@@ -2075,52 +2070,60 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
     if (warp == 0) tc::tmem_dealloc(tmem, ncols);
 }
 
-// Persistent q/k/v projection (cpu.rs:291-297, the three linears as one GEMM
-// over the concatenated weights): one CTA per SM walks row tiles; the whole
-// weight matrix stays in shared memory. Items are (tile, N block):
-//   warp 0     (one lane) TMA-loads each tile's LayerNorm rows into one of two
-//              slots;
-//   warp 1     (one lane) loads the weights once and issues each item's MMAs
-//              into one of two TMEM accumulators;
-//   warps 2-5  add the bias, round to bf16 into one of two 128-byte swizzled
-//              staging areas and store the item with TMA.
+// q/k/v projection (cpu.rs:291-297, the three linears as one GEMM over the
+// concatenated weights), D <= 128. A CTA keeps one N block's weights in shared
+// memory and walks row tiles; the N blocks of a tile go to neighbouring CTAs.
+//   warp 0     (one lane) loads each tile's LayerNorm rows once the MMAs have
+//              read the ones before;
+//   warp 1     (one lane) loads the weights (before the previous kernel has
+//              finished: they never change) and issues each tile's MMAs into one
+//              of two TMEM accumulators;
+//   warps 2-5  add the bias, round to bf16 into a 128-byte swizzled staging
+//              area and store it with TMA.
+// Two CTAs per SM, each with one buffer of a kind: the other CTA's work covers
+// what a CTA waits for, and few tiles still spread over three times the CTAs.
+// SW (D a multiple of 64): the rows arrive as 128-byte swizzled boxes of 64
+// columns, not as 16-byte columns (2048 pieces a tile, which the TMA unit took
+// longer over than the rest of the tile). At 64 K rows: 19 us a launch with all
+// N blocks in one CTA per SM and 16-byte columns, 16 this way; three tiles: 9
+// and 5 us.
 constexpr int kQKVPThreads = 6 * 32;
 
 struct QKVPSmem {
-    size_t b, a, stage, total;
+    size_t a, b, stage, total;
     __host__ __device__ QKVPSmem(int D, int BN) {
-        b = 0;                                            // [3D/BN][D/8][BN][8]
-        a = (size_t)3 * D * D * 2;                        // 2 x [D/8][128][8]
-        stage = (a + 2 * (size_t)D * 256 + 1023) / 1024 * 1024;  // 2 x ceil(BN/64) boxes of 16 KB
-        total = stage + 2 * (size_t)((BN + 63) / 64) * 16384;
+        a = 0;                                                    // [D/64][128][64] swizzled, or [D/8][128][8]
+        b = (size_t)D * 256;                                      // [D/8][BN][8]
+        stage = (b + (size_t)D * BN * 2 + 1023) / 1024 * 1024;    // ceil(BN/64) boxes of 16 KB
+        total = stage + (size_t)((BN + 63) / 64) * 16384;
     }
 };
 
-__global__ void __launch_bounds__(kQKVPThreads, 1) tc_qkv_persistent_kernel(
+template <bool SW>
+__global__ void __launch_bounds__(kQKVPThreads, 2) tc_qkv_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmO, const bf16* __restrict__ W,
     const float* __restrict__ bias, int D, int BN, int R, int* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const QKVPSmem L(D, BN);
-    uint8_t* sB = smem + L.b;
     uint8_t* sA = smem + L.a;
+    uint8_t* sB = smem + L.b;
     uint8_t* sStage = smem + L.stage;
-    __shared__ uint64_t b_full, a_full[2], a_empty[2], acc_full[2], acc_empty[2];
+    __shared__ uint64_t b_full, a_full, a_empty, acc_full[2], acc_empty[2];
     __shared__ __align__(16) float sbias[3 * 128];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int NB = 3 * D / BN;
+    const int NB = 3 * D / BN, nb = (int)blockIdx.x % NB;
+    const int tile0 = (int)blockIdx.x / NB, tstep = (int)gridDim.x / NB;
     const int n_tiles = (R + 127) / 128;
-    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int total = my_tiles * NB;
+    const int total = tile0 < n_tiles ? (n_tiles - 1 - tile0) / tstep + 1 : 0;
     uint32_t ncols = 32;
     while (ncols < 2u * BN) ncols <<= 1;
-    const size_t a_bytes = (size_t)D * 256, st_bytes = (size_t)((BN + 63) / 64) * 16384;
     if (threadIdx.x == 0) {
         tc::mbar_init(&b_full, 1);
+        tc::mbar_init(&a_full, 1);
+        tc::mbar_init(&a_empty, 1);
         for (int i = 0; i < 2; i++) {
-            tc::mbar_init(&a_full[i], 1);
-            tc::mbar_init(&a_empty[i], 1);
             tc::mbar_init(&acc_full[i], 1);
             tc::mbar_init(&acc_empty[i], 4 * 32);
         }
@@ -2131,69 +2134,66 @@ __global__ void __launch_bounds__(kQKVPThreads, 1) tc_qkv_persistent_kernel(
             atomicExch(err, 2);
         }
     }
-    for (int i = threadIdx.x; i < 3 * D && i < 3 * 128; i += blockDim.x) sbias[i] = bias[i];
+    for (int i = threadIdx.x; i < BN && i < 3 * 128; i += blockDim.x) sbias[i] = bias[nb * BN + i];
     if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
     tc::tc_fence_before();
     __syncthreads();
-    JC_PDL_ENTRY;
     tc::tc_fence_after();
+    if (warp == 1 && tc::elect_one() && !failed) {
+        tc::mbar_expect_tx(&b_full, (uint32_t)D * BN * 2);
+        tc::bulk_load(sB, W + (size_t)nb * D * BN, (uint32_t)D * BN * 2, &b_full);
+    }
+    __syncwarp();
+    JC_PDL_ENTRY;
     const uint32_t tmem = tmem_base;
     if (warp == 0) {
-        if (lane == 0 && !failed) {
-            for (int it = 0; it < my_tiles; it++) {
-                const int s = it & 1;
-                if (it >= 2 && !tc::mbar_wait(&a_empty[s], (uint32_t)((it - 2) >> 1) & 1u, err, &failed)) break;
-                const int m0 = ((int)blockIdx.x + it * (int)gridDim.x) * 128;
-                tc::mbar_expect_tx(&a_full[s], (uint32_t)a_bytes);
-                for (int kc = 0; kc < D / 8; kc++)
-                    tc::tma_load_2d(sA + s * a_bytes + kc * 2048, &tmA, kc * 8, m0, &a_full[s]);
+        if (tc::elect_one() && !failed) {
+            for (int it = 0; it < total; it++) {
+                if (it > 0 && !tc::mbar_wait(&a_empty, (uint32_t)(it - 1) & 1u, err, &failed)) break;
+                const int m0 = (tile0 + it * tstep) * 128;
+                tc::mbar_expect_tx(&a_full, (uint32_t)D * 256);
+                if (SW)
+                    for (int c = 0; c < D / 64; c++) tc::tma_load_2d(sA + c * 16384, &tmA, c * 64, m0, &a_full);
+                else
+                    for (int kc = 0; kc < D / 8; kc++) tc::tma_load_2d(sA + kc * 2048, &tmA, kc * 8, m0, &a_full);
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && !failed) {
-            tc::mbar_expect_tx(&b_full, (uint32_t)3 * D * D * 2);
-            tc::bulk_load(sB, W, (uint32_t)3 * D * D * 2, &b_full);
+        if (tc::elect_one() && !failed) {
             bool good = tc::mbar_wait(&b_full, 0, err, &failed);
             const uint32_t idesc = tc::idesc_bf16(128, BN);
-            const uint32_t b0 = tc::smem_u32(sB);
-            for (int g = 0; g < total && good; g++) {
-                const int it = g / NB, nb = g % NB, s = it & 1;
-                if (nb == 0) good = tc::mbar_wait(&a_full[s], (uint32_t)(it >> 1) & 1u, err, &failed);
-                if (good && g >= 2) good = tc::mbar_wait(&acc_empty[g & 1], (uint32_t)((g - 2) >> 1) & 1u, err, &failed);
+            const uint64_t dA = SW ? tc::sdesc_sw128(tc::smem_u32(sA)) : tc::sdesc(tc::smem_u32(sA), 2048, 128);
+            const uint64_t dB = tc::sdesc(tc::smem_u32(sB), BN * 16, 128);
+            for (int it = 0; it < total && good; it++) {
+                good = tc::mbar_wait(&a_full, (uint32_t)it & 1u, err, &failed) &&
+                       (it < 2 || tc::mbar_wait(&acc_empty[it & 1], (uint32_t)((it - 2) >> 1) & 1u, err, &failed));
                 if (!good) break;
                 tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(sA + s * a_bytes);
-                const uint32_t bb = b0 + (uint32_t)nb * D * BN * 2;
-                const uint32_t acc = tmem + (uint32_t)(g & 1) * BN;
+                const uint32_t acc = tmem + (uint32_t)(it & 1) * BN;
                 for (int k = 0; k < D / 16; k++)
-                    tc::mma_bf16(acc, tc::sdesc(a0 + k * 4096, 2048, 128), tc::sdesc(bb + k * 2 * BN * 16, BN * 16, 128),
-                                 idesc, k > 0 ? 1u : 0u);
-                tc::mma_commit(&acc_full[g & 1]);
-                if (nb == NB - 1) tc::mma_commit(&a_empty[s]);  // the tile's last read of A
+                    tc::mma_bf16(acc, tc::sdesc_at(dA, SW ? (k >> 2) * 16384 + (k & 3) * 32 : k * 4096),
+                                 tc::sdesc_at(dB, k * 2 * BN * 16), idesc, k > 0 ? 1u : 0u);
+                tc::mma_commit(&a_empty);
+                tc::mma_commit(&acc_full[it & 1]);
             }
         }
         __syncwarp();
     } else {
         const int r = (warp & 3) * 32 + lane;
-        const bool leader = warp == 2 && lane == 0;
-        for (int g = 0; g < total; g++) {
-            const int it = g / NB, nb = g % NB;
-            const bool ready = tc::mbar_wait(&acc_full[g & 1], (uint32_t)(g >> 1) & 1u, err, &failed);
+        for (int it = 0; it < total; it++) {
+            const bool ready = tc::mbar_wait(&acc_full[it & 1], (uint32_t)(it >> 1) & 1u, err, &failed);
+            if (warp == 2 && tc::elect_one()) tc::bulk_wait_read();  // the last store has read the staging area
             if (!all_of(ready, 1, 128)) break;
             tc::tc_fence_after();
-            // the staging area used two items ago must have been read by its store
-            if (leader && g >= 2) tc::bulk_wait_read_1();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            uint8_t* st = sStage + (size_t)(g & 1) * st_bytes;
-            const uint32_t ta = lane_addr(tmem + (uint32_t)(g & 1) * BN);
+            const uint32_t ta = lane_addr(tmem + (uint32_t)(it & 1) * BN);
             // 32 columns per TMEM round trip (BN is a multiple of 32)
             for (int c = 0; c < BN; c += 32) {
                 float a[32];
                 tc::tmem_ld32(ta + c, a);
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
-                    const float4 bv = *reinterpret_cast<const float4*>(sbias + nb * BN + c + i);
+                    const float4 bv = *reinterpret_cast<const float4*>(sbias + c + i);
                     a[i] += bv.x;
                     a[i + 1] += bv.y;
                     a[i + 2] += bv.z;
@@ -2202,23 +2202,23 @@ __global__ void __launch_bounds__(kQKVPThreads, 1) tc_qkv_persistent_kernel(
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int cc = c + 16 * h;
-                    uint8_t* box = st + (size_t)(cc / 64) * 16384 + (size_t)r * 128;
+                    uint8_t* box = sStage + (size_t)(cc / 64) * 16384 + (size_t)r * 128;
                     const int j0 = (cc % 64) / 8;
                     BfVec<8>::store(reinterpret_cast<bf16*>(box + ((j0 ^ (r & 7)) << 4)), a + 16 * h);
                     BfVec<8>::store(reinterpret_cast<bf16*>(box + (((j0 + 1) ^ (r & 7)) << 4)), a + 16 * h + 8);
                 }
             }
             tc::tc_fence_before();
-            tc::mbar_arrive(&acc_empty[g & 1]);
+            tc::mbar_arrive(&acc_empty[it & 1]);
             tc::fence_async_shared();
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (leader) {
-                const int m0 = ((int)blockIdx.x + it * (int)gridDim.x) * 128;
-                for (int c = 0; c < BN; c += 64) tc::tma_store_2d(&tmO, st + (size_t)(c / 64) * 16384, nb * BN + c, m0);
+            if (warp == 2 && tc::elect_one()) {
+                const int m0 = (tile0 + it * tstep) * 128;
+                for (int c = 0; c < BN; c += 64) tc::tma_store_2d(&tmO, sStage + (size_t)(c / 64) * 16384, nb * BN + c, m0);
                 tc::bulk_commit();
             }
         }
-        if (leader) tc::bulk_wait_read();
+        if (warp == 2 && tc::elect_one()) tc::bulk_wait_read();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -2303,7 +2303,7 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
     const uint32_t tmem = tmem_base;
     const uint32_t wtap = (uint32_t)C * BN * 2;  // bytes of one tap's B block
     const bf16* Wn = Wt + (size_t)nb * 9 * C * BN;
-    if (threadIdx.x == 0 && !failed) {
+    if (warp == 0 && tc::elect_one() && !failed) {
         tc::tensormap_acquire(map);
         tc::tensormap_acquire(omap);
         tc::mbar_expect_tx(&bar_h, (uint32_t)(C / 8) * (kHaloW * kHaloH * 16));
@@ -2315,19 +2315,17 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
         }
         bool good = tc::mbar_wait(&bar_h, 0, err, &failed);
         const uint32_t idesc = tc::idesc_bf16(128, BN);
-        const uint32_t h0 = tc::smem_u32(sHalo);
+        const uint64_t dH = tc::sdesc(tc::smem_u32(sHalo), kHaloPlane, kHaloW * 16), dB = tc::sdesc(tc::smem_u32(sB), BN * 16, 128);
         for (int t = 0; t < 9 && good; t++) {
             const int buf = t % NS;
             good = tc::mbar_wait(&bar_b[buf], (uint32_t)(t / NS) & 1u, err, &failed);
             if (!good) break;
             tc::tc_fence_after();
             const int ky = t / 3, kx = t % 3;
-            const uint32_t b0 = tc::smem_u32(sB + buf * wtap);
-            for (int k = 0; k < C / 16; k++) {
-                uint64_t ad = tc::sdesc(h0 + 2 * k * kHaloPlane + (ky * kHaloW + kx) * 16, kHaloPlane, kHaloW * 16);
-                uint64_t bd = tc::sdesc(b0 + 2 * k * BN * 16, BN * 16, 128);
-                tc::mma_bf16(tmem, ad, bd, idesc, (t > 0 || k > 0) ? 1u : 0u);
-            }
+            const uint64_t dh = tc::sdesc_at(dH, (ky * kHaloW + kx) * 16), db = tc::sdesc_at(dB, buf * wtap);
+            for (int k = 0; k < C / 16; k++)
+                tc::mma_bf16(tmem, tc::sdesc_at(dh, 2 * k * kHaloPlane), tc::sdesc_at(db, 2 * k * BN * 16), idesc,
+                             (t > 0 || k > 0) ? 1u : 0u);
             if (t + NS < 9) {
                 // the stage is refilled once the MMAs reading it are done
                 tc::mma_commit(&bar_m[buf]);
@@ -2373,7 +2371,7 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
         }
         tc::fence_async_shared();
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (int c = 0; c < BN; c += PB)
                 tc::tma_store_3d(omap, stage + (size_t)(c / PB) * 16384, nb * BN + c, x0, y0);
             tc::bulk_commit();
@@ -2499,7 +2497,7 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
         y0 = (tl / tiles_x) * kConvTY;
     };
     if (warp == 0) {
-        if (lane == 0 && !failed) {
+        if (tc::elect_one() && !failed) {
             // halo producer
             for (int it = 0; it < my_tiles; it++) {
                 const int hb = it % HS;
@@ -2514,42 +2512,40 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && !failed) {
+        if (tc::elect_one() && !failed) {
             // MMA issuer: the weights once, then every tile
             tc::mbar_expect_tx(&w_full, wbytes);
             tc::bulk_load(sW, Wt, wbytes, &w_full);
             bool good = tc::mbar_wait(&w_full, 0, err, &failed);
             const uint32_t idesc = tc::idesc_f16(128, 32);  // f16 input and weights, N = 32
-            const uint32_t w0 = tc::smem_u32(sW);
+            const uint64_t dW = tc::sdesc(tc::smem_u32(sW), 32 * 16, 128);
+            const uint64_t dH = tc::sdesc(tc::smem_u32(sHalo), kCellPlane, KIND == kCellConv1 ? kHaloW * 16 : 128);
             for (int it = 0; it < my_tiles && good; it++) {
                 const int b = it & 1, hb = it % HS;
                 good = tc::mbar_wait(&h_full[hb], (uint32_t)(it / HS) & 1u, err, &failed) &&
                        (it < 2 || tc::mbar_wait(&a_empty[b], (uint32_t)((it - 2) >> 1) & 1u, err, &failed));
                 if (!good) break;
                 tc::tc_fence_after();
-                const uint32_t h0 = tc::smem_u32(sHalo + hb * halo_bytes);
+                const uint64_t dh = tc::sdesc_at(dH, hb * (uint32_t)halo_bytes);
                 const uint32_t acc = tmem + (uint32_t)b * BN;
                 if constexpr (KIND == kCellConv1) {
                     // rows = the 8 x 16 output positions (8-row groups 10 positions apart)
-                    for (int t = 0; t < 9; t++) {
-                        const int ky = t / 3, kx = t % 3;
-                        const uint32_t b0 = w0 + (uint32_t)t * C * 32 * 2;
-                        for (int k = 0; k < C / 16; k++) {
-                            uint64_t ad = tc::sdesc(h0 + 2 * k * kCellPlane + (ky * kHaloW + kx) * 16, kCellPlane,
-                                                    kHaloW * 16);
-                            uint64_t bd = tc::sdesc(b0 + 2 * k * 32 * 16, 32 * 16, 128);
-                            tc::mma_bf16(acc, ad, bd, idesc, (t > 0 || k > 0) ? 1u : 0u);
-                        }
-                    }
+#pragma unroll
+                    for (int t = 0; t < 9; t++)
+#pragma unroll
+                        for (int k = 0; k < kZcCh / 16; k++)
+                            tc::mma_bf16(acc, tc::sdesc_at(dh, 2 * k * kCellPlane + ((t / 3) * kHaloW + t % 3) * 16),
+                                         tc::sdesc_at(dW, (t * kZcCh / 8 + 2 * k) * 32 * 16), idesc,
+                                         (t > 0 || k > 0) ? 1u : 0u);
                 } else {
                     // rows = halo positions 0..127 and 128..255 (those past 179,
                     // read past the plane, are never used)
+#pragma unroll
                     for (int m = 0; m < 2; m++)
-                        for (int k = 0; k < C / 16; k++) {
-                            uint64_t ad = tc::sdesc(h0 + 2 * k * kCellPlane + m * 128 * 16, kCellPlane, 128);
-                            uint64_t bd = tc::sdesc(w0 + 2 * k * 32 * 16, 32 * 16, 128);
-                            tc::mma_bf16(acc + (uint32_t)m * 32, ad, bd, idesc, k > 0 ? 1u : 0u);
-                        }
+#pragma unroll
+                        for (int k = 0; k < 2; k++)
+                            tc::mma_bf16(acc + (uint32_t)m * 32, tc::sdesc_at(dh, 2 * k * kCellPlane + m * 128 * 16),
+                                         tc::sdesc_at(dW, 2 * k * 32 * 16), idesc, k > 0 ? 1u : 0u);
                 }
                 tc::mma_commit(&h_empty[hb]);
                 tc::mma_commit(&a_full[b]);
@@ -2559,7 +2555,6 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
     } else {
         // epilogue: thread r = TMEM lane r
         const int r = (warp & 3) * 32 + lane;
-        const bool leader = warp == 2 && lane == 0;
         for (int it = 0; it < my_tiles; it++) {
             const int b = it & 1;
             // the tile's instance, origin and (conv2) state, fetched before
@@ -2623,7 +2618,7 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
                 asm volatile("bar.sync 1, 128;" ::: "memory");  // Z is rewritten by the next tile
             } else {
                 // the staging box used two tiles ago must have been read by its store
-                if (leader && it >= 1) tc::bulk_wait_read();
+                if (warp == 2 && it >= 1 && tc::elect_one()) tc::bulk_wait_read();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 uint8_t* box = sStage + (size_t)r * 16;  // [4 planes][128][8] f16
                 for (int c = 0; c < BN; c += 16) {
@@ -2644,7 +2639,7 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
                 tc::mbar_arrive(&a_empty[b]);
                 tc::fence_async_shared();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (leader) {
+                if (warp == 2 && tc::elect_one()) {
                     const CUtensorMap* omap = maps + kMapsPerInst * ii + 3;
                     tc::tensormap_acquire(omap);
                     tc::tma_store_3d(omap, sStage, x0 * 8, y0, 0);
@@ -2652,7 +2647,7 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
                 }
             }
         }
-        if (KIND == kCellConv1 && leader) tc::bulk_wait_read();
+        if (KIND == kCellConv1 && warp == 2 && tc::elect_one()) tc::bulk_wait_read();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -2841,7 +2836,8 @@ void BF16Path::set_kernel_attributes() {
     set_smem(tc_mlp_serial_kernel, kMlpSmemMax);
     set_smem(tc_proj_mlp_kernel, kPMSmem);
     set_smem(tc_projln_persistent_kernel, 225 * 1024);  // 227 KB per CTA less the static shared memory
-    set_smem(tc_qkv_persistent_kernel, 225 * 1024);
+    set_smem(tc_qkv_kernel<false>, 225 * 1024);
+    set_smem(tc_qkv_kernel<true>, 225 * 1024);
     set_smem(tc_cellconv_kernel<kCellConv1>, 200 * 1024);
     set_smem(tc_cellconv_kernel<kCellConv2>, 200 * 1024);
     set_smem(bf_attn_tile_kernel<32>, 200 * 1024);
@@ -3160,9 +3156,15 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
             KScope k("tc_qkv", s);
             const int BN = bn_qkv;
             if (D <= 128) {
-                const unsigned grid = (unsigned)std::min((int)gm, n_sms_);
-                cuda_check(launch_pdl(tc_qkv_persistent_kernel, grid, kQKVPThreads, QKVPSmem(D, BN).total, s, 1u, m_ln, m_qkv_out, wqkv[l],
-                                                                                         B.bqkv, D, BN, R, p.err), "launch");
+                const int NB = 3 * D / BN;
+                const unsigned grid = (unsigned)(NB * std::min((int)gm, std::max(1, 2 * n_sms_ / NB)));
+                const size_t smem = QKVPSmem(D, BN).total;
+                if (D % 64 == 0)
+                    cuda_check(launch_pdl(tc_qkv_kernel<true>, grid, kQKVPThreads, smem, s, 1u, m_ln_box, m_qkv_out, wqkv[l],
+                                          B.bqkv, D, BN, R, p.err), "launch");
+                else
+                    cuda_check(launch_pdl(tc_qkv_kernel<false>, grid, kQKVPThreads, smem, s, 1u, m_ln, m_qkv_out, wqkv[l],
+                                          B.bqkv, D, BN, R, p.err), "launch");
             } else {
                 GemmEpi ep{B.bqkv, qkv, nullptr, nullptr, nullptr, nullptr, 3 * D};
                 const size_t smem = std::max((size_t)D * 256 + (size_t)D * BN * 2, (size_t)((BN + 63) / 64) * 16384);
