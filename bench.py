@@ -179,7 +179,7 @@ def kernel_work(name: str, B: int, cells: int, D: int, F: int):
     R, N = B * cells // 16, B * cells
     flop = {"tc_qkv": 2 * R * D * 3 * D, "tc_proj_ln": 2 * R * D * D, "tc_mlp": 4 * R * D * F,
             "tc_proj_mlp": 2 * R * D * D + 4 * R * D * F,
-            "tc_token_mix": 18 * R * D * D, "tc_to_cells": 2 * R * D * 32, "tc_conv1": 2 * N * 35 * 9 * 32,
+            "tc_token_mix": 18 * R * D * D, "tc_mix_cells": 18 * R * D * D + 2 * R * D * 32, "tc_to_cells": 2 * R * D * 32, "tc_conv1": 2 * N * 35 * 9 * 32,
             "f32_ln_qkv": 2 * R * D * 3 * D, "f32_proj": 2 * R * D * D, "f32_ln_ff1": 2 * R * D * F,
             "f32_ff2": 2 * R * F * D, "f32_token_mix": 18 * R * D * D, "f32_to_cells": 2 * R * D * 32,
             "f32_conv1": 2 * N * 35 * 9 * 32, "tc_conv2": 2 * N * 32 * 9 * 3, "f32_conv2_step": 2 * N * 32 * 9 * 3}

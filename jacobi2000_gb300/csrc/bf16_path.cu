@@ -2383,6 +2383,232 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
     if (warp == 0) tc::tmem_dealloc(tmem, ncols);
 }
 
+// token_mix and to_cells for dims up to 128 (cpu.rs:326-334): t1 = xn + gelu(
+// conv3x3(xn) + b) rounded to bf16, z0 = t1 @ Wtc + b. Persistent, one CTA per SM
+// walking 8 x 16 token tiles, its stages on separate warps:
+//   0-3  copy each tile's halo (10 x 18 positions of xn) into one of two buffers
+//        [C/8 planes][18][10][8], 16 bytes a copy, zeros outside the grid;
+//   4    (one lane) loads the tap weights, one after another, into a ring of
+//        three, and Wtc once, all before the previous kernel has finished where
+//        they can be;
+//   5    (one lane) issues the MMAs: 9 taps x C / 16 K steps into one of two TMEM
+//        accumulators (tap (ky, kx) is the halo from position (ky, kx)), and
+//        to_cells' from t1 in TMEM;
+//   6-9  (one TMEM lane quarter each) the GELU and the residual, t1 packed into
+//        TMEM, z0 to memory.
+// A plane takes kMixPlane bytes, 16 more than its positions, so that a warp's
+// copies (16 planes of two positions) fall on different banks. The MMA order is
+// that of tc_conv3_kernel and tc_gemm_kernel, which serve wider models.
+// At 64 K rows both took 48 us (the halo as 2880 16-byte pieces a tile through
+// the TMA unit, two taps in flight, t1 through memory), this takes 0; four
+// tiles: 19 and 0.
+constexpr int kMixThreads = 10 * 32, kMixTaps = 3;
+constexpr int kMixPlane = kHaloW * kHaloH * 16 + 16;
+
+struct MixSmem {
+    size_t halo, halo_bytes, w, tap, wtc, total;
+    __host__ __device__ explicit MixSmem(int C) {
+        halo = 0;
+        halo_bytes = ((size_t)(C / 8) * kMixPlane + 127) / 128 * 128;
+        w = (2 * halo_bytes + 1023) / 1024 * 1024;
+        tap = (size_t)2 * C * C;  // [C/8][C][8]
+        wtc = w + kMixTaps * tap;
+        total = wtc + (size_t)64 * C;  // [C/8][32][8]
+    }
+};
+
+__global__ void __launch_bounds__(kMixThreads, 1) tc_mix_cells_kernel(
+    const bf16* __restrict__ xn, const bf16* __restrict__ Wt, const float* __restrict__ bias,
+    const bf16* __restrict__ Wtc, const float* __restrict__ tc_bias, int C, int n_tiles, const InstDev* inst, int n_inst,
+    float* __restrict__ z0, int* err) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    constexpr int HD = 32, NS = kMixTaps;
+    const MixSmem L(C);
+    const uint32_t tap = (uint32_t)L.tap;
+    __shared__ uint64_t h_full[2], h_empty[2], w_full[NS], w_empty[NS], wtc_full, acc_full[2], acc_empty[2], t_full, z_full;
+    __shared__ __align__(16) float sbias[128], szb[HD];
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int failed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; i++) {
+            tc::mbar_init(&h_full[i], 128);
+            tc::mbar_init(&h_empty[i], 1 + 4);  // the MMAs have read the halo, and the epilogue warps its centre
+            tc::mbar_init(&acc_full[i], 1);
+            tc::mbar_init(&acc_empty[i], 4);
+        }
+        for (int i = 0; i < NS; i++) {
+            tc::mbar_init(&w_full[i], 1);
+            tc::mbar_init(&w_empty[i], 1);
+        }
+        tc::mbar_init(&wtc_full, 1);
+        tc::mbar_init(&t_full, 4);
+        tc::mbar_init(&z_full, 1);
+        tc::fence_barrier_init();
+        failed = 0;
+        if ((tc::smem_u32(smem) & 1023u) || C > 128 || C % 32) {
+            failed = 1;
+            atomicExch(err, 2);
+        }
+    }
+    for (int i = threadIdx.x; i < C && i < 128; i += kMixThreads) sbias[i] = bias[i];
+    if (threadIdx.x < HD) szb[threadIdx.x] = tc_bias[threadIdx.x];
+    if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tT = tmem_base + 256, tZ = tmem_base + 320;  // accumulators | t1 (C / 2 columns) | z0
+    auto tile_of = [&](int it, int& x0, int& y0) {  // by a whole warp
+        const int tile = (int)blockIdx.x + it * (int)gridDim.x;
+        const int ii = warp_find_last_le(n_inst, tile, [&](int i) { return (long long)inst[i].tt0; });
+        const int tiles_x = (inst[ii].tx + kConvTX - 1) / kConvTX, tl = tile - inst[ii].tt0;
+        x0 = (tl % tiles_x) * kConvTX;
+        y0 = (tl / tiles_x) * kConvTY;
+        return ii;
+    };
+    if (warp < 4) {
+        JC_PDL_ENTRY;
+        const int np = C / 8;
+        for (int it = 0; it < my_tiles; it++) {
+            const int hb = it & 1;
+            int x0, y0;
+            const InstDev& I = inst[tile_of(it, x0, y0)];
+            const int tx = I.tx, ty = I.ty;
+            const bf16* base = xn + (size_t)I.row0 * C;
+            bool ok = it < 2 || tc::mbar_wait(&h_empty[hb], (uint32_t)((it - 2) >> 1) & 1u, err, &failed);
+            if (!__all_sync(0xffffffffu, ok ? 1 : 0)) break;
+            uint8_t* dst = smem + L.halo + hb * L.halo_bytes;
+            for (int e = threadIdx.x; e < kHaloW * kHaloH * np; e += 128) {
+                const int pos = e / np, pl = e - pos * np;
+                const int y = y0 + pos / kHaloW - 1, x = x0 + pos % kHaloW - 1;
+                const bool in = y >= 0 && x >= 0 && y < ty && x < tx;
+                cp_async16(dst + (size_t)pl * kMixPlane + pos * 16, in ? base + ((size_t)y * tx + x) * C + pl * 8 : xn, in);
+            }
+            cp_async_wait_all();
+            tc::fence_async_shared();  // read by the MMAs
+            tc::mbar_arrive(&h_full[hb]);
+        }
+    } else if (warp == 4) {
+        if (tc::elect_one() && !failed) {
+            bool ok = true;
+            tc::mbar_expect_tx(&wtc_full, 64u * C);
+            tc::bulk_load(smem + L.wtc, Wtc, 64u * C, &wtc_full);
+            for (int g = 0; g < 9 * my_tiles && ok; g++) {
+                const int sl = g % NS;
+                if (g >= NS) ok = tc::mbar_wait(&w_empty[sl], (uint32_t)(g / NS - 1) & 1u, err, &failed);
+                if (!ok) break;
+                tc::mbar_expect_tx(&w_full[sl], tap);
+                tc::bulk_load(smem + L.w + sl * tap, Wt + (size_t)(g % 9) * C * C, tap, &w_full[sl]);
+            }
+        }
+        __syncwarp();
+        JC_PDL_ENTRY;
+    } else if (warp == 5) {
+        JC_PDL_ENTRY;
+        if (tc::elect_one() && !failed) {
+            const uint32_t idC = tc::idesc_bf16(128, C), idZ = tc::idesc_bf16(128, HD);
+            const uint64_t dH = tc::sdesc(tc::smem_u32(smem + L.halo), kMixPlane, kHaloW * 16);
+            const uint64_t dW = tc::sdesc(tc::smem_u32(smem + L.w), C * 16, 128);
+            const uint64_t dZ = tc::sdesc(tc::smem_u32(smem + L.wtc), HD * 16, 128);
+            int z_done = 0;  // tiles whose to_cells has been issued
+            auto issue_z = [&]() {
+                tc::tc_fence_after();
+                for (int k = 0; k < C / 16; k++)
+                    tc::mma_bf16_ta(tZ, tT + k * 8, tc::sdesc_at(dZ, k * 2 * HD * 16), idZ, k > 0 ? 1u : 0u);
+                tc::mma_commit(&z_full);
+                z_done++;
+            };
+            bool ok = tc::mbar_wait(&wtc_full, 0, err, &failed);
+            int g = 0;
+            for (int it = 0; it < my_tiles && ok; it++) {
+                const int b = it & 1;
+                ok = tc::mbar_wait(&h_full[b], (uint32_t)(it >> 1) & 1u, err, &failed) &&
+                     (it < 2 || tc::mbar_wait(&acc_empty[b], (uint32_t)((it - 2) >> 1) & 1u, err, &failed));
+                const uint64_t dh = tc::sdesc_at(dH, b * (uint32_t)L.halo_bytes);
+                for (int t = 0; t < 9 && ok; t++, g++) {
+                    const int sl = g % NS;
+                    ok = tc::mbar_wait(&w_full[sl], (uint32_t)(g / NS) & 1u, err, &failed);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    const uint64_t a = tc::sdesc_at(dh, ((t / 3) * kHaloW + t % 3) * 16), w = tc::sdesc_at(dW, sl * tap);
+                    for (int k = 0; k < C / 16; k++)
+                        tc::mma_bf16(tmem_base + b * 128, tc::sdesc_at(a, 2 * k * kMixPlane), tc::sdesc_at(w, 2 * k * C * 16),
+                                     idC, (t > 0 || k > 0) ? 1u : 0u);
+                    tc::mma_commit(&w_empty[sl]);
+                    // the tile before has its t1: its to_cells goes in between
+                    if (z_done < it && tc::mbar_try_wait(&t_full, (uint32_t)z_done & 1u)) issue_z();
+                }
+                if (!ok) break;
+                tc::mma_commit(&h_empty[b]);
+                tc::mma_commit(&acc_full[b]);
+                if (z_done < it) {
+                    ok = tc::mbar_wait(&t_full, (uint32_t)z_done & 1u, err, &failed);
+                    if (ok) issue_z();
+                }
+            }
+            if (ok && z_done < my_tiles && tc::mbar_wait(&t_full, (uint32_t)z_done & 1u, err, &failed)) issue_z();
+        }
+        __syncwarp();
+    } else {
+        JC_PDL_ENTRY;
+        const int r = (warp & 3) * 32 + lane;
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
+            const bool good = __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, err, &failed) ? 1 : 0) != 0;
+            tc::tc_fence_after();
+            return good;
+        };
+        for (int it = 0; it < my_tiles; it++) {
+            const int b = it & 1;
+            int x0, y0;
+            const InstDev& I = inst[tile_of(it, x0, y0)];
+            const int x = x0 + r % kConvTX, y = y0 + r / kConvTX;
+            const bool inside = x < I.tx && y < I.ty;
+            float* out = z0 + ((size_t)I.row0 + (inside ? (size_t)y * I.tx + x : 0)) * HD;
+            if (!warp_wait(&h_full[b], (uint32_t)(it >> 1) & 1u) || !warp_wait(&acc_full[b], (uint32_t)(it >> 1) & 1u)) break;
+            // the centre of the halo is xn at this token
+            const uint8_t* centre = smem + L.halo + b * L.halo_bytes + ((r / kConvTX + 1) * kHaloW + r % kConvTX + 1) * 16;
+            for (int c = 0; c < C; c += 32) {
+                float a[32];
+                tc::tmem_ld32(lane_addr(tmem_base + b * 128 + c), a);
+                uint32_t h[16];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float xv[8];
+                    BfVec<8>::load(reinterpret_cast<const bf16*>(centre + (size_t)(c / 8 + q) * kMixPlane), xv);
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        float &v0 = a[8 * q + i], &v1 = a[8 * q + i + 1];
+                        gelu_fast_pair(v0, v1, sbias[c + 8 * q + i], sbias[c + 8 * q + i + 1]);
+                        __nv_bfloat162 t = __floats2bfloat162_rn(xv[i] + v0, xv[i + 1] + v1);
+                        h[4 * q + i / 2] = *reinterpret_cast<uint32_t*>(&t);
+                    }
+                }
+                tc::tmem_st16(lane_addr(tT + c / 2), h);
+            }
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                tc::mbar_arrive(&acc_empty[b]);
+                tc::mbar_arrive(&h_empty[b]);
+                tc::mbar_arrive(&t_full);
+            }
+            if (!warp_wait(&z_full, (uint32_t)it & 1u)) break;
+            float z[HD];
+            tc::tmem_ld32(lane_addr(tZ), z);
+            if (inside) {
+#pragma unroll
+                for (int i = 0; i < HD; i += 4)
+                    *reinterpret_cast<float4*>(out + i) =
+                        make_float4(z[i] + szb[i], z[i + 1] + szb[i + 1], z[i + 2] + szb[i + 2], z[i + 3] + szb[i + 3]);
+            }
+        }
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+}
+
 // Persistent cell-head convolutions on the tensor cores, one CTA walking
 // cell tiles tile = blockIdx.x + k gridDim.x with its stages on separate
 // warps, so the halo loads, the MMAs and the epilogue of consecutive tiles
@@ -2843,6 +3069,7 @@ void BF16Path::set_kernel_attributes() {
     set_smem(bf_attn_tile_kernel<32>, 200 * 1024);
     set_smem(bf_attn_tile_kernel<64>, 200 * 1024);
     set_smem(tc_conv3_kernel<CONV_TOKMIX>, 200 * 1024);
+    set_smem(tc_mix_cells_kernel, 225 * 1024);
     set_smem(bf_embed_kernel<1>, 100 * 1024);
     set_smem(bf_embed_kernel<2>, 100 * 1024);
     set_smem(bf_embed_kernel<3>, 100 * 1024);
@@ -3205,20 +3432,27 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
             check_launch("tc_mlp");
         }
     }
-    {
-        KScope k("tc_token_mix", s);
-        const int BN = bn_tm;
-        const int NS = conv3_smem(D, BN, 9) <= 100 * 1024 ? 9 : 2;
-        cuda_check(launch_pdl(tc_conv3_kernel<CONV_TOKMIX>, dim3(p.n_ttiles, D / BN), 128, conv3_launch_smem(D, BN, NS, 2), s, 1u, 
-            reinterpret_cast<const CUtensorMap*>(p.tmaps), 0, 2, wtm, w.tm_b, D, BN, NS, p.inst, n, p.err), "launch");
-        check_launch("tc_token_mix");
-    }
-    {
-        KScope k("tc_to_cells", s);
-        GemmEpi ep{w.tc_b, nullptr, p.z0, nullptr, nullptr, nullptr, d.HD};
-        const size_t smem = std::max((size_t)D * 256 + (size_t)D * d.HD * 2, (size_t)((d.HD + 31) / 32) * 16384);
-        cuda_check(launch_pdl(tc_gemm_kernel<EPI_F32>, dim3(gm, 1), 128, smem, s, 1u, m_t1, m_z0_out, wtc, D, d.HD, R, ep, p.err), "launch");
-        check_launch("tc_to_cells");
+    if (D <= 128) {
+        KScope k("tc_mix_cells", s);
+        cuda_check(launch_pdl(tc_mix_cells_kernel, (unsigned)std::min(p.n_ttiles, n_sms_), kMixThreads, MixSmem(D).total, s, 1u,
+                              ln, wtm, w.tm_b, wtc, w.tc_b, D, p.n_ttiles, p.inst, n, p.z0, p.err), "launch");
+        check_launch("tc_mix_cells");
+    } else {
+        {
+            KScope k("tc_token_mix", s);
+            const int BN = bn_tm;
+            const int NS = conv3_smem(D, BN, 9) <= 100 * 1024 ? 9 : 2;
+            cuda_check(launch_pdl(tc_conv3_kernel<CONV_TOKMIX>, dim3(p.n_ttiles, D / BN), 128, conv3_launch_smem(D, BN, NS, 2), s, 1u, 
+                reinterpret_cast<const CUtensorMap*>(p.tmaps), 0, 2, wtm, w.tm_b, D, BN, NS, p.inst, n, p.err), "launch");
+            check_launch("tc_token_mix");
+        }
+        {
+            KScope k("tc_to_cells", s);
+            GemmEpi ep{w.tc_b, nullptr, p.z0, nullptr, nullptr, nullptr, d.HD};
+            const size_t smem = std::max((size_t)D * 256 + (size_t)D * d.HD * 2, (size_t)((d.HD + 31) / 32) * 16384);
+            cuda_check(launch_pdl(tc_gemm_kernel<EPI_F32>, dim3(gm, 1), 128, smem, s, 1u, m_t1, m_z0_out, wtc, D, d.HD, R, ep, p.err), "launch");
+            check_launch("tc_to_cells");
+        }
     }
     {
         KScope k("bf_upsample", s);
