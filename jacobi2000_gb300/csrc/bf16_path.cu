@@ -2400,8 +2400,8 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
 // copies (16 planes of two positions) fall on different banks. The MMA order is
 // that of tc_conv3_kernel and tc_gemm_kernel, which serve wider models.
 // At 64 K rows both took 48 us (the halo as 2880 16-byte pieces a tile through
-// the TMA unit, two taps in flight, t1 through memory), this takes 0; four
-// tiles: 19 and 0.
+// the TMA unit, two taps in flight, t1 through memory), this takes 33; four
+// tiles: 19 and 13.
 constexpr int kMixThreads = 10 * 32, kMixTaps = 3;
 constexpr int kMixPlane = kHaloW * kHaloH * 16 + 16;
 
