@@ -14,6 +14,7 @@
 #include "engine.hpp"
 #include "fp32_kernels.cuh"
 #include "launch.hpp"
+#include "tc.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -768,6 +769,198 @@ projection_kernel(Dims d, const InstDev* inst, ProjSlot* slots, int init, int ca
     cluster.sync();  // peers may still read this CTA's segment totals
 }
 
+// projection_kernel for instances of up to NV segments per CTA of the cluster
+// (projection() has the rule): the same sums in the same order, arranged for
+// latency. The unit of work is one warp of a segment's 512 threads: the cluster's
+// warps share an instance's 16 x (segments) units, a thread keeps its cells of a
+// unit in registers from the load to the store, and each unit's double-f32 total
+// goes straight into every CTA's shared memory (st.async on a barrier; no
+// cluster-wide barrier between the passes). One warp per segment then adds the
+// segment's 16 totals in the block tree's order, one thread the segments' in f64.
+// A projection is a chain of three such passes: one 100 x 60 grid took 34 K
+// cycles with segments as units, cells in shared memory and two cluster barriers
+// a pass (17 us); 0 us this way, 256 x 256: 29 and 0, 64 x 128 x 128: 23 and 0.
+__device__ __forceinline__ uint32_t peer_smem(const void* p, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(tc::smem_u32(p)), "r"(rank));
+    return a;
+}
+
+constexpr int kProjUnits = kProjThreads / 32;  // units of a segment
+
+template <int NV>
+__global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, const InstDev* inst, ProjSlot* slots,
+                                                                        int init, int seg_cap, int* err) {
+    extern __shared__ __align__(16) float4 xch[];  // [3][16 seg_cap]: per pass, the units' totals (a.hi, a.lo, b.hi, b.lo)
+    __shared__ uint64_t bar[3];
+    __shared__ double segtot[NV * kProjCluster][2];
+    __shared__ double tot[2];
+    __shared__ float bc;
+    __shared__ volatile int failed;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), ii = blockIdx.x / cs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 3; i++) tc::mbar_init(&bar[i], 1);
+        tc::fence_barrier_init();
+        failed = 0;
+    }
+    cluster.sync();  // every CTA's barriers exist
+    JC_PDL_ENTRY;
+    const InstDev& I = inst[ii];
+    if (I.flags & 4u) return;  // no projection and no energy record for this instance (the whole cluster)
+    ProjSlot& S = I.slot ? *I.slot : slots[ii];
+    float* s = I.state;
+    const unsigned flags = init ? 0u : I.flags;
+    const int n = I.nx * I.ny, nseg = (n + kProjSeg - 1) / kProjSeg, nu = nseg * kProjUnits;
+    const int u0 = nu * rank / cs, u1 = nu * (rank + 1) / cs;
+    constexpr int kPer = kProjSeg / kProjThreads;  // cells of a thread in a unit
+    float H[NV][kPer], U[NV][kPer], V[NV][kPer];
+    int i0[NV];  // this thread's first cell of each of its units (past the last cell: no unit); cell k is 512 k further
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        const int u = u0 + warp + kProjUnits * q;
+        i0[q] = u < u1 ? u / kProjUnits * kProjSeg + (u % kProjUnits) * 32 + lane : n;
+    }
+#pragma unroll
+    for (int q = 0; q < NV; q++)
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            const int i = i0[q] + k * kProjThreads;
+            const bool in = i < n;
+            H[q][k] = in ? s[i] : 0.f;
+            U[q][k] = in ? s[n + i] : 0.f;
+            V[q][k] = in ? s[2 * (long long)n + i] : 0.f;
+        }
+    double prev = 0.0, mass0 = 0.0;
+    if (threadIdx.x == 0) {
+        prev = S.energy;
+        mass0 = S.mass0;
+        for (int i = 0; i < 3; i++) tc::mbar_expect_tx(&bar[i], (uint32_t)nu * 16);
+    }
+    // Kahan sums of term(q, k) -> (a, b) over each unit of this warp, every CTA's
+    // copy of all units' totals, then the instance totals in tot[] (thread 0)
+    auto reduce = [&](int ps, auto&& term) {
+        float4* mine = xch + (size_t)ps * seg_cap * kProjUnits;
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            const int u = u0 + warp + kProjUnits * q;
+            if (u >= u1) continue;
+            Kahan a, b;
+            a.init();
+            b.init();
+#pragma unroll
+            for (int k = 0; k < kPer; k++)
+                if (i0[q] + k * kProjThreads < n) {
+                    float ta, tb;
+                    term(q, k, ta, tb);
+                    a.add(ta);
+                    b.add(tb);
+                }
+            DF A = warp_sum_df(DF{a.s, -a.c}), B = warp_sum_df(DF{b.s, -b.c});
+            A.hi = __shfl_sync(0xffffffffu, A.hi, 0);
+            A.lo = __shfl_sync(0xffffffffu, A.lo, 0);
+            B.hi = __shfl_sync(0xffffffffu, B.hi, 0);
+            B.lo = __shfl_sync(0xffffffffu, B.lo, 0);
+            if (lane < cs)
+                asm volatile(
+                    "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                        peer_smem(mine + u, lane)),
+                    "f"(A.hi), "f"(A.lo), "f"(B.hi), "f"(B.lo), "r"(peer_smem(&bar[ps], lane))
+                    : "memory");
+        }
+        const bool ok = tc::mbar_wait(&bar[ps], 0, err, &failed);
+        for (int g = warp; g < nseg && ok; g += kProjUnits) {
+            const float4 t = lane < kProjUnits ? mine[g * kProjUnits + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const DF A = warp_sum_df(DF{t.x, t.y}), B = warp_sum_df(DF{t.z, t.w});
+            if (lane == 0) {
+                segtot[g][0] = (double)A.hi + (double)A.lo;
+                segtot[g][1] = (double)B.hi + (double)B.lo;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t[2] = {0.0, 0.0};
+            for (int g = 0; g < nseg; g++) {
+                t[0] += segtot[g][0];
+                t[1] += segtot[g][1];
+            }
+            tot[0] = t[0];
+            tot[1] = t[1];
+        }
+    };
+    // pass 1: mass
+    double M = 0.0;
+    if (init || (flags & 1u))
+        reduce(0, [&](int q, int k, float& a, float& b) {
+            a = H[q][k];
+            b = 0.f;
+        });
+    if (threadIdx.x == 0) {
+        if (init || (flags & 1u)) M = tot[0];
+        bc = (flags & 1u) ? (float)(mass0 - M / (double)n) : 0.0f;
+    }
+    __syncthreads();
+    // pass 2: mass shift, then potential and kinetic energy
+    const float delta = bc;
+    reduce(1, [&](int q, int k, float& pot, float& kin) {
+        if (flags & 1u) H[q][k] = __fadd_rn(H[q][k], delta);
+        pk_terms(d, H[q][k], U[q][k], V[q][k], pot, kin);
+    });
+    if (flags & 2u) {
+        // pass 3: energy scale of (u, v), then the energy of the stored state
+        double sc = 1.0;
+        if (threadIdx.x == 0) {
+            const double bound = prev * (double)d.energy_r_max;
+            double budget = bound - tot[0];
+            if (!(budget > 0.0)) budget = 0.0;
+            const double K = tot[1] > 1e-12 ? tot[1] : 1e-12;
+            if (!(budget >= K)) {  // else the square root is at least 1 and is clamped to it
+                sc = sqrt(budget / K);
+                sc = sc < 0.0 ? 0.0 : (sc > 1.0 ? 1.0 : sc);
+            }
+            bc = (float)sc;
+        }
+        __syncthreads();
+        const float s32 = bc;
+        reduce(2, [&](int q, int k, float& pot, float& kin) {
+            float u = __fadd_rn(__fmul_rn(U[q][k], d.norm_std[1]), d.norm_mean[1]);
+            float v = __fadd_rn(__fmul_rn(V[q][k], d.norm_std[2]), d.norm_mean[2]);
+            u = __fdiv_rn(__fsub_rn(__fmul_rn(u, s32), d.norm_mean[1]), d.norm_std[1]);
+            v = __fdiv_rn(__fsub_rn(__fmul_rn(v, s32), d.norm_mean[2]), d.norm_std[2]);
+            U[q][k] = u;
+            V[q][k] = v;
+            pk_terms(d, H[q][k], u, v, pot, kin);
+        });
+        if (rank == 0 && threadIdx.x == 0) S.last_scale = sc;
+    }
+#pragma unroll
+    for (int q = 0; q < NV; q++)
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            const int i = i0[q] + k * kProjThreads;
+            if (i >= n) continue;
+            if (flags & 1u) s[i] = H[q][k];
+            if (flags & 2u) {
+                s[n + i] = U[q][k];
+                s[2 * (long long)n + i] = V[q][k];
+            }
+        }
+    if (rank == 0 && threadIdx.x == 0) {
+        const double E = tot[0] + tot[1];
+        if (init) {
+            S.mass0 = M / (double)n;
+            S.energy = E;
+            S.max_viol = 0.0;
+            S.last_scale = 1.0;
+        } else {
+            const double viol = (E - prev * (double)d.energy_r_max) / prev;
+            if (viol > S.max_viol) S.max_viol = viol;
+            S.energy = E;
+        }
+    }
+}
+
 }  // namespace f32k
 
 template <class T, class AL, class EP>
@@ -884,14 +1077,33 @@ void conv2_step(const Dims& d, const float* c1, const WeightsF32& w, const Pack&
     check_launch(name);
 }
 
+template <int NV>
+static void projection_units(const Dims& d, const Pack& p, int init, int cs, int nseg, cudaStream_t s) {
+    const size_t smem = (size_t)3 * nseg * f32k::kProjUnits * sizeof(float4);
+    cuda_check_attr(launch_pdl(f32k::projection_units_kernel<NV>, dim3((unsigned)(p.n_inst * cs)), dim3(f32k::kProjThreads),
+                               smem, s, (unsigned)cs, d, (const InstDev*)p.inst, p.proj, init, nseg, p.err));
+    check_launch("projection");
+}
+
 void projection(const Dims& d, const Pack& p, int init, cudaStream_t s) {
     KScope k("projection", s);
+    const long long nseg = (p.max_inst_cells + f32k::kProjSeg - 1) / f32k::kProjSeg;
+    // Cells in registers while a thread has two units at most (16 segments of
+    // 4096 cells in a cluster of eight: 256 x 256 cells; four would not fit the
+    // registers); the largest cluster that leaves the CTAs two to an SM, since a
+    // CTA's own work is what a pass waits for.
+    if (nseg <= 2 * f32k::kProjCluster && p.err) {
+        int cs = 1;
+        while (cs < f32k::kProjCluster && ((long long)p.n_inst * cs <= 152 || nseg > 2 * cs)) cs *= 2;
+        if (nseg <= cs) projection_units<1>(d, p, init, cs, (int)nseg, s);
+        else projection_units<2>(d, p, init, cs, (int)nseg, s);
+        return;
+    }
     static std::atomic<unsigned long long> attr{0};
     set_smem_per_device(f32k::projection_kernel, 200 * 1024, attr);
     // cluster size: the smallest whose slices fit in shared memory, and about
     // one CTA per SM (152 here) when the instances are few; the sums do not
     // depend on it (segment totals in segment order)
-    const long long nseg = (p.max_inst_cells + f32k::kProjSeg - 1) / f32k::kProjSeg;
     int cs = 1;
     while (cs < f32k::kProjCluster && (nseg + cs - 1) / cs * f32k::kProjSeg > f32k::kProjSmemCells) cs *= 2;
     while (cs < f32k::kProjCluster && (long long)p.n_inst * cs < 152 && nseg >= 2LL * cs) cs *= 2;
