@@ -153,7 +153,15 @@ class Model {
     float* d_inc_ = nullptr;
     double* d_energies_ = nullptr;
     int energies_cap_ = 0;
-    float* h_pinned_ = nullptr;  // staging for host calls: state | out | meta
+    float* h_pinned_ = nullptr;  // staging for host calls: state | meta (64) | out, wait flag
+    // forward_host / step_host: buffers, descriptor and captured calls (by tick
+    // mode and autotuning switch)
+    float *d_host_in_ = nullptr, *d_host_out_ = nullptr;
+    Pack host_pack_{};
+    int host_calls_ = 0;
+    std::map<std::pair<int, int>, cudaGraphExec_t> host_graphs_;
+    void enqueue_host(int mode);
+    void host_call(const float* state, const float* meta, float* out, int mode);
     void put_instance(float* state, float* out, const float* meta, uint32_t flags, cudaStream_t s);
     void enqueue_rollout(int ticks, double* d_energies_out, float* d_traj, cudaStream_t s);
     struct GraphKey {
