@@ -1501,25 +1501,6 @@ constexpr int kPMX = kPMD * 512;             // bytes of a tile's residual rows
 constexpr int kPMOffX = kPMD * 256, kPMOffW = kPMOffX + 2 * kPMX;
 constexpr int kPMSmem = kPMOffW + kPMSlots * kPMBlock;
 
-__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
-    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\t"
-        "mov.b64 {%0, %1}, a;\n\t}"
-        : "+f"(a.x), "+f"(a.y)
-        : "f"(b.x), "f"(b.y));
-    return a;
-}
-__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
-    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tmul.rn.f32x2 a, a, b;\n\t"
-        "mov.b64 {%0, %1}, a;\n\t}"
-        : "+f"(a.x), "+f"(a.y)
-        : "f"(b.x), "f"(b.y));
-    return a;
-}
-__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
-    fma2_f32(c.x, c.y, a.x, a.y, b.x, b.y);
-    return c;
-}
-
 // The logical output column in column p of the weights arranged for
 // tc_proj_mlp_kernel (fragment groups 2 m and 2 m + 1 give a thread columns 2 j,
 // 2 j + 1 of each).

@@ -67,6 +67,28 @@ __device__ __forceinline__ void fma2_f32(float& d0, float& d1, float a0, float a
         : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
 
+// Two lanes at once, each rounded like the scalar operation.
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a.x), "+f"(a.y)
+        : "f"(b.x), "f"(b.y));
+    return a;
+}
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tmul.rn.f32x2 a, a, b;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a.x), "+f"(a.y)
+        : "f"(b.x), "f"(b.y));
+    return a;
+}
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+    fma2_f32(c.x, c.y, a.x, a.y, b.x, b.y);
+    return c;
+}
+// a - b, as b times -1 + a in one rounding
+__device__ __forceinline__ float2 sub_f32x2(float2 a, float2 b) { return fma_f32x2(b, make_float2(-1.f, -1.f), a); }
+
 // Index of the instance owning token row r: the last i with inst[i].row0 <= r.
 __device__ __forceinline__ int inst_of_row(const InstDev* inst, int n, int r) {
     int lo = 0, hi = n - 1;
@@ -121,6 +143,10 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool vali
 __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
                  "l"(src), "r"(valid ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
 // Waits for every copy this thread issued (a __syncthreads() must follow

@@ -21,20 +21,17 @@ namespace ev {
 
 // ---- solver: shallow_water.rs:149-238 ---------------------------------------
 
-constexpr int kSwTX = 64, kSwTY = 32;     // output tile
-constexpr int kSwThreads = 512;           // 4 cells per thread
-constexpr int kSwPX = kSwTX + 4, kSwPY = kSwTY + 4;  // inputs with a 2-cell apron
-constexpr int kSwNX = kSwTX + 2, kSwNY = kSwTY + 2;  // new depth with a 1-cell apron
-
 struct SwDev {
     int nx, ny;
     float r, dt, g, nu, inv2dx, invdx2;
+    float nzero;  // -0, at run time only (see mul2)
 };
 
 SwDev sw_dev(const jc_sw_params& p) {
     SwDev d;
     d.nx = p.nx;
     d.ny = p.ny;
+    d.nzero = -0.0f;
     d.r = p.dt / p.dx;                     // shallow_water.rs:175
     d.dt = p.dt;
     d.g = p.g;
@@ -44,124 +41,218 @@ SwDev sw_dev(const jc_sw_params& p) {
     return d;
 }
 
-// Face flux 0.5 (h_a + h_b) 0.5 (q_a + q_b), rounded step by step in the
-// order shallow_water.rs:160,169 evaluates it.
-__device__ __forceinline__ float face_flux(float ha, float hb, float qa, float qb) {
-    return __fmul_rn(__fmul_rn(__fmul_rn(0.5f, __fadd_rn(ha, hb)), 0.5f), __fadd_rn(qa, qb));
+// The rounded products of two pairs, as a b + (-0) with a zero that the compiler
+// does not know: it merges a paired product and the paired sum that follows into
+// one rounding, explicit rounding or not.
+__device__ __forceinline__ float2 mul2(const SwDev& p, float2 a, float2 b) {
+    return fma_f32x2(a, b, make_float2(p.nzero, p.nzero));
 }
 
-struct SwSmem {
-    float h[kSwPY][kSwPX + 1], u[kSwPY][kSwPX + 1], v[kSwPY][kSwPX + 1];
-    float hn[kSwNY][kSwNX + 1];
+// Face fluxes 0.5 (h_a + h_b) 0.5 (q_a + q_b) of two faces, rounded step by step
+// in the order shallow_water.rs:160,169 evaluates them.
+__device__ __forceinline__ float2 face_flux(const SwDev& p, float2 ha, float2 hb, float2 qa, float2 qb) {
+    const float2 half = make_float2(0.5f, 0.5f);
+    return mul2(p, mul2(p, mul2(p, half, add_f32x2(ha, hb)), half), add_f32x2(qa, qb));
+}
+
+// One solver step as a pipeline of rows: push(r) takes row r of a lane's two
+// neighbouring columns (x, y) and leaves the stepped row r - 2 in oh, ou, ov.
+// Continuity in flux form (zero flux through the walls) at row r - 1, then
+// momentum at row r - 2 on the new surface with mirrored ghost cells (h even,
+// normal velocity odd, tangential velocity even). A face between two columns or
+// two rows is computed once; a lane's neighbours to either side come by
+// shuffles; the two columns' arithmetic is paired (each lane of a pair rounds
+// like the scalar operation; -a - b is taken as -(a + b), the same value).
+// Rows above the first pushed one are unknown, so the first two results are
+// good only if that row is row 0; likewise the warp's two outermost columns on
+// a side that is not a wall.
+struct SwStage {
+    float2 h, u, v;           // row r - 1
+    float2 u1, v1, hn1;       // row r - 2: velocities, new depth
+    float2 u2, v2, hn2;       // row r - 3
+    float2 fy;                // flux between rows r - 2 and r - 1
+    float ul, ul1;            // the left neighbour's u in rows r - 1, r - 2
+    float2 oh, ou, ov;
+
+    __device__ __forceinline__ void push(const SwDev& p, int r, float2 H, float2 U, float2 V, bool wall_l, bool wall_r0,
+                                         bool wall_r1) {
+        const unsigned all = 0xffffffffu;
+        const float2 i2dx = make_float2(p.inv2dx, p.inv2dx), idx2 = make_float2(p.invdx2, p.invdx2);
+        auto dup = [](float a) { return make_float2(a, a); };
+        // continuity at row r - 1 (shallow_water.rs:160-181)
+        const float hl = __shfl_up_sync(all, h.y, 1);
+        float2 fl = face_flux(p, make_float2(hl, h.x), h, make_float2(ul, u.x), u);  // left faces of the two columns
+        if (wall_l) fl.x = 0.f;
+        if (wall_r0) fl.y = 0.f;
+        const float f2 = __shfl_down_sync(all, fl.x, 1);
+        const float2 fr = make_float2(fl.y, wall_r1 ? 0.f : f2);
+        float2 up = face_flux(p, h, H, v, V);
+        // the walls above and below: branches that the whole warp takes alike
+        if (r == 1) fy = dup(0.f);
+        if (r == p.ny) up = dup(0.f);
+        const float2 hn = sub_f32x2(h, mul2(p, dup(p.r), add_f32x2(sub_f32x2(fr, fl), sub_f32x2(up, fy))));
+        fy = up;
+        // momentum at row r - 2, centred differences on the new surface (:188-232)
+        if (r == 2) {
+            hn2 = hn1;
+            u2 = u1;
+            v2 = make_float2(-v1.x, -v1.y);
+        }
+        float2 hu = hn, uu = u, vu = v;
+        if (r == p.ny + 1) {
+            hu = hn1;
+            uu = u1;
+            vu = make_float2(-v1.x, -v1.y);
+        }
+        const float hnl = __shfl_up_sync(all, hn1.y, 1), hnr = __shfl_down_sync(all, hn1.x, 1);
+        const float ur1 = __shfl_down_sync(all, u1.x, 1);
+        const float vl1 = __shfl_up_sync(all, v1.y, 1), vr1 = __shfl_down_sync(all, v1.x, 1);
+        const float2 hL = make_float2(wall_l ? hn1.x : hnl, hn1.x);
+        const float2 hR = make_float2(wall_r0 ? hn1.x : hn1.y, wall_r1 ? hn1.y : hnr);
+        const float2 uL = make_float2(wall_l ? -u1.x : ul1, u1.x);
+        const float2 uR = make_float2(wall_r0 ? -u1.x : u1.y, wall_r1 ? -u1.y : ur1);
+        const float2 vL = make_float2(wall_l ? v1.x : vl1, v1.x);
+        const float2 vR = make_float2(wall_r0 ? v1.x : v1.y, wall_r1 ? v1.y : vr1);
+        auto diff = [&](float2 a, float2 b) { return mul2(p, sub_f32x2(a, b), i2dx); };
+        auto lap = [&](float2 l, float2 rr, float2 d, float2 t, float2 c) {
+            return mul2(p, sub_f32x2(add_f32x2(add_f32x2(add_f32x2(l, rr), d), t), mul2(p, dup(4.0f), c)), idx2);
+        };
+        const float2 tu = sub_f32x2(mul2(p, dup(p.nu), lap(uL, uR, u2, uu, u1)),
+                                    add_f32x2(add_f32x2(mul2(p, u1, diff(uR, uL)), mul2(p, v1, diff(uu, u2))),
+                                              mul2(p, dup(p.g), diff(hR, hL))));
+        const float2 tv = sub_f32x2(mul2(p, dup(p.nu), lap(vL, vR, v2, vu, v1)),
+                                    add_f32x2(add_f32x2(mul2(p, u1, diff(vR, vL)), mul2(p, v1, diff(vu, v2))),
+                                              mul2(p, dup(p.g), diff(hu, hn2))));
+        oh = hn1;
+        ou = add_f32x2(u1, mul2(p, dup(p.dt), tu));
+        ov = add_f32x2(v1, mul2(p, dup(p.dt), tv));
+        ul1 = ul;
+        ul = __shfl_up_sync(all, U.y, 1);
+        u2 = u1;
+        v2 = v1;
+        hn2 = hn1;
+        u1 = u;
+        v1 = v;
+        hn1 = hn;
+        h = H;
+        u = U;
+        v = V;
+    }
 };
 
-// One forward-backward step of every state: continuity in flux form (zero
-// flux through the walls), then momentum on the new surface with mirrored
-// ghost cells (h even, normal velocity odd, tangential velocity even).
-// grid (x tiles, y tiles, states); src and dst are [states][3][ny][nx]. A
-// 64x32 tile per CTA keeps enough loads in flight per SM to cover the DRAM
-// latency (the step is a pure stream: 12 bytes read and 12 written per cell).
-__global__ void __launch_bounds__(kSwThreads)
-sw_step_kernel(SwDev p, const float* __restrict__ src, float* __restrict__ dst) {
-    __shared__ SwSmem sm;
-    const int nx = p.nx, ny = p.ny;
-    const long long n = (long long)nx * ny;
-    const float* H = src + (long long)blockIdx.z * 3 * n;
-    const float* U = H + n;
-    const float* V = U + n;
-    const int x0 = blockIdx.x * kSwTX, y0 = blockIdx.y * kSwTY;
-    const int tid = threadIdx.x;
-    // inputs on [y0-2, y0+TY+2) x [x0-2, x0+TX+2); apron positions outside
-    // the grid hold a clamped neighbour and are never read below. Thread t
-    // keeps column t % kSwPX and walks rows t / kSwPX, + kLoadRows, ...
-    constexpr int kLoadRows = kSwThreads / kSwPX;  // 7 rows per pass
-    if (tid < kLoadRows * kSwPX) {
-        const int lx = tid % kSwPX;
-        const int gx = min(max(x0 - 2 + lx, 0), nx - 1);
+// STEPS forward-backward steps of every state; src and dst are [states][3][ny][nx].
+// A warp takes 64 columns of a band of rows, two columns a lane, and walks down
+// the rows through STEPS stages in registers; bands and columns overlap by the
+// 2 STEPS that a step's result reaches on each side that is not a wall. Two
+// steps a pass halve the memory traffic of a step (24 bytes a cell); the rows
+// in registers take a third of the shared-memory tile's instructions. 96 states
+// of 256 x 256: a step took 46 us with 64 x 32 shared-memory tiles, 39 us in
+// passes of one step and 34 us in passes of two (2.2 TB/s: what bounds it now is
+// instruction issue, 64% of the cycles; unrolled by 3, as many as the rows that
+// rotate through the registers, 570 us for 16 steps against 620 by 2).
+constexpr int kSwWarps = 1;  // warps share nothing: alone in their CTAs they fill the SMs evenly
+
+template <int STEPS>
+__global__ void __launch_bounds__(32 * kSwWarps) sw_rows_kernel(SwDev p, const float* __restrict__ src,
+                                                                float* __restrict__ dst, int strips, int bands,
+                                                                int band_rows, long long units, int vec) {
+    constexpr int A = 2 * STEPS;
+    const long long unit = (long long)blockIdx.x * kSwWarps + (threadIdx.x >> 5);
+    if (unit >= units) return;
+    const int lane = threadIdx.x & 31, nx = p.nx, ny = p.ny;
+    const int strip = (int)(unit % strips), band = (int)(unit / strips % bands);
+    const long long n = (long long)nx * ny, off = unit / ((long long)strips * bands) * 3 * n;
+    const int c0 = strip * (64 - 2 * A), x = c0 + 2 * lane;
+    const int ys = band * band_rows, ye = min(ys + band_rows, ny), r0 = max(0, ys - A);
+    // columns this warp stores
+    const int lo = strip > 0 ? c0 + A : 0, hi = strip + 1 < strips ? c0 + 64 - A : nx;
+    const bool s0 = x >= lo && x < hi && x < nx, s1 = x + 1 >= lo && x + 1 < hi && x + 1 < nx;
+    const bool wall_l = x == 0, wall_r0 = x == nx - 1, wall_r1 = x + 1 == nx - 1;
+    const int xa = min(x, nx - 1), xb = min(x + 1, nx - 1), xv = min(x, nx - 2);
+    const float* H = src + off;
+    // rows ahead in flight, each lane's own part (nothing to wait for but its own copies)
+    constexpr int kRing = 8, kAhead = 6;
+    __shared__ float2 ring[kSwWarps][kRing][3][32];
+    float2 (*rg)[3][32] = ring[threadIdx.x >> 5];
+    auto fetch = [&](int r) {
+        const float* q = H + (long long)min(r, ny - 1) * nx;
 #pragma unroll
-        for (int ly = tid / kSwPX; ly < kSwPY; ly += kLoadRows) {
-            const int gy = min(max(y0 - 2 + ly, 0), ny - 1);
-            const long long o = (long long)gy * nx + gx;
-            sm.h[ly][lx] = __ldg(H + o);
-            sm.u[ly][lx] = __ldg(U + o);
-            sm.v[ly][lx] = __ldg(V + o);
+        for (int a = 0; a < 3; a++, q += n) {
+            float2* to = &rg[r & (kRing - 1)][a][lane];
+            if (vec) {
+                cp_async8(to, q + xv);
+            } else {
+                cp_async4(&to->x, q + xa, true);
+                cp_async4(&to->y, q + xb, true);
+            }
+        }
+        cp_async_commit();
+    };
+    SwStage st[STEPS] = {};
+    for (int r = r0; r < r0 + kAhead; r++) fetch(r);
+    // the second stage takes the row that the first made in the iteration
+    // before, so that the two are independent within an iteration
+    constexpr int kLag = A + (STEPS - 1);
+#pragma unroll 3
+    for (int r = r0; r < ye + kLag; r++) {
+        fetch(r + kAhead);
+        cp_async_wait_group<kAhead>();
+        const float2 h = rg[r & (kRing - 1)][0][lane], u = rg[r & (kRing - 1)][1][lane], v = rg[r & (kRing - 1)][2][lane];
+        if (STEPS == 2) st[STEPS - 1].push(p, r - 3, st[0].oh, st[0].ou, st[0].ov, wall_l, wall_r0, wall_r1);
+        st[0].push(p, r, h, u, v, wall_l, wall_r0, wall_r1);
+        const int y = r - kLag;
+        if (y >= ys) {
+            const SwStage& o = st[STEPS - 1];
+            float* D = dst + off + (long long)y * nx + x;
+            if (vec && s0 && s1) {
+                *reinterpret_cast<float2*>(D) = o.oh;
+                *reinterpret_cast<float2*>(D + n) = o.ou;
+                *reinterpret_cast<float2*>(D + 2 * n) = o.ov;
+            } else {
+                if (s0) {
+                    D[0] = o.oh.x;
+                    D[n] = o.ou.x;
+                    D[2 * n] = o.ov.x;
+                }
+                if (s1) {
+                    D[1] = o.oh.y;
+                    D[n + 1] = o.ou.y;
+                    D[2 * n + 1] = o.ov.y;
+                }
+            }
         }
     }
-    __syncthreads();
-    // continuity on the tile and its 1-cell apron (cells inside the grid);
-    // thread t keeps column t % kSwNX
-    constexpr int kContRows = kSwThreads / kSwNX;  // 7 rows per pass
-    if (tid < kContRows * kSwNX) {
-        const int lx = tid % kSwNX;
-        const int gx = x0 - 1 + lx;
-        const bool xin = gx >= 0 && gx < nx;
-        const bool wl = gx == 0, wr = gx == nx - 1;
-        const int sx = lx + 1;
-        for (int ly = tid / kSwNX; ly < kSwNY; ly += kContRows) {
-            const int gy = y0 - 1 + ly;
-            if (!xin || gy < 0 || gy >= ny) continue;
-            const int sy = ly + 1;
-            const float h = sm.h[sy][sx];
-            const float fxl = wl ? 0.f : face_flux(sm.h[sy][sx - 1], h, sm.u[sy][sx - 1], sm.u[sy][sx]);
-            const float fxr = wr ? 0.f : face_flux(h, sm.h[sy][sx + 1], sm.u[sy][sx], sm.u[sy][sx + 1]);
-            const float fyl = gy == 0 ? 0.f : face_flux(sm.h[sy - 1][sx], h, sm.v[sy - 1][sx], sm.v[sy][sx]);
-            const float fyr = gy == ny - 1 ? 0.f : face_flux(h, sm.h[sy + 1][sx], sm.v[sy][sx], sm.v[sy + 1][sx]);
-            sm.hn[ly][lx] = __fsub_rn(h, __fmul_rn(p.r, __fadd_rn(__fsub_rn(fxr, fxl), __fsub_rn(fyr, fyl))));
+}
+
+template <int STEPS>
+static void sw_pass(const SwDev& p, const float* src, float* dst, int count, cudaStream_t s) {
+    KScope k("sw_step", s);
+    constexpr int A = 2 * STEPS;
+    const int strips = p.nx <= 64 ? 1 : (p.nx - 2 * A + (64 - 2 * A) - 1) / (64 - 2 * A);
+    // Rows of a band: a band computes about 2 A rows more than it stores, and the
+    // launch lasts as many rounds of bands as its warps fill the SMs (152, with 14
+    // or 20 warps by their registers): the height with the fewest rows in all.
+    const long long slots = 152LL * (STEPS == 2 ? 14 : 20);
+    int band_rows = p.ny;
+    long long least = -1;
+    for (int rows = 8; rows <= 256; rows += 4) {
+        const int nb = (p.ny + rows - 1) / rows, even = (p.ny + nb - 1) / nb;
+        const long long rounds = ((long long)count * strips * nb + slots - 1) / slots, cost = rounds * (even + 2 * A + 6);
+        if (least < 0 || cost < least) {
+            least = cost;
+            band_rows = even;
         }
     }
-    __syncthreads();
-    float* D = dst + (long long)blockIdx.z * 3 * n;
-    // momentum, centred differences on the new surface (:188-232); thread t
-    // keeps column t % kSwTX and takes rows t / kSwTX, + 8, ...
-    const int tx = tid % kSwTX;
-    const int gx = x0 + tx;
-    const int sx = tx + 2, qx = tx + 1;  // in h, u, v / in hn
-    const int dxm = gx == 0 ? 0 : -1, dxp = gx == nx - 1 ? 0 : 1;
-    const float sxm = gx == 0 ? -1.f : 1.f, sxp = gx == nx - 1 ? -1.f : 1.f;
-#pragma unroll
-    for (int c = 0; c < (kSwTX * kSwTY) / kSwThreads; c++) {
-        const int ty = tid / kSwTX + c * (kSwThreads / kSwTX);
-        const int gy = y0 + ty;
-        if (gx >= nx || gy >= ny) continue;
-        const int sy = ty + 2, qy = ty + 1;
-        const int dym = gy == 0 ? 0 : -1, dyp = gy == ny - 1 ? 0 : 1;
-        const float sym = gy == 0 ? -1.f : 1.f, syp = gy == ny - 1 ? -1.f : 1.f;
-        const float hl = sm.hn[qy][qx + dxm], hr = sm.hn[qy][qx + dxp];
-        const float hd = sm.hn[qy + dym][qx], hu = sm.hn[qy + dyp][qx];
-        const float ul = __fmul_rn(sxm, sm.u[sy][sx + dxm]), ur = __fmul_rn(sxp, sm.u[sy][sx + dxp]);
-        const float ud = sm.u[sy + dym][sx], uu = sm.u[sy + dyp][sx];
-        const float vl = sm.v[sy][sx + dxm], vr = sm.v[sy][sx + dxp];
-        const float vd = __fmul_rn(sym, sm.v[sy + dym][sx]), vu = __fmul_rn(syp, sm.v[sy + dyp][sx]);
-        const float u0 = sm.u[sy][sx], v0 = sm.v[sy][sx];
-        const float dudx = __fmul_rn(__fsub_rn(ur, ul), p.inv2dx), dudy = __fmul_rn(__fsub_rn(uu, ud), p.inv2dx);
-        const float dvdx = __fmul_rn(__fsub_rn(vr, vl), p.inv2dx), dvdy = __fmul_rn(__fsub_rn(vu, vd), p.inv2dx);
-        const float dhdx = __fmul_rn(__fsub_rn(hr, hl), p.inv2dx), dhdy = __fmul_rn(__fsub_rn(hu, hd), p.inv2dx);
-        const float lap_u =
-            __fmul_rn(__fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(ul, ur), ud), uu), __fmul_rn(4.0f, u0)), p.invdx2);
-        const float lap_v =
-            __fmul_rn(__fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(vl, vr), vd), vu), __fmul_rn(4.0f, v0)), p.invdx2);
-        const float tu = __fadd_rn(
-            __fsub_rn(__fsub_rn(__fmul_rn(-u0, dudx), __fmul_rn(v0, dudy)), __fmul_rn(p.g, dhdx)),
-            __fmul_rn(p.nu, lap_u));
-        const float tv = __fadd_rn(
-            __fsub_rn(__fsub_rn(__fmul_rn(-u0, dvdx), __fmul_rn(v0, dvdy)), __fmul_rn(p.g, dhdy)),
-            __fmul_rn(p.nu, lap_v));
-        const long long o = (long long)gy * nx + gx;
-        D[o] = sm.hn[qy][qx];
-        D[n + o] = __fadd_rn(u0, __fmul_rn(p.dt, tu));
-        D[2 * n + o] = __fadd_rn(v0, __fmul_rn(p.dt, tv));
-    }
+    const int bands = (p.ny + band_rows - 1) / band_rows;
+    const long long units = (long long)count * strips * bands;
+    const int vec = p.nx % 2 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 7) == 0;
+    sw_rows_kernel<STEPS><<<(unsigned)((units + kSwWarps - 1) / kSwWarps), 32 * kSwWarps, 0, s>>>(p, src, dst, strips, bands,
+                                                                                             band_rows, units, vec);
+    cuda_check(cudaGetLastError(), "sw_step launch");
 }
 
 void sw_step(const SwDev& p, const float* src, float* dst, int count, cudaStream_t s) {
-    KScope k("sw_step", s);
-    const int gx = (p.nx + kSwTX - 1) / kSwTX, gy = (p.ny + kSwTY - 1) / kSwTY;
-    const long long stride = 3LL * p.nx * p.ny;
-    for (int c0 = 0; c0 < count; c0 += 65535) {
-        const int c = std::min(65535, count - c0);
-        sw_step_kernel<<<dim3(gx, gy, c), kSwThreads, 0, s>>>(p, src + c0 * stride, dst + c0 * stride);
-    }
-    cuda_check(cudaGetLastError(), "sw_step launch");
+    if (count > 0) sw_pass<1>(p, src, dst, count, s);
 }
 
 void check_params(const jc_sw_params& p) {
@@ -177,8 +268,15 @@ void check_params(const jc_sw_params& p) {
 void sw_run(const SwDev& d, float* states, float* scratch, int count, int steps, cudaStream_t s) {
     float* a = states;
     float* b = scratch;
-    for (int t = 0; t < steps; t++) {
-        sw_step(d, a, b, count, s);
+    // passes of two steps, and an even number of passes where that can be (the
+    // result is then in place: a copy costs more than a pass of one step)
+    int passes = (steps + 1) / 2;
+    if (passes % 2 && steps > 1) passes++;
+    for (int left = steps; left > 0; passes--) {
+        const bool two = left > passes;
+        if (two) sw_pass<2>(d, a, b, count, s);
+        else sw_pass<1>(d, a, b, count, s);
+        left -= two ? 2 : 1;
         std::swap(a, b);
     }
     if (a != states)

@@ -779,7 +779,7 @@ projection_kernel(Dims d, const InstDev* inst, ProjSlot* slots, int init, int ca
 // segment's 16 totals in the block tree's order, one thread the segments' in f64.
 // A projection is a chain of three such passes: one 100 x 60 grid took 34 K
 // cycles with segments as units, cells in shared memory and two cluster barriers
-// a pass (17 us); 0 us this way, 256 x 256: 29 and 0, 64 x 128 x 128: 23 and 0.
+// a pass (17 us); 10 us this way, 256 x 256: 29 and 20, 64 x 128 x 128: 23 and 15.
 __device__ __forceinline__ uint32_t peer_smem(const void* p, int rank) {
     uint32_t a;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(tc::smem_u32(p)), "r"(rank));
