@@ -75,12 +75,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Waits for the phase with the given parity to complete. Returns false (and
 // sets *err) when the wait exceeds limit_ns (kWaitNs unless a caller passes
-// a shorter limit); a wait that already failed in this CTA returns false at
-// once.
+// a shorter limit); once a wait has failed in this CTA, one that would have to
+// wait returns false at once. The barrier is asked first: looking at the flag
+// before it added 70 cycles to each wait, most of which find the phase complete.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, volatile int* cta_failed,
                                           unsigned long long limit_ns = kWaitNs) {
-    if (*cta_failed) return false;
     if (mbar_try_wait(bar, parity)) return true;
+    if (*cta_failed) return false;
     const unsigned long long t0 = globaltimer();
     while (true) {
         if (mbar_try_wait(bar, parity)) return true;
