@@ -1462,50 +1462,56 @@ __device__ __forceinline__ bool all_of(bool v, int bar, int n) {
 // Wp + bp, A = LN2(x), x += gelu(A @ W1 + b1) @ W2 + b2, ln = LN(x) for the next
 // step. Persistent: one CTA per SM walks 128-row tiles, its stages on separate
 // warps:
-//   0-7  the row work: both residual + LayerNorms and the GELUs;
-//   8    (one lane) loads the weights in 16 KB blocks, in the order the MMAs
+//   0-15 the row work: both residual + LayerNorms and the GELUs;
+//   16   (one lane) loads the weights in 16 KB blocks, in the order the MMAs
 //        take them, into a ring of kPMSlots slots, tiles ahead included;
-//   9    (one lane) issues every MMA;
-//   10   (one lane) loads the attention and residual rows, a tile ahead, and
+//   17   (one lane) issues every MMA;
+//   18   (one lane) loads the attention and residual rows, a tile ahead, and
 //        stores each tile's rows.
 // The hidden columns go through in chunks of 128: S_c = A @ W1_c into one of two
 // TMEM accumulators, h_c = gelu(S_c + b1_c) rounded to bf16 back over S_c's own
 // columns (a thread holds all it reads before it writes), O += h_c @ W2_c with
 // h_c as the MMA's A operand straight from TMEM. S_{c+1} runs while the row
 // warps work on S_c, and the next tile's projection P, in the accumulator that
-// chunk n - 2 has left, while they work on the last chunk: they wait for an MMA
-// only at the two ends of a tile. A (packed bf16) lies in TMEM too. The residual
-// rows stay in the row warps' registers from one LayerNorm to the other (64 of
-// 168); they come and go through two shared-memory buffers, tiles alternating
-// (an SM writes about 30 bytes a cycle: stored by the row warps themselves the
-// 64 KB held them 2500 cycles a tile).
-// The residual + LayerNorm rows are read from TMEM as 16 x 8 fragments: a warp
-// owns 16 rows and a row lies in four lanes. Wp's and W2's output columns are
-// stored in the order (pm_column) that gives lane j of the four the columns 16 m
-// + 4 j .. + 3: it moves its part of a row as float4s, and a row's sum takes two
-// shuffles, where a row spread over a warp takes five (and the fragments'
-// own column order 17). The arithmetic and its order are those of
-// rows_resid_ln_t (D = 128), so every form gives the same bits. The MMAs' K
-// order is that of tc_mlp_serial_kernel.
-// What bounds it: the GELUs' MUFU operations (two for each of 65,536 hidden
-// values a tile, 8192 cycles) and the row work around them. At 64 K rows:
-// 76 us a launch for the form before it (two CTAs per SM, one accumulator, the
-// chunk through shared memory, CTA barriers around every step), 51 for this one;
-// a tile alone on its SM: 28 and 16 us. A tile's 19.4 K cycles: the four chunks'
-// GELUs 9.8 K, S_0 1.4 K, the last O 1.5 K, the LayerNorms 2.3 K and 2.8 K.
-constexpr int kPMThreads = 11 * 32;
+// chunk n - 2 has left, while they work on the last LayerNorm: they wait for an
+// MMA only at the two ends of a tile. A (packed bf16) lies in TMEM too. The
+// residual rows stay in the row warps' registers from one LayerNorm to the other;
+// they come and go through one shared-memory buffer: each thread takes the next
+// tile's values out of the places that it puts this tile's in. That leaves the
+// weights 112 KB (with two buffers of rows 48 KB, and a chunk's MMAs waited 650
+// cycles for each block). The rows leave by bulk copies (an SM writes about 30
+// bytes a cycle: stored by the row warps themselves the 64 KB held them 2500
+// cycles a tile).
+// The residual + LayerNorm rows are read from TMEM as 16 x 8 fragments: two warps
+// share 16 rows, half of the columns each, and a row lies in four lanes of each.
+// Wp's and W2's output columns are stored in the order (pm_column) that gives
+// lane j of the four the columns 16 m + 4 j .. + 3, m even in one warp and odd in
+// the other: it moves its part of a row as float4s, and a row's sum takes one
+// exchange between the warps and two shuffles, in tree32's order. The arithmetic
+// and its order are those of rows_resid_ln_t (D = 128), so every form gives the
+// same bits. The MMAs' K order is that of tc_mlp_serial_kernel.
+// What bounds it: the GELUs' MUFU operations (an ex2 at 32 and a reciprocal at 16
+// a cycle for each of 65,536 hidden values a tile, 6.1 K cycles) and, while they
+// wait, the row work around them, which shared memory's 128 bytes a cycle bound
+// (the rows' exchange alone 128 KB). At 64 K rows: 76 us a launch for the form
+// before it (two CTAs per SM, one accumulator, the chunk through shared memory,
+// CTA barriers around every step), 51 with 8 row warps and two row buffers, 46 for
+// this one; a tile alone on its SM 28, 17.5 and 16.5 us. A tile's 18.4 K cycles: the
+// four chunks' GELUs 8.9 K, S_0 1.1 K, the last O 1.1 K, the LayerNorms 2.0 K and
+// 2.2 K, the rows' exchange 1.4 K.
+constexpr int kPMRowWarps = 16, kPMThreads = (kPMRowWarps + 3) * 32;
 constexpr int kPMD = 128, kPMNC = 128;       // width; hidden columns per chunk
 constexpr int kPMBlock = 64 * kPMD * 2;      // bytes of a weight block: 64 hidden columns (or half of Wp's K)
-constexpr int kPMSlots = 3;
+constexpr int kPMSlots = 7;
 constexpr int kPMX = kPMD * 512;             // bytes of a tile's residual rows
-constexpr int kPMOffX = kPMD * 256, kPMOffW = kPMOffX + 2 * kPMX;
+constexpr int kPMOffX = kPMD * 256, kPMOffW = kPMOffX + kPMX;
 constexpr int kPMSmem = kPMOffW + kPMSlots * kPMBlock;
 
 // The logical output column in column p of the weights arranged for
-// tc_proj_mlp_kernel (fragment groups 2 m and 2 m + 1 give a thread columns 2 j,
-// 2 j + 1 of each).
+// tc_proj_mlp_kernel: the even 16-column groups, then the odd ones, and within a
+// group the order in which a fragment pair gives lane j of a row's four columns 4 j .. + 3.
 __host__ __device__ constexpr int pm_column(int p) {
-    return (p & ~15) + 4 * ((p >> 1) & 3) + 2 * ((p >> 3) & 1) + (p & 1);
+    return 16 * (2 * ((p >> 4) & 3) + (p >> 6)) + 4 * ((p >> 1) & 3) + 2 * ((p >> 3) & 1) + (p & 1);
 }
 
 // A layer's weights as tc_proj_mlp_kernel reads them, from the arrangements the
@@ -1532,30 +1538,45 @@ __global__ void pm_arrange_kernel(const uint4* __restrict__ wp, const uint4* __r
     }
 }
 
-// The sum of a row that lies in four lanes (p[m] = slot 4 m + lane % 4) in
-// tree32's order.
-__device__ __forceinline__ float frag_row_sum(float (&p)[8]) {
+// Sums of two rows that lie in four lanes of two warps, in tree32's order: p[k][i]
+// is row k's slot 4 (2 i + half) + lane % 4, and the other warp of the pair has the
+// other half's. xch: this pair's two blocks of 32 partial sums.
+__device__ __forceinline__ float2 frag_row_sums(float (&p)[2][4], int half, float2 (*xch)[32], int pair) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1)
+    for (int k = 0; k < 2; k++)
+        p[k][0] = __fadd_rn(__fadd_rn(p[k][0], p[k][2]), __fadd_rn(p[k][1], p[k][3]));
+    xch[half][lane] = make_float2(p[0][0], p[1][0]);
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+    const float2 o = xch[half ^ 1][lane];
+    float2 t = make_float2(__fadd_rn(p[0][0], o.x), __fadd_rn(p[1][0], o.y));
 #pragma unroll
-        for (int i = 0; i < o; i++) p[i] = __fadd_rn(p[i], p[i + o]);
-    p[0] = __fadd_rn(p[0], __shfl_xor_sync(0xffffffffu, p[0], 2));
-    return __fadd_rn(p[0], __shfl_xor_sync(0xffffffffu, p[0], 1));
+    for (int d = 2; d > 0; d >>= 1) {
+        t.x = __fadd_rn(t.x, __shfl_xor_sync(0xffffffffu, t.x, d));
+        t.y = __fadd_rn(t.y, __shfl_xor_sync(0xffffffffu, t.y, d));
+    }
+    return t;
 }
 
-// x[2 m + k] holds columns 16 m + 4 (lane % 4) .. + 3 of row k (rows lane / 4 and
-// lane / 4 + 8 of the warp's 16): x += acc + bias (acc: the warp's 16 TMEM lanes at
-// tacc), and the rows' mean and 1 / sqrt(variance + eps).
-__device__ __forceinline__ void frag_resid(float4 (&x)[16], uint32_t tacc, const float* bias, float (&mean)[2],
-                                           float (&rstd)[2]) {
-    const float4* b4 = reinterpret_cast<const float4*>(bias) + (threadIdx.x & 3);
+// A row warp's place in the residual + LayerNorm work.
+struct FragPos {
+    int half, pair;       // column half; the two warps of the same rows have one pair number
+    float2 (*xch)[2][32]; // their exchange: [sum, squares][half][lane]
+};
+
+// x[2 i + k] holds columns 16 (2 i + half) + 4 (lane % 4) .. + 3 of row k (rows
+// lane / 4 and lane / 4 + 8 of the warp's 16): x += acc + bias (acc: the warp's 16
+// TMEM lanes and 64 columns at tacc), and the rows' mean and 1 / sqrt(variance + eps).
+__device__ __forceinline__ void frag_resid(float4 (&x)[8], uint32_t tacc, const float* bias, const FragPos& at,
+                                           float (&mean)[2], float (&rstd)[2]) {
+    const float4* b4 = reinterpret_cast<const float4*>(bias) + 4 * at.half + (threadIdx.x & 3);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < 2; q++) {
         float a[16];
         tc::tmem_ld_frag32(tacc + 32 * q, a);
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const float4 bb = b4[4 * (2 * q + i)];
+            const float4 bb = b4[8 * (2 * q + i)];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 float4& v = x[2 * (2 * q + i) + k];
@@ -1568,28 +1589,30 @@ __device__ __forceinline__ void frag_resid(float4 (&x)[16], uint32_t tacc, const
             }
         }
     }
+    float p[2][4];
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        float p[8];
+    for (int k = 0; k < 2; k++)
 #pragma unroll
-        for (int m = 0; m < 8; m++) p[m] = sum4(x[2 * m + k]);
-        mean[k] = frag_row_sum(p) / (float)kPMD;
-    }
+        for (int i = 0; i < 4; i++) p[k][i] = sum4(x[2 * i + k]);
+    const float2 sum = frag_row_sums(p, at.half, at.xch[0], at.pair);
+    mean[0] = sum.x / (float)kPMD;
+    mean[1] = sum.y / (float)kPMD;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         const float2 nm = make_float2(-mean[k], -mean[k]);
-        float p[8];
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const float4 v = x[2 * m + k];
+        for (int i = 0; i < 4; i++) {
+            const float4 v = x[2 * i + k];
             const float2 e = add_f32x2(make_float2(v.x, v.y), nm), f = add_f32x2(make_float2(v.z, v.w), nm);
-            p[m] = __fadd_rn(__fmaf_rn(e.x, e.x, __fmul_rn(e.y, e.y)), __fmaf_rn(f.x, f.x, __fmul_rn(f.y, f.y)));
+            p[k][i] = __fadd_rn(__fmaf_rn(e.x, e.x, __fmul_rn(e.y, e.y)), __fmaf_rn(f.x, f.x, __fmul_rn(f.y, f.y)));
         }
-        rstd[k] = ln_rstd(frag_row_sum(p), kPMD);
     }
+    const float2 sq = frag_row_sums(p, at.half, at.xch[1], at.pair);
+    rstd[0] = ln_rstd(sq.x, kPMD);
+    rstd[1] = ln_rstd(sq.y, kPMD);
 }
 
-// LayerNorm(x) of columns 16 m + 4 (lane % 4) .. + 3 of row k, as two bf16 pairs.
+// LayerNorm(x) of four columns of row k, as two bf16 pairs.
 __device__ __forceinline__ uint2 frag_ln4(const float4 v, float mean, float rstd, const float4 g, const float4 b) {
     const float2 nm = make_float2(-mean, -mean), rs = make_float2(rstd, rstd);
     const float2 lo = fma_f32x2(mul_f32x2(add_f32x2(make_float2(v.x, v.y), nm), rs), make_float2(g.x, g.y),
@@ -1599,42 +1622,39 @@ __device__ __forceinline__ uint2 frag_ln4(const float4 v, float mean, float rstd
     const __nv_bfloat162 l = __floats2bfloat162_rn(lo.x, lo.y), h = __floats2bfloat162_rn(hi.x, hi.y);
     return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
 }
-// Into TMEM as an MMA's A operand: the 64 packed columns at tA.
-__device__ __forceinline__ void frag_ln_tmem(const float4 (&x)[16], const float (&mean)[2], const float (&rstd)[2],
-                                             const float* g, const float* b, uint32_t tA) {
-    const float4 *g4 = reinterpret_cast<const float4*>(g) + (threadIdx.x & 3),
-                 *b4 = reinterpret_cast<const float4*>(b) + (threadIdx.x & 3);
+// Into TMEM as an MMA's A operand: this half's groups of 8 of the 64 packed columns at tA.
+__device__ __forceinline__ void frag_ln_tmem(const float4 (&x)[8], const float (&mean)[2], const float (&rstd)[2],
+                                             const float* g, const float* b, int half, uint32_t tA) {
+    const int at = 4 * half + (threadIdx.x & 3);
+    const float4 *g4 = reinterpret_cast<const float4*>(g) + at, *b4 = reinterpret_cast<const float4*>(b) + at;
+    uint32_t r[16];
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        uint32_t r[16];
+    for (int i = 0; i < 4; i++) {
+        const float4 gg = g4[8 * i], be = b4[8 * i];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int m = 4 * q + i;
-            const float4 gg = g4[4 * m], be = b4[4 * m];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const uint2 u = frag_ln4(x[2 * m + k], mean[k], rstd[k], gg, be);
-                r[4 * i + 2 * k] = u.x;
-                r[4 * i + 2 * k + 1] = u.y;
-            }
+        for (int k = 0; k < 2; k++) {
+            const uint2 u = frag_ln4(x[2 * i + k], mean[k], rstd[k], gg, be);
+            r[4 * i + 2 * k] = u.x;
+            r[4 * i + 2 * k + 1] = u.y;
         }
-        tc::tmem_st_frag32(tA + 32 * q, r);
     }
+    tc::tmem_st_frag8x4(tA + 8 * half, r);
 }
 // Into the swizzled tile sOut (boxes of 64 columns x 128 rows; tr = the tile row
 // that lane / 4 falls on).
-__device__ __forceinline__ void frag_ln_smem(const float4 (&x)[16], const float (&mean)[2], const float (&rstd)[2],
-                                             const float* g, const float* b, uint8_t* sOut, int tr) {
+__device__ __forceinline__ void frag_ln_smem(const float4 (&x)[8], const float (&mean)[2], const float (&rstd)[2],
+                                             const float* g, const float* b, int half, uint8_t* sOut, int tr) {
     const int j = threadIdx.x & 3, sw = tr & 7;
-    const float4 *g4 = reinterpret_cast<const float4*>(g) + j, *b4 = reinterpret_cast<const float4*>(b) + j;
+    const float4 *g4 = reinterpret_cast<const float4*>(g) + 4 * half + j, *b4 = reinterpret_cast<const float4*>(b) + 4 * half + j;
     uint8_t* row = sOut + (size_t)tr * 128 + (j & 1) * 8;
 #pragma unroll
-    for (int m = 0; m < 8; m++) {
-        const float4 gg = g4[4 * m], be = b4[4 * m];
-        uint8_t* at = row + (m >> 2) * 16384 + (((2 * (m & 3) + (j >> 1)) ^ sw) << 4);
+    for (int i = 0; i < 4; i++) {
+        const int m = 2 * i + half;
+        const float4 gg = g4[8 * i], be = b4[8 * i];
+        uint8_t* to = row + (m >> 2) * 16384 + (((2 * (m & 3) + (j >> 1)) ^ sw) << 4);
 #pragma unroll
         for (int k = 0; k < 2; k++)
-            *reinterpret_cast<uint2*>(at + k * 8 * 128) = frag_ln4(x[2 * m + k], mean[k], rstd[k], gg, be);
+            *reinterpret_cast<uint2*>(to + k * 8 * 128) = frag_ln4(x[2 * i + k], mean[k], rstd[k], gg, be);
     }
 }
 
@@ -1648,10 +1668,11 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
     constexpr int D = kPMD, NC = kPMNC, NS = kPMSlots;
     constexpr uint32_t kB = kPMBlock;
     uint8_t* sAT = smem;            // attention rows, then the tile's LayerNorm rows: 2 x [128][64] swizzled
-    uint8_t* sX = smem + kPMOffX;   // residual rows, tiles alternating: 2 x (8 x [128][16] f32)
+    uint8_t* sX = smem + kPMOffX;   // residual rows on their way in or out: 8 x [128][16] f32
     uint8_t* sW = smem + kPMOffW;   // weight ring
     __shared__ __align__(16) float sb1[1024], sv[6][D];          // bp, g2, be2, b2, g, b
-    __shared__ uint64_t w_full[NS], w_empty[NS], at_full, at_empty, x_full[2], p_full, a_full, s_full[2], h_full[2],
+    __shared__ float2 s_xch[8][2][2][32];                        // the row warps' partial sums, by pair
+    __shared__ uint64_t w_full[NS], w_empty[NS], at_full, at_empty, x_full, x_taken, p_full, a_full, s_full[2], h_full[2],
         o_full, out_full;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
@@ -1664,8 +1685,8 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
             tc::mbar_init(&w_full[i], 1);
             tc::mbar_init(&w_empty[i], 1);
         }
-        for (uint64_t* q : {&at_full, &at_empty, &x_full[0], &x_full[1], &p_full, &s_full[0], &s_full[1], &o_full}) tc::mbar_init(q, 1);
-        for (uint64_t* q : {&a_full, &h_full[0], &h_full[1], &out_full}) tc::mbar_init(q, 8);  // one arrival per row warp
+        for (uint64_t* q : {&at_full, &at_empty, &x_full, &p_full, &s_full[0], &s_full[1], &o_full}) tc::mbar_init(q, 1);
+        for (uint64_t* q : {&x_taken, &a_full, &h_full[0], &h_full[1], &out_full}) tc::mbar_init(q, kPMRowWarps);  // one arrival per row warp
         tc::fence_barrier_init();
         failed = 0;
         if (tc::smem_u32(smem) & 1023u) {  // operand tiles need aligned shared memory
@@ -1685,7 +1706,7 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
     const uint32_t tO = tmem_base, tS = tmem_base + 128, tA = tmem_base + 384;  // O | S_0 | S_1 | A (64 columns)
     const uint32_t tP = tS + (n & 1) * NC;                // P: the accumulator that chunk n - 2 used
     auto blocks_of = [&](int c) { return min(NC, F - c * NC) / 64; };
-    if (warp == 8) {
+    if (warp == kPMRowWarps) {
         // the weights never change: their loads do not wait for the previous kernel
         if (tc::elect_one() && !failed) {
             int cnt = 0;
@@ -1709,103 +1730,120 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
             for (int it = 0; it < my_tiles && ok; it++) {
                 for (int c = 0; c < 2 && c < n; c++) put_chunk(W1, c);
                 for (int c = 0; c < n && ok; c++) {
-                    if (c == n - 1 && it + 1 < my_tiles) put_p();
                     put_chunk(W2, c);
                     if (c + 2 < n) put_chunk(W1, c + 2);
+                    if (c == n - 1 && it + 1 < my_tiles) put_p();
                 }
             }
         }
         __syncwarp();
         JC_PDL_ENTRY;
-    } else if (warp == 9) {
+    } else if (warp == kPMRowWarps + 1) {
         JC_PDL_ENTRY;
         if (tc::elect_one() && !failed) {
             constexpr uint32_t id128 = tc::idesc_bf16(128, D), id64 = tc::idesc_bf16(128, 64);
             const uint64_t dAT = tc::sdesc_sw128(tc::smem_u32(sAT));
             const uint64_t dW128 = tc::sdesc(tc::smem_u32(sW), D * 16, 128), dW64 = tc::sdesc(tc::smem_u32(sW), 64 * 16, 128);
-            int sl = 0;
-            uint32_t ph_w = 0;
+            // Weight blocks are waited for (take) ahead of what their MMAs wait for
+            // last, and given back after the commit that somebody waits for.
+            int t_sl = 0, u_sl = 0, ahead = 0, used = 0;
+            uint32_t t_ph = 0;
             bool ok = true;
-            auto take = [&]() {  // the next weight block has arrived
-                ok = ok && tc::mbar_wait(&w_full[sl], ph_w, err, &failed);
+            auto take = [&](int k) {
+                for (; ok && ahead < k; ahead++) {
+                    ok = tc::mbar_wait(&w_full[t_sl], t_ph, err, &failed);
+                    if (++t_sl == NS) {
+                        t_sl = 0;
+                        t_ph ^= 1u;
+                    }
+                }
                 tc::tc_fence_after();
-                return ok;
             };
-            auto done = [&]() {
-                tc::mma_commit(&w_empty[sl]);
-                if (++sl == NS) {
-                    sl = 0;
-                    ph_w ^= 1u;
+            auto slot = [&]() {  // the next taken block's offset
+                const int at = u_sl + used++;
+                ahead--;
+                return (uint32_t)(at < NS ? at : at - NS) * kB;
+            };
+            auto give_back = [&]() {
+                for (; used > 0; used--) {
+                    tc::mma_commit(&w_empty[u_sl]);
+                    if (++u_sl == NS) u_sl = 0;
                 }
             };
             auto issue_p = [&](int it) {  // P = attn @ Wp
+                take(2);
                 ok = ok && tc::mbar_wait(&at_full, (uint32_t)it & 1u, err, &failed);
+                if (!ok) return;
+                tc::tc_fence_after();
+#pragma unroll
                 for (int q = 0; q < 2; q++) {
-                    if (!take()) return;
-                    const uint64_t w = tc::sdesc_at(dW128, sl * kB), a = tc::sdesc_at(dAT, q * 16384);
+                    const uint64_t w = tc::sdesc_at(dW128, slot()), a = tc::sdesc_at(dAT, q * 16384);
 #pragma unroll
                     for (int k = 0; k < 4; k++)
                         tc::mma_bf16(tP, tc::sdesc_at(a, k * 32), tc::sdesc_at(w, k * 2 * D * 16), id128,
                                      k > 0 ? 1u : (uint32_t)q);
-                    done();
                 }
-                tc::mma_commit(&at_empty);
                 tc::mma_commit(&p_full);
+                give_back();
+                tc::mma_commit(&at_empty);
             };
             auto issue_s = [&](int c) {  // S_c = A @ W1_c: 128 columns in two K halves, or 64 in one block
                 const int nb = blocks_of(c);
                 const uint32_t t = tS + (c & 1) * NC;
-                for (int q = 0; q < nb; q++) {
-                    if (!take()) return;
-                    if (nb == 2) {
-                        const uint64_t w = tc::sdesc_at(dW128, sl * kB);
+                take(nb);
+                if (!ok) return;
+                if (nb == 2) {
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        const uint64_t w = tc::sdesc_at(dW128, slot());
 #pragma unroll
                         for (int k = 0; k < 4; k++)
                             tc::mma_bf16_ta(t, tA + q * 32 + k * 8, tc::sdesc_at(w, k * 2 * 128 * 16), id128,
                                             k > 0 ? 1u : (uint32_t)q);
-                    } else {
-                        const uint64_t w = tc::sdesc_at(dW64, sl * kB);
-#pragma unroll
-                        for (int k = 0; k < D / 16; k++)
-                            tc::mma_bf16_ta(t, tA + k * 8, tc::sdesc_at(w, k * 2 * 64 * 16), id64, k > 0 ? 1u : 0u);
                     }
-                    done();
+                } else {
+                    const uint64_t w = tc::sdesc_at(dW64, slot());
+#pragma unroll
+                    for (int k = 0; k < D / 16; k++)
+                        tc::mma_bf16_ta(t, tA + k * 8, tc::sdesc_at(w, k * 2 * 64 * 16), id64, k > 0 ? 1u : 0u);
                 }
                 tc::mma_commit(&s_full[c & 1]);
+                give_back();
             };
             auto issue_o = [&](int c) {  // O += h_c @ W2_c; 32 columns of h lie packed in the first 16 of their own
                 const int nb = blocks_of(c);
                 for (int q = 0; q < nb; q++) {
-                    if (!take()) return;
-                    const uint64_t w = tc::sdesc_at(dW128, sl * kB);
+                    const uint64_t w = tc::sdesc_at(dW128, slot());
                     const uint32_t t = tS + (c & 1) * NC + q * 64;
 #pragma unroll
                     for (int k = 0; k < 4; k++)
                         tc::mma_bf16_ta(tO, t + (k >> 1) * 32 + (k & 1) * 8, tc::sdesc_at(w, k * 2 * D * 16), id128,
                                         k > 0 ? 1u : (uint32_t)(c + q > 0));
-                    done();
                 }
                 if (c == n - 1) tc::mma_commit(&o_full);
+                give_back();
             };
-            uint32_t ph_h[2] = {0u, 0u};
+            uint32_t ph_h = 0u;  // a bit for each accumulator
             if (my_tiles > 0) issue_p(0);
             for (int it = 0; it < my_tiles && ok; it++) {
-                ok = tc::mbar_wait(&a_full, (uint32_t)it & 1u, err, &failed);
+                take(blocks_of(0));
+                ok = ok && tc::mbar_wait(&a_full, (uint32_t)it & 1u, err, &failed);
                 tc::tc_fence_after();
                 for (int c = 0; c < 2 && c < n && ok; c++) issue_s(c);
                 for (int c = 0; c < n && ok; c++) {
-                    if (c == n - 1 && it + 1 < my_tiles) issue_p(it + 1);  // after O_{n-2}, which reads tP's columns
-                    ok = ok && tc::mbar_wait(&h_full[c & 1], ph_h[c & 1], err, &failed);
-                    ph_h[c & 1] ^= 1u;
+                    take(blocks_of(c));
+                    ok = ok && tc::mbar_wait(&h_full[c & 1], ph_h >> (c & 1) & 1u, err, &failed);
+                    ph_h ^= 1u << (c & 1);
                     if (!ok) break;
                     tc::tc_fence_after();
                     issue_o(c);
                     if (c + 2 < n && ok) issue_s(c + 2);  // after O_c, which reads h_c from its columns
+                    if (c == n - 1 && it + 1 < my_tiles) issue_p(it + 1);
                 }
             }
         }
         __syncwarp();
-    } else if (warp == 10) {
+    } else if (warp == kPMRowWarps + 2) {
         JC_PDL_ENTRY;
         if (tc::elect_one() && !failed) {
             auto m0_of = [&](int it) { return ((int)blockIdx.x + it * (int)gridDim.x) * 128; };
@@ -1814,9 +1852,8 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
                 for (int c = 0; c < 2; c++) tc::tma_load_2d(sAT + c * 16384, &tmAttn, 64 * c, m0_of(it), &at_full);
             };
             auto load_x = [&](int it) {
-                tc::mbar_expect_tx(&x_full[it & 1], kPMX);
-                for (int m = 0; m < 8; m++)
-                    tc::tma_load_2d(sX + (it & 1) * kPMX + m * 8192, &tmX, 16 * m, m0_of(it), &x_full[it & 1]);
+                tc::mbar_expect_tx(&x_full, kPMX);
+                for (int m = 0; m < 8; m++) tc::tma_load_2d(sX + m * 8192, &tmX, 16 * m, m0_of(it), &x_full);
             };
             bool ok = true;
             if (my_tiles > 0) {
@@ -1824,15 +1861,16 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
                 load_x(0);
             }
             if (my_tiles > 1) {
-                load_x(1);
-                ok = tc::mbar_wait(&at_empty, 0, err, &failed);
+                ok = tc::mbar_wait(&x_taken, 0, err, &failed);
+                if (ok) load_x(1);
+                ok = ok && tc::mbar_wait(&at_empty, 0, err, &failed);
                 if (ok) load_attn(1);
             }
             for (int it = 0; it < my_tiles && ok; it++) {
                 ok = tc::mbar_wait(&out_full, (uint32_t)it & 1u, err, &failed);
                 if (!ok) break;
                 for (int c = 0; c < 2; c++) tc::tma_store_2d(&tmLn, sAT + c * 16384, 64 * c, m0_of(it));
-                for (int m = 0; m < 8; m++) tc::tma_store_2d(&tmX, sX + (it & 1) * kPMX + m * 8192, 16 * m, m0_of(it));
+                for (int m = 0; m < 8; m++) tc::tma_store_2d(&tmX, sX + m * 8192, 16 * m, m0_of(it));
                 tc::bulk_commit();
                 tc::bulk_wait_read();
                 if (it + 2 < my_tiles) {
@@ -1844,72 +1882,82 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
         __syncwarp();
     } else {
         JC_PDL_ENTRY;
-        const int quarter = warp & 3, half = warp >> 2;
-        const int tr = 32 * quarter + 16 * half + (lane >> 2);  // tile row of this thread's first row
-        const uint32_t trow = (uint32_t)(32 * quarter + 16 * half) << 16;
-        const uint32_t lane_s = ((uint32_t)(32 * quarter) << 16) + half * 64;
+        // warps 4 s + q on TMEM lanes 32 q ..: 16 of them (s % 2) and half of the
+        // columns (s / 2) in the LayerNorms, all 32 and 32 of a chunk's columns in the GELUs
+        const int quarter = warp & 3, sub = warp >> 2, half = sub >> 1, pair = warp & 7;
+        const FragPos at{half, pair, s_xch[pair]};
+        const int tr = 32 * quarter + 16 * (sub & 1) + (lane >> 2);  // tile row of this thread's first row
+        const uint32_t trow = (uint32_t)(32 * quarter + 16 * (sub & 1)) << 16;
+        const uint32_t lane_s = ((uint32_t)(32 * quarter) << 16) + 32 * sub;
+        // A failed wait ends no loop here: every later wait fails at once, the other
+        // warps issue no more copies and MMAs, and no warp is left alone at a pair's barrier.
         auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
-            const bool good = __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, err, &failed) ? 1 : 0) != 0;
+            tc::mbar_wait(bar, parity, err, &failed);
+            __syncwarp();
             tc::tc_fence_after();
-            return good;
         };
         auto warp_arrive = [&](uint64_t* bar) {
             tc::tc_fence_before();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(bar);
         };
-        uint32_t ph_s[2] = {0u, 0u};
-        for (int it = 0; it < my_tiles; it++) {
-            float4 x[16];
-            float mean[2], rstd[2];
-            uint8_t* xs = sX + (it & 1) * kPMX + tr * 64 + (lane & 3) * 16;  // this thread's part of its rows
-            bool ok = warp_wait(&x_full[it & 1], (uint32_t)(it >> 1) & 1u);
-            if (!ok) break;
+        uint32_t ph_s = 0u;  // a bit for each accumulator
+        // this thread's part of its rows: boxes 2 i + half
+        uint8_t* xs = sX + half * 8192 + tr * 64 + (lane & 3) * 16;
+        float4 x[8];
+        if (my_tiles > 0) {
+            warp_wait(&x_full, 0);
 #pragma unroll
-            for (int m = 0; m < 8; m++) {
-                x[2 * m] = *reinterpret_cast<const float4*>(xs + m * 8192);
-                x[2 * m + 1] = *reinterpret_cast<const float4*>(xs + m * 8192 + 8 * 64);
-            }
-            if (!warp_wait(&p_full, (uint32_t)it & 1u)) break;
-            frag_resid(x, tP + trow, sv[0], mean, rstd);
-            frag_ln_tmem(x, mean, rstd, sv[1], sv[2], tA + trow);
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int k = 0; k < 2; k++) x[2 * i + k] = *reinterpret_cast<const float4*>(xs + i * 16384 + k * 8 * 64);
+            warp_arrive(&x_taken);
+        }
+        for (int it = 0; it < my_tiles; it++) {
+            float mean[2], rstd[2];
+            if (it == 0) warp_wait(&p_full, 0);
+            frag_resid(x, tP + trow + 64 * half, sv[0], at, mean, rstd);
+            frag_ln_tmem(x, mean, rstd, sv[1], sv[2], half, tA + trow);
             warp_arrive(&a_full);
             for (int c = 0; c < n; c++) {
-                ok = warp_wait(&s_full[c & 1], ph_s[c & 1]);
-                ph_s[c & 1] ^= 1u;
-                if (!ok) break;
-                if (half < blocks_of(c)) {
-                    const float* bj = sb1 + c * NC + half * 64;
-#pragma unroll 1
-                    for (int q = 0; q < 2; q++) {
-                        const uint32_t ts = tS + (c & 1) * NC + lane_s + 32 * q;
-                        float a[32];
-                        tc::tmem_ld32(ts, a);
-                        uint32_t h[16];
+                warp_wait(&s_full[c & 1], ph_s >> (c & 1) & 1u);
+                ph_s ^= 1u << (c & 1);
+                if (sub < 2 * blocks_of(c)) {
+                    const float* bj = sb1 + c * NC + sub * 32;
+                    const uint32_t ts = tS + (c & 1) * NC + lane_s;
+                    float a[32];
+                    tc::tmem_ld32(ts, a);
+                    uint32_t h[16];
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4) {
-                            const float4 bb = *reinterpret_cast<const float4*>(bj + 32 * q + i);
-                            gelu_fast_pair(a[i], a[i + 1], bb.x, bb.y);
-                            gelu_fast_pair(a[i + 2], a[i + 3], bb.z, bb.w);
-                            __nv_bfloat162 lo = __floats2bfloat162_rn(a[i], a[i + 1]);
-                            __nv_bfloat162 hi = __floats2bfloat162_rn(a[i + 2], a[i + 3]);
-                            h[i / 2] = *reinterpret_cast<uint32_t*>(&lo);
-                            h[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
-                        }
-                        tc::tmem_st16(ts, h);
+                    for (int i = 0; i < 32; i += 4) {
+                        const float4 bb = *reinterpret_cast<const float4*>(bj + i);
+                        gelu_fast_pair(a[i], a[i + 1], bb.x, bb.y);
+                        gelu_fast_pair(a[i + 2], a[i + 3], bb.z, bb.w);
+                        __nv_bfloat162 lo = __floats2bfloat162_rn(a[i], a[i + 1]);
+                        __nv_bfloat162 hi = __floats2bfloat162_rn(a[i + 2], a[i + 3]);
+                        h[i / 2] = *reinterpret_cast<uint32_t*>(&lo);
+                        h[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
                     }
+                    tc::tmem_st16(ts, h);
                 }
                 warp_arrive(&h_full[c & 1]);
             }
-            if (!ok || !warp_wait(&o_full, (uint32_t)it & 1u)) break;
-            frag_resid(x, tO + trow, sv[3], mean, rstd);
-            // P of the next tile has been computed (before the last O): its attention rows are no longer read
-            frag_ln_smem(x, mean, rstd, sv[4], sv[5], sAT, tr);
+            warp_wait(&o_full, (uint32_t)it & 1u);
+            frag_resid(x, tO + trow + 64 * half, sv[3], at, mean, rstd);
+            // the LayerNorm rows go over the next tile's attention rows: its P has read them by now
+            if (it + 1 < my_tiles) warp_wait(&p_full, (uint32_t)(it + 1) & 1u);
+            frag_ln_smem(x, mean, rstd, sv[4], sv[5], half, sAT, tr);
+            // the next tile's rows in, this one's out
+            if (it + 1 < my_tiles) warp_wait(&x_full, (uint32_t)(it + 1) & 1u);
 #pragma unroll
-            for (int m = 0; m < 8; m++) {
-                *reinterpret_cast<float4*>(xs + m * 8192) = x[2 * m];
-                *reinterpret_cast<float4*>(xs + m * 8192 + 8 * 64) = x[2 * m + 1];
-            }
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    float4* slot = reinterpret_cast<float4*>(xs + i * 16384 + k * 8 * 64);
+                    const float4 next = *slot;
+                    *slot = x[2 * i + k];
+                    x[2 * i + k] = next;
+                }
             tc::fence_async_shared();
             warp_arrive(&out_full);
         }
