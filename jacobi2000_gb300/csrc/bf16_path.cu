@@ -149,11 +149,10 @@ static CUtensorMap tile_store_map(const void* base, int C, int nx, int ny, bool 
 // edges), landing as [planes][18][10][8]; tile stores: 8 x 16 positions of
 // every plane from [planes][16][8][8] (positions outside the grid are not
 // written).
-static CUtensorMap cell_plane_map(const void* base, int planes, long long plane, int nx, int ny, bool halo) {
+static CUtensorMap cell_plane_map(const void* base, int planes, long long plane, int nx, int ny) {
     uint64_t dims[3] = {(uint64_t)nx * 8, (uint64_t)ny, (uint64_t)planes};
     uint64_t strides[2] = {(uint64_t)nx * 16, (uint64_t)plane};
-    uint32_t box[3] = {(uint32_t)(halo ? (kConvTX + 2) * 8 : kConvTX * 8), (uint32_t)(halo ? kConvTY + 2 : kConvTY),
-                       (uint32_t)planes};
+    uint32_t box[3] = {(uint32_t)(kConvTX + 2) * 8, (uint32_t)kConvTY + 2, (uint32_t)planes};
     return make_map(base, 3, dims, strides, box, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
 }
 
@@ -2154,7 +2153,7 @@ __global__ void __launch_bounds__(kQKVPThreads, 2) tc_qkv_kernel(
         tc::mbar_init(&a_empty, 1);
         for (int i = 0; i < 2; i++) {
             tc::mbar_init(&acc_full[i], 1);
-            tc::mbar_init(&acc_empty[i], 4 * 32);
+            tc::mbar_init(&acc_empty[i], 4);
         }
         tc::fence_barrier_init();
         failed = 0;
@@ -2238,7 +2237,8 @@ __global__ void __launch_bounds__(kQKVPThreads, 2) tc_qkv_kernel(
                 }
             }
             tc::tc_fence_before();
-            tc::mbar_arrive(&acc_empty[it & 1]);
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&acc_empty[it & 1]);
             tc::fence_async_shared();
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (warp == 2 && tc::elect_one()) {
@@ -2649,9 +2649,12 @@ __global__ void __launch_bounds__(kMixThreads, 1) tc_mix_cells_kernel(
 // kCellConv1, conv1 (cpu.rs:343-346): the 3x3 conv of the cell-head input zc
 // (48 f16 channels) to 32 channels as 9 taps x 3 MMAs (tap (ky, kx) is the
 // halo tile addressed from position (ky, kx)), + bias, GELU, stored as f16
-// (c1) through one staged box (the next tile's epilogue waits until the
-// store has read it) and a TMA store; the MMA order and the epilogue
-// arithmetic are those of tc_conv3_kernel.
+// (c1) by each epilogue warp for itself: 128-byte runs of 8 cells in each of the
+// four planes. Shared memory's 128 bytes a cycle bound it (the MMAs read 135 KB
+// of A and weights a tile, 1080 cycles), so its epilogue stays out of there:
+// with staged boxes, barrier arrivals by each thread instead of each warp and two
+// CTA barriers a tile, a tick of 64 x 128 x 128 cells took 652 us, not 630.
+// The MMA order and the epilogue arithmetic are those of tc_conv3_kernel.
 // kCellConv2, conv2 and the step (cpu.rs:347-348, 84-88): 32 -> 3 channels.
 // With 3 outputs the per-tap form would re-read the whole halo tile from
 // shared memory for 9 tiny MMAs; instead one GEMM gives every halo position
@@ -2671,13 +2674,13 @@ constexpr int kC1PHaloStages = 2;
 constexpr int kHaloPos = kHaloW * kHaloH;  // 180 halo positions
 constexpr int kZPitch = 33;                // f32 per staged Z row (bank-conflict-free column reads)
 
-// TMEM columns per accumulator, weight bytes and staged bytes of each kind.
+// TMEM columns per accumulator, weight bytes and staged bytes (Z) of each kind.
 __host__ __device__ constexpr int cellconv_bn(int kind) { return kind == kCellConv1 ? 32 : 64; }
 __host__ __device__ constexpr size_t cellconv_wbytes(int kind, int C) {
     return kind == kCellConv1 ? (size_t)9 * C * 32 * 2 : (size_t)C * 32 * 2;
 }
 __host__ __device__ constexpr size_t cellconv_stage(int kind) {
-    return kind == kCellConv1 ? (size_t)128 * 32 * 2 : (size_t)kHaloPos * kZPitch * 4;
+    return kind == kCellConv1 ? 0 : (size_t)kHaloPos * kZPitch * 4;
 }
 
 struct C1PSmem {
@@ -2685,7 +2688,7 @@ struct C1PSmem {
     __host__ __device__ C1PSmem(int kind, int C) {
         halo = 0;                                                          // stages x [C/8][18][10][8]
         w = halo + (size_t)kC1PHaloStages * (C / 8) * kCellPlane;          // the weight blocks
-        stage = (w + cellconv_wbytes(kind, C) + 1023) / 1024 * 1024;       // staged output
+        stage = (w + cellconv_wbytes(kind, C) + 1023) / 1024 * 1024;       // conv2's Z
         total = stage + cellconv_stage(kind);
     }
 };
@@ -2695,10 +2698,11 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
                                                                    const bf16* __restrict__ Wt,
                                                                    const float* __restrict__ bias, int C,
                                                                    int n_tiles, const InstDev* inst, int n_inst,
-                                                                   int mode, int* err) {
+                                                                   int mode, __half* __restrict__ c1,
+                                                                   long long c1_plane, int* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int BN = cellconv_bn(KIND);
-    constexpr int kInSlot = KIND == kCellConv1 ? 1 : 6;  // zc halo | c1 halo
+    constexpr int kInSlot = KIND == kCellConv1 ? 1 : 3;  // zc halo | c1 halo
     const C1PSmem L(KIND, C);
     uint8_t* sHalo = smem + L.halo;
     uint8_t* sW = smem + L.w;
@@ -2721,7 +2725,7 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
         }
         for (int i = 0; i < 2; i++) {
             tc::mbar_init(&a_full[i], 1);
-            tc::mbar_init(&a_empty[i], 4 * 32);
+            tc::mbar_init(&a_empty[i], 4);  // the epilogue warps
         }
         tc::fence_barrier_init();
         failed = 0;
@@ -2827,18 +2831,18 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
 #pragma unroll
                 for (int co = 0; co < 3; co++) st[co] = I.state[co * plane + cl];
             }
-            const bool ready = tc::mbar_wait(&a_full[b], (uint32_t)(it >> 1) & 1u, err, &failed);
-            uint32_t all_ready;
-            asm volatile(
-                "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.red.and.pred p, 1, 128, q;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}"
-                : "=r"(all_ready)
-                : "r"(ready ? 1u : 0u)
-                : "memory");
-            if (!all_ready) break;
-            tc::tc_fence_after();
             const uint32_t ta = lane_addr(tmem + (uint32_t)b * BN);
             if constexpr (KIND == kCellConv2) {
+                const bool ready = tc::mbar_wait(&a_full[b], (uint32_t)(it >> 1) & 1u, err, &failed);
+                uint32_t all_ready;
+                asm volatile(
+                    "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.red.and.pred p, 1, 128, q;\n\t"
+                    "selp.u32 %0, 1, 0, p;\n\t}"
+                    : "=r"(all_ready)
+                    : "r"(ready ? 1u : 0u)
+                    : "memory");
+                if (!all_ready) break;
+                tc::tc_fence_after();
                 // Z rows r and 128 + r -> shared memory, then output cell r
                 float* Z = reinterpret_cast<float*>(sStage);
 #pragma unroll
@@ -2852,7 +2856,8 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
                     }
                 }
                 tc::tc_fence_before();
-                tc::mbar_arrive(&a_empty[b]);
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&a_empty[b]);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 const int lx = r & 7, ly = r >> 3;
                 float v[3] = {0.f, 0.f, 0.f};
@@ -2870,39 +2875,30 @@ __global__ void __launch_bounds__(kC1PThreads) tc_cellconv_kernel(const CUtensor
                         I.out[co * plane + cl] = o;
                     }
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // Z is rewritten by the next tile
+                // (the next tile's first barrier comes before Z is written again)
             } else {
-                // the staging box used two tiles ago must have been read by its store
-                if (warp == 2 && it >= 1 && tc::elect_one()) tc::bulk_wait_read();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                uint8_t* box = sStage + (size_t)r * 16;  // [4 planes][128][8] f16
-                for (int c = 0; c < BN; c += 16) {
-                    float a[16];
-                    tc::tmem_ld16(ta + c, a);
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) gelu_fast_pair(a[i], a[i + 1], sbias[c + i], sbias[c + i + 1]);
-                    uint32_t w[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        __half2 h = __floats2half2_rn(a[2 * i], a[2 * i + 1]);
-                        w[i] = *reinterpret_cast<uint32_t*>(&h);
-                    }
-                    *reinterpret_cast<uint4*>(box + (c / 8) * 2048) = make_uint4(w[0], w[1], w[2], w[3]);
-                    *reinterpret_cast<uint4*>(box + (c / 8 + 1) * 2048) = make_uint4(w[4], w[5], w[6], w[7]);
-                }
+                // the warps go their own ways: no staging, no barrier
+                if (!__all_sync(0xffffffffu, tc::mbar_wait(&a_full[b], (uint32_t)(it >> 1) & 1u, err, &failed) ? 1 : 0)) break;
+                tc::tc_fence_after();
+                float a[32];
+                tc::tmem_ld32(ta, a);
                 tc::tc_fence_before();
-                tc::mbar_arrive(&a_empty[b]);
-                tc::fence_async_shared();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp == 2 && tc::elect_one()) {
-                    const CUtensorMap* omap = maps + kMapsPerInst * ii + 3;
-                    tc::tensormap_acquire(omap);
-                    tc::tma_store_3d(omap, sStage, x0 * 8, y0, 0);
-                    tc::bulk_commit();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&a_empty[b]);
+                __half* o = c1 + ((size_t)I.cell0 + cl) * 8;
+#pragma unroll
+                for (int c = 0; c < 32; c += 8) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        gelu_fast_pair(a[c + i], a[c + i + 1], sbias[c + i], sbias[c + i + 1]);
+                        __half2 h = __floats2half2_rn(a[c + i], a[c + i + 1]);
+                        w[i / 2] = *reinterpret_cast<uint32_t*>(&h);
+                    }
+                    if (inside) *reinterpret_cast<uint4*>(o + (c / 8) * c1_plane) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
         }
-        if (KIND == kCellConv1 && warp == 2 && tc::elect_one()) tc::bulk_wait_read();
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -3350,10 +3346,9 @@ void BF16Path::prepare(const Dims& d, const Pack& p, const InstDev* hinst, cudaS
         const InstDev& I = hinst[i];
         CUtensorMap* m = &maps[(size_t)kMapsPerInst * i];
         m[0] = halo_map(p.bt[0] + (size_t)I.row0 * p.bt_stride[0], d.D, I.tx, I.ty);
-        m[1] = cell_plane_map(p.bc[0] + (size_t)I.cell0 * 16, kZcCh / 8, p.bc_plane[0], I.nx, I.ny, true);
+        m[1] = cell_plane_map(p.bc[0] + (size_t)I.cell0 * 16, kZcCh / 8, p.bc_plane[0], I.nx, I.ny);
         m[2] = tile_store_map(p.bt[3] + (size_t)I.row0 * p.bt_stride[3], d.D, I.tx, I.ty, false);
-        m[3] = cell_plane_map(p.bc[1] + (size_t)I.cell0 * 16, d.HD / 8, p.bc_plane[1], I.nx, I.ny, false);
-        m[6] = cell_plane_map(p.bc[1] + (size_t)I.cell0 * 16, d.HD / 8, p.bc_plane[1], I.nx, I.ny, true);
+        m[3] = cell_plane_map(p.bc[1] + (size_t)I.cell0 * 16, d.HD / 8, p.bc_plane[1], I.nx, I.ny);
         if (attn_tile_ok(d)) {
             m[4] = att_map(p.bt[1] + (size_t)I.row0 * p.bt_stride[1], d.D, I.tx, I.ty, kAttHalo);
             m[5] = att_map(p.bt[1] + (size_t)I.row0 * p.bt_stride[1], d.D, I.tx, I.ty, kAttTile);
@@ -3495,7 +3490,7 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
         cuda_check(launch_pdl(tc_cellconv_kernel<kCellConv1>, grid, kC1PThreads,
                               C1PSmem(kCellConv1, kZcCh).total, s, 1u,
                               reinterpret_cast<const CUtensorMap*>(p.tmaps), wc1, w.c1_b, kZcCh, p.n_ctiles, p.inst, n,
-                              mode, p.err),
+                              mode, reinterpret_cast<__half*>(p.bc[1]), p.bc_plane[1] / 2, p.err),
                    "launch");
         check_launch("tc_conv1");
     }
@@ -3504,7 +3499,7 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
         const unsigned grid = (unsigned)std::min(p.n_ctiles, 4 * n_sms_);
         cuda_check(launch_pdl(tc_cellconv_kernel<kCellConv2>, grid, kC1PThreads, C1PSmem(kCellConv2, d.HD).total, s, 1u,
                               reinterpret_cast<const CUtensorMap*>(p.tmaps), wc2, w.c2_b, d.HD, p.n_ctiles, p.inst, n,
-                              mode, p.err),
+                              mode, nullptr, 0, p.err),
                    "launch");
         check_launch("tc_conv2");
     }
