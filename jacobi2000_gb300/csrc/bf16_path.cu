@@ -1658,12 +1658,34 @@ __device__ __forceinline__ void frag_ln_smem(const float4 (&x)[8], const float (
     }
 }
 
+// The same to global memory (row: this thread's first row there; those from R on are not written).
+__device__ __forceinline__ void frag_ln_global(const float4 (&x)[8], const float (&mean)[2], const float (&rstd)[2],
+                                               const float* g, const float* b, int half, bf16* ln, int row, int R) {
+    const int at = 4 * half + (threadIdx.x & 3);
+    const float4 *g4 = reinterpret_cast<const float4*>(g) + at, *b4 = reinterpret_cast<const float4*>(b) + at;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float4 gg = g4[8 * i], be = b4[8 * i];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint2 u = frag_ln4(x[2 * i + k], mean[k], rstd[k], gg, be);
+            if (row + 8 * k < R) reinterpret_cast<uint2*>(ln + (size_t)(row + 8 * k) * kPMD)[8 * i + at] = u;
+        }
+    }
+}
+
+// SPLIT: two CTAs take one tile, each the row work of 16 lanes of every 32
+// (blockIdx.x % 2), one tile a CTA; the MMAs, whose time does not depend on the
+// rows, they both do (each also loads the other's rows, which may
+// change meanwhile, and does not use them). The rows go straight to global memory.
+template <bool SPLIT>
 __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
     const __grid_constant__ CUtensorMap tmAttn, const __grid_constant__ CUtensorMap tmLn,
     const __grid_constant__ CUtensorMap tmX, const bf16* __restrict__ Wp,
     const bf16* __restrict__ W1, const bf16* __restrict__ W2, const float* __restrict__ bp, const float* __restrict__ g2,
     const float* __restrict__ be2, const float* __restrict__ b1, const float* __restrict__ b2,
-    const float* __restrict__ g, const float* __restrict__ b, int F, int R, float* __restrict__ xg, int* err) {
+    const float* __restrict__ g, const float* __restrict__ b, int F, int R, float* __restrict__ xg, bf16* __restrict__ ln,
+    int* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int D = kPMD, NC = kPMNC, NS = kPMSlots;
     constexpr uint32_t kB = kPMBlock;
@@ -1678,7 +1700,9 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
     __shared__ volatile int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = (R + 127) / 128;
-    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int first = SPLIT ? blockIdx.x / 2 : blockIdx.x, step = SPLIT ? n_tiles : gridDim.x;
+    const int my_tiles = first < n_tiles ? (n_tiles - 1 - first) / step + 1 : 0;
+    auto m0_of = [&](int it) { return (first + it * step) * 128; };
     const int n = (F + NC - 1) / NC;  // chunks; the last may have 64 columns
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) {
@@ -1846,7 +1870,6 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
     } else if (warp == kPMRowWarps + 2) {
         JC_PDL_ENTRY;
         if (tc::elect_one() && !failed) {
-            auto m0_of = [&](int it) { return ((int)blockIdx.x + it * (int)gridDim.x) * 128; };
             auto load_attn = [&](int it) {
                 tc::mbar_expect_tx(&at_full, D * 256);
                 for (int c = 0; c < 2; c++) tc::tma_load_2d(sAT + c * 16384, &tmAttn, 64 * c, m0_of(it), &at_full);
@@ -1866,7 +1889,7 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
                 ok = ok && tc::mbar_wait(&at_empty, 0, err, &failed);
                 if (ok) load_attn(1);
             }
-            for (int it = 0; it < my_tiles && ok; it++) {
+            for (int it = 0; it < my_tiles && ok && !SPLIT; it++) {
                 ok = tc::mbar_wait(&out_full, (uint32_t)it & 1u, err, &failed);
                 if (!ok) break;
                 for (int c = 0; c < 2; c++) tc::tma_store_2d(&tmLn, sAT + c * 16384, 64 * c, m0_of(it));
@@ -1888,7 +1911,9 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
         const FragPos at{half, pair, s_xch[pair]};
         const int tr = 32 * quarter + 16 * (sub & 1) + (lane >> 2);  // tile row of this thread's first row
         const uint32_t trow = (uint32_t)(32 * quarter + 16 * (sub & 1)) << 16;
-        const uint32_t lane_s = ((uint32_t)(32 * quarter) << 16) + 32 * sub;
+        const int part = SPLIT ? blockIdx.x & 1 : 0;
+        const bool norms = !SPLIT || (sub & 1) == part;  // whether this warp has rows in the LayerNorms
+        const uint32_t lane_s = ((uint32_t)(32 * quarter + 16 * part) << 16) + 32 * sub;
         // A failed wait ends no loop here: every later wait fails at once, the other
         // warps issue no more copies and MMAs, and no warp is left alone at a pair's barrier.
         auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
@@ -1916,8 +1941,10 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
         for (int it = 0; it < my_tiles; it++) {
             float mean[2], rstd[2];
             if (it == 0) warp_wait(&p_full, 0);
-            frag_resid(x, tP + trow + 64 * half, sv[0], at, mean, rstd);
-            frag_ln_tmem(x, mean, rstd, sv[1], sv[2], half, tA + trow);
+            if (norms) {
+                frag_resid(x, tP + trow + 64 * half, sv[0], at, mean, rstd);
+                frag_ln_tmem(x, mean, rstd, sv[1], sv[2], half, tA + trow);
+            }
             warp_arrive(&a_full);
             for (int c = 0; c < n; c++) {
                 warp_wait(&s_full[c & 1], ph_s >> (c & 1) & 1u);
@@ -1925,24 +1952,53 @@ __global__ void __launch_bounds__(kPMThreads, 1) tc_proj_mlp_kernel(
                 if (sub < 2 * blocks_of(c)) {
                     const float* bj = sb1 + c * NC + sub * 32;
                     const uint32_t ts = tS + (c & 1) * NC + lane_s;
-                    float a[32];
-                    tc::tmem_ld32(ts, a);
-                    uint32_t h[16];
+                    if constexpr (SPLIT) {
+                        float a[16];
+                        tc::tmem_ld_frag32(ts, a);
+                        uint32_t h[8];
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        const float4 bb = *reinterpret_cast<const float4*>(bj + i);
-                        gelu_fast_pair(a[i], a[i + 1], bb.x, bb.y);
-                        gelu_fast_pair(a[i + 2], a[i + 3], bb.z, bb.w);
-                        __nv_bfloat162 lo = __floats2bfloat162_rn(a[i], a[i + 1]);
-                        __nv_bfloat162 hi = __floats2bfloat162_rn(a[i + 2], a[i + 3]);
-                        h[i / 2] = *reinterpret_cast<uint32_t*>(&lo);
-                        h[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
+                        for (int i = 0; i < 4; i++) {
+                            const float2 bb = *reinterpret_cast<const float2*>(bj + 8 * i + 2 * (lane & 3));
+#pragma unroll
+                            for (int k = 0; k < 2; k++) {
+                                gelu_fast_pair(a[4 * i + 2 * k], a[4 * i + 2 * k + 1], bb.x, bb.y);
+                                __nv_bfloat162 p = __floats2bfloat162_rn(a[4 * i + 2 * k], a[4 * i + 2 * k + 1]);
+                                h[2 * i + k] = *reinterpret_cast<uint32_t*>(&p);
+                            }
+                        }
+                        tc::tmem_st_pack16(ts, h);
+                    } else {
+                        float a[32];
+                        tc::tmem_ld32(ts, a);
+                        uint32_t h[16];
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) {
+                            const float4 bb = *reinterpret_cast<const float4*>(bj + i);
+                            gelu_fast_pair(a[i], a[i + 1], bb.x, bb.y);
+                            gelu_fast_pair(a[i + 2], a[i + 3], bb.z, bb.w);
+                            __nv_bfloat162 lo = __floats2bfloat162_rn(a[i], a[i + 1]);
+                            __nv_bfloat162 hi = __floats2bfloat162_rn(a[i + 2], a[i + 3]);
+                            h[i / 2] = *reinterpret_cast<uint32_t*>(&lo);
+                            h[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
+                        }
+                        tc::tmem_st16(ts, h);
                     }
-                    tc::tmem_st16(ts, h);
                 }
                 warp_arrive(&h_full[c & 1]);
             }
             warp_wait(&o_full, (uint32_t)it & 1u);
+            if constexpr (SPLIT) {
+                if (norms) {
+                    const int row = m0_of(it) + tr;
+                    frag_resid(x, tO + trow + 64 * half, sv[3], at, mean, rstd);
+                    frag_ln_global(x, mean, rstd, sv[4], sv[5], half, ln, row, R);
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (row + 8 * (i & 1) < R)
+                            reinterpret_cast<float4*>(xg + (size_t)(row + 8 * (i & 1)) * D)[4 * (2 * (i >> 1) + half) + (lane & 3)] = x[i];
+                }
+                continue;
+            }
             frag_resid(x, tO + trow + 64 * half, sv[3], at, mean, rstd);
             // the LayerNorm rows go over the next tile's attention rows: its P has read them by now
             if (it + 1 < my_tiles) warp_wait(&p_full, (uint32_t)(it + 1) & 1u);
@@ -3097,7 +3153,8 @@ void BF16Path::set_kernel_attributes() {
     set_smem(tc_gemm_kernel<EPI_F32>, 200 * 1024);
     set_smem(tc_gemm_kernel<EPI_RESID_LN>, 200 * 1024);
     set_smem(tc_mlp_serial_kernel, kMlpSmemMax);
-    set_smem(tc_proj_mlp_kernel, kPMSmem);
+    set_smem(tc_proj_mlp_kernel<false>, kPMSmem);
+    set_smem(tc_proj_mlp_kernel<true>, kPMSmem);
     set_smem(tc_projln_persistent_kernel, 225 * 1024);  // 227 KB per CTA less the static shared memory
     set_smem(tc_qkv_kernel<false>, 225 * 1024);
     set_smem(tc_qkv_kernel<true>, 225 * 1024);
@@ -3209,8 +3266,15 @@ void BF16Path::launch_mlp(const Dims& d, const WeightsF32& w, int l, const Tunin
     bf16* ln = reinterpret_cast<bf16*>(p.bt[0]);
     if (m_attn) {
         if (!proj_fuses(tu)) throw Error(JC_LIMIT, "the fused projection needs dim 128 and 64-column MLP chunks");
-        cuda_check(launch_pdl(tc_proj_mlp_kernel, (unsigned)std::min((R + 127) / 128, n_sms_), kPMThreads, kPMSmem, s, 1u, *m_attn, m_ln,
-                              *m_x, pm_w_[l], pm_w_[l] + D * D, pm_w_[l] + D * D + (size_t)d.F * D, B.bp, B.n2g, B.n2b, B.b1, B.b2, ng, nbeta, d.F, R, p.x, p.err),
+        // While half of the SMs would stand idle two CTAs share a tile: 3 tiles
+        // took 16 us a launch with one CTA each and take 13, 32 tiles 16.5 and 13.5.
+        // From there on a second CTA would wait for an SM.
+        const int tiles = (R + 127) / 128;
+        const bool split = 2 * tiles <= n_sms_;
+        cuda_check(launch_pdl(split ? tc_proj_mlp_kernel<true> : tc_proj_mlp_kernel<false>,
+                              (unsigned)(split ? 2 * tiles : std::min(tiles, n_sms_)), kPMThreads, kPMSmem, s, 1u, *m_attn, m_ln,
+                              *m_x, pm_w_[l], pm_w_[l] + D * D, pm_w_[l] + D * D + (size_t)d.F * D, B.bp, B.n2g, B.n2b, B.b1, B.b2, ng,
+                              nbeta, d.F, R, p.x, ln, p.err),
                    "launch");
         return;
     }
