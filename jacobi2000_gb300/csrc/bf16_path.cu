@@ -196,55 +196,54 @@ constexpr int kCellPlane = kHaloW * kHaloH * 16;
 __device__ __forceinline__ float bf2f(bf16 v) { return __bfloat162float(v); }
 
 // Token embedding and the first LayerNorm (cpu.rs:253-280, 289). Persistent
-// CTAs walk tiles of 64 token rows: the embed weights [pd][D] are staged in
+// CTAs walk tiles of 8 RW token rows: the embed weights [pd][D] are staged in
 // shared memory once per CTA, and each tile's patches arrive as 16-byte
 // asynchronous copies (one per (row, channel, patch row): 4 cells), double-
 // buffered so the next tile's patches are in flight while this one is
 // summed. Patches sit as [channel, patch row][row][4] floats. Warp w owns
-// rows 8w..8w+7 and lane l owns the CPL = D/32 consecutive outputs
-// [CPL l, CPL l + CPL): per group of 4 patch elements it reads 8 patch
-// float4s and 4 x CPL weights and does 32 x CPL FMAs. Each output is summed in
+// RW rows from RW w and lane l owns the CPL = D/32 consecutive outputs
+// [CPL l, CPL l + CPL): per group of 4 patch elements it reads RW patch
+// float4s and 4 x CPL weights and does 4 x RW x CPL FMAs. Each output is summed in
 // the reference's order (bias, then the patch elements in order, then + pos,
 // + the meta linear); x is written f32 and LayerNorm(x) bf16, with vector
-// stores. The pos rows of a warp's 8 rows are loaded together before the
+// stores. The pos rows of a warp's rows are loaded together before the
 // LayerNorms, and the meta linear is kept while the instance stays the same
 // (across tiles too).
-constexpr int kEmbedRows = 64;
 constexpr int kEmbedGroups = 12;  // 3 channels x 4 patch rows, 4 patch columns each
 
-__host__ __device__ constexpr size_t embed_smem(int D) {
-    return ((size_t)48 * D + 2 * (size_t)kEmbedGroups * kEmbedRows * 4) * sizeof(float);
+__host__ __device__ constexpr size_t embed_smem(int D, int rows) {
+    return ((size_t)48 * D + 2 * (size_t)kEmbedGroups * rows * 4) * sizeof(float);
 }
 
-template <int CPL>
+template <int CPL, int RW>
 __global__ void __launch_bounds__(256, (CPL <= 4 ? 3 : 1)) bf_embed_kernel(Dims d, const float* __restrict__ We,
                                                        const float* __restrict__ be, const float* __restrict__ Wm,
                                                        const float* __restrict__ bm, const float* __restrict__ g,
                                                        const float* __restrict__ b, const InstDev* inst, int n_inst,
                                                        int R, float* __restrict__ x, bf16* __restrict__ ln) {
-    JC_PDL_ENTRY;
     extern __shared__ __align__(16) float esm[];
-    constexpr int D = 32 * CPL;
+    constexpr int D = 32 * CPL, kRows = 8 * RW;
     constexpr int P = 4, pd = 3 * P * P;  // 3 channels, patch 4 (checked when the path is built)
     float* sW = esm;                      // [pd][D]
-    float4* sP = reinterpret_cast<float4*>(esm + (size_t)pd * D);  // 2 x [groups][kEmbedRows] float4
-    __shared__ int rinst[2][kEmbedRows];
-    const int n_tiles = (R + kEmbedRows - 1) / kEmbedRows;
+    float4* sP = reinterpret_cast<float4*>(esm + (size_t)pd * D);  // 2 x [groups][kRows] float4
+    __shared__ int rinst[2][kRows];
+    const int n_tiles = (R + kRows - 1) / kRows;
     for (int i = threadIdx.x; i < pd * D / 4; i += blockDim.x)
         cp_async16(reinterpret_cast<float4*>(sW) + i, reinterpret_cast<const float4*>(We) + i, true);
+    JC_PDL_ENTRY;  // the weights do not wait for the previous kernel
     // the patches of tile t into buffer `buf` (and each row's instance); with
     // 256 threads, a multiple of the tile's rows, a thread copies the patches
-    // of one row (threadIdx.x % kEmbedRows), so it finds that row's instance once
-    static_assert(256 % kEmbedRows == 0, "embed copy layout");
+    // of one row (threadIdx.x % kRows), so it finds that row's instance once
+    static_assert(256 % kRows == 0, "embed copy layout");
     auto issue = [&](int t, int buf) {
-        const int i = threadIdx.x % kEmbedRows, r = t * kEmbedRows + i;
+        const int i = threadIdx.x % kRows, r = t * kRows + i;
         // a warp's rows are consecutive: the instance of its first row by a
         // warp-wide search, then at most a step or two per lane
         int ii = warp_find_last_le(n_inst, __shfl_sync(0xffffffffu, r, 0), [&](int k) { return (long long)inst[k].row0; });
         while (ii + 1 < n_inst && inst[ii + 1].row0 <= r) ii++;
         if (r >= R) ii = -1;
-        for (int e = threadIdx.x; e < kEmbedRows * kEmbedGroups; e += blockDim.x) {
-            const int gq = e / kEmbedRows;  // (channel, patch row)
+        for (int e = threadIdx.x; e < kRows * kEmbedGroups; e += blockDim.x) {
+            const int gq = e / kRows;  // (channel, patch row)
             if (gq == 0) rinst[buf][i] = ii;
             const float* src = We;
             if (ii >= 0) {
@@ -253,12 +252,12 @@ __global__ void __launch_bounds__(256, (CPL <= 4 ? 3 : 1)) bf_embed_kernel(Dims 
                 src = I.state + (size_t)c * I.nx * I.ny + ((size_t)(tk / I.tx) * P + py) * I.nx +
                       (size_t)(tk % I.tx) * P;
             }
-            cp_async16(sP + ((size_t)buf * kEmbedGroups + gq) * kEmbedRows + i, src, ii >= 0);
+            cp_async16(sP + ((size_t)buf * kEmbedGroups + gq) * kRows + i, src, ii >= 0);
         }
         cp_async_commit();
     };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = warp * 8;  // this warp's 8 rows
+    const int i0 = warp * RW;  // this warp's RW rows
     const int o0 = CPL * lane;
     int k = 0;
     int m_inst = -1;  // the instance whose meta linear m holds
@@ -273,19 +272,19 @@ __global__ void __launch_bounds__(256, (CPL <= 4 ? 3 : 1)) bf_embed_kernel(Dims 
             cp_async_wait_group<0>();
         }
         __syncthreads();
-        const int r0 = t * kEmbedRows;
+        const int r0 = t * kRows;
         if (r0 + i0 < R) {
-            float v[8][CPL];
+            float v[RW][CPL];
 #pragma unroll
-            for (int q = 0; q < 8; q++)
+            for (int q = 0; q < RW; q++)
 #pragma unroll
                 for (int c = 0; c < CPL; c++) v[q][c] = be[o0 + c];
-            const float4* pb = sP + (size_t)buf * kEmbedGroups * kEmbedRows + i0;
+            const float4* pb = sP + (size_t)buf * kEmbedGroups * kRows + i0;
 #pragma unroll 2
             for (int gq = 0; gq < kEmbedGroups; gq++) {
-                float4 p4[8];
+                float4 p4[RW];
 #pragma unroll
-                for (int q = 0; q < 8; q++) p4[q] = pb[gq * kEmbedRows + q];
+                for (int q = 0; q < RW; q++) p4[q] = pb[gq * kRows + q];
 #pragma unroll
                 for (int px = 0; px < 4; px++) {
                     const int f = gq * 4 + px;
@@ -301,7 +300,7 @@ __global__ void __launch_bounds__(256, (CPL <= 4 ? 3 : 1)) bf_embed_kernel(Dims 
                         for (int c = 0; c < CPL; c++) wv[c] = sW[f * D + o0 + c];
                     }
 #pragma unroll
-                    for (int q = 0; q < 8; q++) {
+                    for (int q = 0; q < RW; q++) {
                         const float pv = px == 0 ? p4[q].x : px == 1 ? p4[q].y : px == 2 ? p4[q].z : p4[q].w;
                         if (CPL % 2 == 0) {
 #pragma unroll
@@ -313,10 +312,10 @@ __global__ void __launch_bounds__(256, (CPL <= 4 ? 3 : 1)) bf_embed_kernel(Dims 
                     }
                 }
             }
-            // + pos for the warp's 8 rows, the loads of all rows in flight together
-            int rii[8];
+            // + pos for the warp's rows, the loads of all rows in flight together
+            int rii[RW];
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
+            for (int q = 0; q < RW; q++) {
                 const int r = r0 + i0 + q;
                 rii[q] = r < R ? rinst[buf][i0 + q] : -1;
                 if (rii[q] >= 0) {
@@ -335,7 +334,7 @@ __global__ void __launch_bounds__(256, (CPL <= 4 ? 3 : 1)) bf_embed_kernel(Dims 
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
+            for (int q = 0; q < RW; q++) {
                 const int r = r0 + i0 + q;
                 if (r >= R) continue;  // warp-uniform
                 const int ii = rii[q];
@@ -3164,14 +3163,22 @@ void BF16Path::set_kernel_attributes() {
     set_smem(bf_attn_tile_kernel<64>, 200 * 1024);
     set_smem(tc_conv3_kernel<CONV_TOKMIX>, 200 * 1024);
     set_smem(tc_mix_cells_kernel, 225 * 1024);
-    set_smem(bf_embed_kernel<1>, 100 * 1024);
-    set_smem(bf_embed_kernel<2>, 100 * 1024);
-    set_smem(bf_embed_kernel<3>, 100 * 1024);
-    set_smem(bf_embed_kernel<4>, 100 * 1024);
-    set_smem(bf_embed_kernel<5>, 100 * 1024);
-    set_smem(bf_embed_kernel<6>, 100 * 1024);
-    set_smem(bf_embed_kernel<7>, 100 * 1024);
-    set_smem(bf_embed_kernel<8>, 100 * 1024);
+    set_smem(bf_embed_kernel<1, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<1, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<2, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<2, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<3, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<3, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<4, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<4, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<5, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<5, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<6, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<6, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<7, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<7, 8>, 100 * 1024);
+    set_smem(bf_embed_kernel<8, 2>, 100 * 1024);
+    set_smem(bf_embed_kernel<8, 8>, 100 * 1024);
 }
 
 void BF16Path::arrange(DeviceArena& arena, cudaStream_t s) {
@@ -3454,21 +3461,26 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
     const Tuning tu = tuning_for(R);
     {
         KScope k("bf_embed", s);
-        const int tiles = (R + kEmbedRows - 1) / kEmbedRows;
-        const size_t smem = embed_smem(D);
-        // persistent: as many CTAs as fit on the SMs at once
-        static int occupancy[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // CTAs per SM, per D / 32
-        auto grid_for = [&](auto kernel) {
-            int& per_sm = occupancy[D / 32];
+        // persistent: as many CTAs as fit on the SMs at once. While tiles of 16 rows
+        // (two a warp) all run at once they are the shorter chain: 375 rows of 128 took
+        // 11 us with eight rows a warp and take 7, 4096 rows 11 and 9. With more rows
+        // than that eight a warp read the weights less often (four: 48 us for 64 K, 43).
+        static int occupancy[2][9] = {};  // CTAs per SM, per rows a warp and D / 32
+        auto launch = [&](auto kernel, int rw) {
+            const int rows = 8 * rw;
+            int& per_sm = occupancy[rw == 8][D / 32];
             if (per_sm == 0)
-                cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem), "occupancy");
-            return (unsigned)std::min(tiles, std::max(1, per_sm) * n_sms_);
+                cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, embed_smem(D, rows)), "occupancy");
+            const int slots = std::max(1, per_sm) * n_sms_;
+            if (rw == 2 && (R + rows - 1) / rows > slots) return false;
+            cuda_check(launch_pdl(kernel, (unsigned)std::min((R + rows - 1) / rows, slots), 256, embed_smem(D, rows), s, 1u, d,
+                                  w.embed_w, w.embed_b, w.meta_w, w.meta_b, w.blk[0].n1g, w.blk[0].n1b, p.inst, n, R, p.x, ln),
+                       "launch");
+            return true;
         };
-#define JC_EMBED(CPL)                                                                                            \
-    case CPL:                                                                                                    \
-        cuda_check(launch_pdl(bf_embed_kernel<CPL>, grid_for(bf_embed_kernel<CPL>), 256, smem, s, 1u, d, w.embed_w, \
-                              w.embed_b, w.meta_w, w.meta_b, w.blk[0].n1g, w.blk[0].n1b, p.inst, n, R, p.x, ln),     \
-                   "launch");                                                                                    \
+#define JC_EMBED(CPL)                                                              \
+    case CPL:                                                                      \
+        if (!launch(bf_embed_kernel<CPL, 2>, 2)) launch(bf_embed_kernel<CPL, 8>, 8); \
         break;
         switch (D / 32) {
             JC_EMBED(1) JC_EMBED(2) JC_EMBED(3) JC_EMBED(4) JC_EMBED(5) JC_EMBED(6) JC_EMBED(7) JC_EMBED(8)
