@@ -1445,6 +1445,157 @@ __global__ void __launch_bounds__(kMlpSerialThreads, 2) tc_mlp_serial_kernel(con
     if (warp == 0) tc::tmem_dealloc(tmem_base, ncols);
 }
 
+// The same for dims above 128 that are multiples of 64, one 128-row tile a CTA, its
+// stages on separate warps:
+//   0-15 the GELUs (16 columns of a chunk and the 32 lanes of a TMEM quarter each)
+//        and the residual + LayerNorm;
+//   16   (one lane) loads the weights, two chunks of W1 and two of W2 in flight;
+//   17   (one lane) loads A (swizzled boxes of 64 columns) and issues the MMAs.
+// Chunks of 64 hidden columns go through two TMEM accumulators: S_{j+1} runs while
+// the row warps work on S_j; h_j lies packed over S_j's own columns and is O's A
+// operand from there. The MMAs' K order is that of the kernel above. That one,
+// with one buffer of everything and CTA barriers between its steps, took 44 us
+// for 32 tiles of dim 256 with 1024 hidden columns (one tile an SM, 16 chunks in
+// a chain); this takes 27.
+constexpr int kMWRowWarps = 16, kMWThreads = (kMWRowWarps + 2) * 32, kMWNC = 64;
+__host__ __device__ constexpr size_t mlp_wide_smem(int D) { return (size_t)D * 256 + 4 * (size_t)D * kMWNC * 2; }
+static bool mlp_wide(int D, int nc) { return D > 128 && D % 64 == 0 && nc == kMWNC; }
+
+__global__ void __launch_bounds__(kMWThreads, 1) tc_mlp_wide_kernel(
+    const __grid_constant__ CUtensorMap tmA, const bf16* __restrict__ W1, const bf16* __restrict__ W2,
+    const float* __restrict__ b1, const float* __restrict__ b2, int D, int F, int R, float* __restrict__ x,
+    const float* __restrict__ g, const float* __restrict__ b, bf16* __restrict__ ln, int* err) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    constexpr int NC = kMWNC;
+    const uint32_t wb = (uint32_t)D * NC * 2;
+    uint8_t *sA = smem, *sW1 = smem + (size_t)D * 256, *sW2 = sW1 + 2 * (size_t)wb;
+    __shared__ __align__(16) float sb1[1024];
+    __shared__ uint64_t a_full, w1_full[2], w1_empty[2], w2_full[2], w2_empty[2], s_full[2], h_full[2], o_full;
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int failed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.x * 128, n = F / NC;
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&a_full, 1);
+        tc::mbar_init(&o_full, 1);
+        for (int i = 0; i < 2; i++) {
+            for (uint64_t* q : {&w1_full[i], &w1_empty[i], &w2_full[i], &w2_empty[i], &s_full[i]}) tc::mbar_init(q, 1);
+            tc::mbar_init(&h_full[i], kMWRowWarps);
+        }
+        tc::fence_barrier_init();
+        failed = 0;
+        if (tc::smem_u32(smem) & 1023u) {  // operand tiles need aligned shared memory
+            failed = 1;
+            atomicExch(err, 2);
+        }
+    }
+    for (int i = threadIdx.x; i < F; i += kMWThreads) sb1[i] = b1[i];
+    if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tO = tmem_base, tS = tmem_base + 256;  // O | S_0 | S_1
+    if (warp == kMWRowWarps) {
+        // the weights never change: their loads do not wait for the previous kernel
+        if (tc::elect_one() && !failed) {
+            bool ok = true;
+            auto put = [&](uint8_t* ring, const bf16* W, uint64_t* full, uint64_t* empty, int j) {
+                if (j >= n || !ok) return;
+                if (j >= 2) ok = tc::mbar_wait(&empty[j & 1], (uint32_t)(j / 2 - 1) & 1u, err, &failed);
+                if (!ok) return;
+                tc::mbar_expect_tx(&full[j & 1], wb);
+                tc::bulk_load(ring + (j & 1) * (size_t)wb, W + (size_t)j * D * NC, wb, &full[j & 1]);
+            };
+            put(sW1, W1, w1_full, w1_empty, 0);
+            put(sW1, W1, w1_full, w1_empty, 1);
+            for (int j = 0; j < n && ok; j++) {
+                put(sW2, W2, w2_full, w2_empty, j);
+                put(sW1, W1, w1_full, w1_empty, j + 2);
+            }
+        }
+        __syncwarp();
+        JC_PDL_ENTRY;
+    } else if (warp == kMWRowWarps + 1) {
+        JC_PDL_ENTRY;
+        if (tc::elect_one() && !failed) {
+            tc::mbar_expect_tx(&a_full, (uint32_t)D * 256);
+            for (int c = 0; c < D / 64; c++) tc::tma_load_2d(sA + c * 16384, &tmA, 64 * c, m0, &a_full);
+            const uint32_t idS = tc::idesc_bf16(128, NC), idO = tc::idesc_bf16(128, D);
+            const uint64_t dA = tc::sdesc_sw128(tc::smem_u32(sA)), dW1 = tc::sdesc(tc::smem_u32(sW1), NC * 16, 128),
+                           dW2 = tc::sdesc(tc::smem_u32(sW2), D * 16, 128);
+            auto issue_s = [&](int j) {  // S_j = A @ W1_j
+                const uint64_t w = tc::sdesc_at(dW1, (j & 1) * wb);
+                tc::tc_fence_after();
+                for (int k = 0; k < D / 16; k++)
+                    tc::mma_bf16(tS + (j & 1) * NC, tc::sdesc_at(dA, (k >> 2) * 16384 + (k & 3) * 32),
+                                 tc::sdesc_at(w, k * 2 * NC * 16), idS, k > 0 ? 1u : 0u);
+                tc::mma_commit(&s_full[j & 1]);
+                tc::mma_commit(&w1_empty[j & 1]);
+            };
+            bool ok = tc::mbar_wait(&a_full, 0, err, &failed);
+            for (int j = 0; j < 2 && j < n && ok; j++) {
+                ok = tc::mbar_wait(&w1_full[j], 0, err, &failed);
+                if (ok) issue_s(j);
+            }
+            for (int j = 0; j < n && ok; j++) {
+                const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+                ok = tc::mbar_wait(&w2_full[j & 1], ph, err, &failed) && tc::mbar_wait(&h_full[j & 1], ph, err, &failed);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint64_t w = tc::sdesc_at(dW2, (j & 1) * wb);
+#pragma unroll
+                for (int k = 0; k < NC / 16; k++)  // 16 columns of h lie packed in the first 8 of their own
+                    tc::mma_bf16_ta(tO, tS + (j & 1) * NC + 16 * k, tc::sdesc_at(w, k * 2 * D * 16), idO,
+                                    (j > 0 || k > 0) ? 1u : 0u);
+                tc::mma_commit(j == n - 1 ? &o_full : &w2_empty[j & 1]);
+                if (j + 2 < n) {  // after O_j, which reads h_j from S_j's columns
+                    ok = tc::mbar_wait(&w1_full[j & 1], ph ^ 1u, err, &failed);
+                    if (ok) issue_s(j + 2);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        JC_PDL_ENTRY;
+        const int sub = warp >> 2;
+        for (int j = 0; j < n; j++) {
+            // (after a failed wait the later ones fail at once; every warp reaches the barriers below)
+            tc::mbar_wait(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, err, &failed);
+            __syncwarp();
+            tc::tc_fence_after();
+            const uint32_t ts = lane_addr(tS + (j & 1) * NC + 16 * sub);
+            const float* bj = sb1 + j * NC + 16 * sub;
+            float a[16];
+            tc::tmem_ld16(ts, a);
+            uint32_t h[8];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                gelu_fast_pair(a[i], a[i + 1], bj[i], bj[i + 1]);
+                __nv_bfloat162 p = __floats2bfloat162_rn(a[i], a[i + 1]);
+                h[i / 2] = *reinterpret_cast<uint32_t*>(&p);
+            }
+            tc::tmem_st8(ts, h);
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&h_full[j & 1]);
+        }
+    }
+    const bool ok = __syncthreads_and(tc::mbar_wait(&o_full, 0, err, &failed) ? 1 : 0) != 0;
+    tc::tc_fence_after();
+    // every MMA is complete: reuse the operand shared memory for the f32 O tile
+    float* tile = reinterpret_cast<float*>(smem);
+    if (ok && warp < kMWRowWarps) {
+        const int sub = warp >> 2, c0 = sub * (D / 4);
+        stage_rows(lane_addr(tO), (warp & 3) * 32 + lane, D, c0, c0 + D / 4, tile);
+    }
+    __syncthreads();
+    if (ok && warp < kMWRowWarps)
+        rows_resid_ln_any<false>(tile, D, m0, R, b2, x, g, b, ln, warp, kMWRowWarps);
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+}
+
 // One decision for the `n` threads (whole warps) that meet at named barrier `bar`.
 __device__ __forceinline__ bool all_of(bool v, int bar, int n) {
     uint32_t r;
@@ -3152,6 +3303,7 @@ void BF16Path::set_kernel_attributes() {
     set_smem(tc_gemm_kernel<EPI_F32>, 200 * 1024);
     set_smem(tc_gemm_kernel<EPI_RESID_LN>, 200 * 1024);
     set_smem(tc_mlp_serial_kernel, kMlpSmemMax);
+    set_smem(tc_mlp_wide_kernel, mlp_wide_smem(256));
     set_smem(tc_proj_mlp_kernel<false>, kPMSmem);
     set_smem(tc_proj_mlp_kernel<true>, kPMSmem);
     set_smem(tc_projln_persistent_kernel, 225 * 1024);  // 227 KB per CTA less the static shared memory
@@ -3282,6 +3434,12 @@ void BF16Path::launch_mlp(const Dims& d, const WeightsF32& w, int l, const Tunin
                               (unsigned)(split ? 2 * tiles : std::min(tiles, n_sms_)), kPMThreads, kPMSmem, s, 1u, *m_attn, m_ln,
                               *m_x, pm_w_[l], pm_w_[l] + D * D, pm_w_[l] + D * D + (size_t)d.F * D, B.bp, B.n2g, B.n2b, B.b1, B.b2, ng,
                               nbeta, d.F, R, p.x, ln, p.err),
+                   "launch");
+        return;
+    }
+    if (mlp_wide(D, tu.nc)) {
+        cuda_check(launch_pdl(tc_mlp_wide_kernel, (unsigned)((R + 127) / 128), kMWThreads, mlp_wide_smem(D), s, 1u,
+                              store_map(ln, D, R, D, false), w1v[v][l], w2v[v][l], B.b1, B.b2, D, d.F, R, p.x, ng, nbeta, ln, p.err),
                    "launch");
         return;
     }

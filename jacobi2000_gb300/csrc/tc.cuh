@@ -321,6 +321,15 @@ __device__ __forceinline__ void tmem_st_pack16(uint32_t taddr, const uint32_t* r
         : "memory");
 }
 
+// 8 32-bit columns of this thread's TMEM lane, complete on return.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+        "r"(r[7]), "r"(taddr)
+        : "memory");
+}
+
 // 16 32-bit columns of this thread's TMEM lane, complete on return
 // (warp-collective).
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
