@@ -1093,7 +1093,7 @@ void projection(const Dims& d, const Pack& p, int init, cudaStream_t s) {
     // registers); the largest cluster that leaves the CTAs two to an SM, since a
     // CTA's own work is what a pass waits for.
     if (nseg <= 2 * f32k::kProjCluster && p.err) {
-        int cs = 1;
+        int cs = 2;  // never one: a launch without clusters has no peers for st.async to send to (an illegal instruction)
         while (cs < f32k::kProjCluster && ((long long)p.n_inst * cs <= 152 || nseg > 2 * cs)) cs *= 2;
         if (nseg <= cs) projection_units<1>(d, p, init, cs, (int)nseg, s);
         else projection_units<2>(d, p, init, cs, (int)nseg, s);
