@@ -23,7 +23,7 @@ def _family(dim, nx, ny, layers=1, seed=3):
 
 
 @pytest.mark.parametrize("dim,nx,ny,count", [(128, 64, 128, 40), (128, 100, 60, 28), (256, 68, 132, 20),
-                                              (128, 36, 20, 160)])
+                                              (128, 36, 20, 160), (32, 36, 20, 440), (64, 132, 68, 36)])
 def test_alone_equals_large_batch(dim, nx, ny, count):
     cfg, t, cj, raw = _family(dim, nx, ny)
     xs, meta = [random_drops(cfg, seed=k) for k in range(count)], meta_of(cfg)
