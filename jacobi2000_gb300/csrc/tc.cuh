@@ -136,10 +136,8 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* src, 
                  : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Waits until the committed bulk stores have read their shared memory (all,
-// or all but the most recent group).
+// Waits until the committed bulk stores have read their shared memory.
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 
 // Generic-proxy writes to shared memory become visible to the tensor core.
 __device__ __forceinline__ void fence_async_shared() {
@@ -289,19 +287,8 @@ __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// The store of tmem_ld_frag32's layout: 16 lanes x 32 32-bit columns, complete
-// on return.
-__device__ __forceinline__ void tmem_st_frag32(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15};\n\t"
-        "tcgen05.wait::st.sync.aligned;" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-        "r"(taddr)
-        : "memory");
-}
-
-// The same for four groups of 8 columns, group i at taddr + 16 i.
+// The store of tmem_ld_frag32's layout for four groups of 8 columns, group i at taddr + 16 i;
+// complete on return.
 __device__ __forceinline__ void tmem_st_frag8x4(uint32_t taddr, const uint32_t* r) {
 #pragma unroll
     for (int i = 0; i < 4; i++)
