@@ -465,6 +465,14 @@ jc_status jc_roundtrip_run(jc_roundtrip* r, const jc_drop* drops, int32_t n, con
  * with satisfy = 1 the barrier completes and the call returns JC_OK. */
 jc_status jc_selftest_device_wait(int32_t satisfy, uint32_t limit_us);
 
+/* The same for the projection, whose CTAs wait for one another's sums: one sum
+ * of pass 0 (mass), 1 (energies) or 2 (energies after the scale) is not sent, to
+ * every CTA or (one_peer != 0) to the one that records the instance's energy.
+ * Returns JC_DEVICE_TIMEOUT; JC_CUDA_ERROR if a CTA whose sums are not whole
+ * has stored any result; with pass = -1 everything is sent and the call
+ * returns JC_OK. */
+jc_status jc_selftest_projection_wait(int32_t pass, int32_t one_peer, uint32_t limit_us);
+
 /* Thread-local description of the last failure on this thread ("" if none). */
 const char* jc_last_error(void);
 

@@ -164,6 +164,10 @@ jc_status jc_selftest_device_wait(int32_t satisfy, uint32_t limit_us) {
     return guard([&] { jc::selftest_device_wait(satisfy, limit_us); });
 }
 
+jc_status jc_selftest_projection_wait(int32_t pass, int32_t one_peer, uint32_t limit_us) {
+    return guard([&] { jc::selftest_projection_wait(pass, one_peer, limit_us); });
+}
+
 jc_status jc_batch_create(jc_model* const* models, int32_t n_models, int32_t max_instances, int64_t max_cells,
                           jc_batch** out) {
     if (!out) return fail(JC_BAD_ARGUMENT, "out is null");

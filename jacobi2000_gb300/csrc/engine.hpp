@@ -90,6 +90,9 @@ void conv2_step(const Dims& d, const float* c1, const WeightsF32& w, const Pack&
 // Projection of every instance's state (mass, then energy, per the instance's
 // flags), f64 sums. init = 1 records mass0 and the energy of the state.
 void projection(const Dims& d, const Pack& p, int init, cudaStream_t s);
+// The same (not init, up to 8 segments) with waits of limit_ns and one total unsent in
+// pass `pass`, to all CTAs of the cluster or (one) to the first: for the self-test.
+void projection_selftest(const Dims& d, const Pack& p, int pass, int one, unsigned long long limit_ns, cudaStream_t s);
 
 // One reconstruct instance of a batch: its space-time volume X[0..H], the
 // step results F_t = step_F(X_{t-1}) (t = 1..H) and R_t = step_R(X_{t+1})

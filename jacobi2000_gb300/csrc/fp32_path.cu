@@ -788,9 +788,17 @@ __device__ __forceinline__ uint32_t peer_smem(const void* p, int rank) {
 
 constexpr int kProjUnits = kProjThreads / 32;  // units of a segment
 
-template <int NV>
+// The self-test's form (TEST) of the kernel waits for limit_ns and leaves unit 0's
+// total of pass `pass` unsent, to every CTA or (one) to the cluster's first alone.
+struct ProjTest {
+    unsigned long long limit_ns;
+    int pass, one;
+};
+
+// When a wait runs out (*err is set) the CTA stores nothing: its sums are not whole.
+template <int NV, bool TEST = false>
 __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, const InstDev* inst, ProjSlot* slots,
-                                                                        int init, int seg_cap, int* err) {
+                                                                        int init, int seg_cap, int* err, ProjTest test) {
     extern __shared__ __align__(16) float4 xch[];  // [3][16 seg_cap]: per pass, the units' totals (a.hi, a.lo, b.hi, b.lo)
     __shared__ uint64_t bar[3];
     __shared__ double segtot[NV * kProjCluster][2];
@@ -839,7 +847,8 @@ __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, 
         for (int i = 0; i < 3; i++) tc::mbar_expect_tx(&bar[i], (uint32_t)nu * 16);
     }
     // Kahan sums of term(q, k) -> (a, b) over each unit of this warp, every CTA's
-    // copy of all units' totals, then the instance totals in tot[] (thread 0)
+    // copy of all units' totals, then the instance totals in tot[] (thread 0). False,
+    // for the whole CTA alike, when the wait for the totals ran out.
     auto reduce = [&](int ps, auto&& term) {
         float4* mine = xch + (size_t)ps * seg_cap * kProjUnits;
 #pragma unroll
@@ -862,14 +871,14 @@ __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, 
             A.lo = __shfl_sync(0xffffffffu, A.lo, 0);
             B.hi = __shfl_sync(0xffffffffu, B.hi, 0);
             B.lo = __shfl_sync(0xffffffffu, B.lo, 0);
-            if (lane < cs)
+            if (lane < cs && !(TEST && ps == test.pass && u == 0 && (lane == 0 || !test.one)))
                 asm volatile(
                     "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
                         peer_smem(mine + u, lane)),
                     "f"(A.hi), "f"(A.lo), "f"(B.hi), "f"(B.lo), "r"(peer_smem(&bar[ps], lane))
                     : "memory");
         }
-        const bool ok = tc::mbar_wait(&bar[ps], 0, err, &failed);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&bar[ps], 0, err, &failed, TEST ? test.limit_ns : tc::kWaitNs));
         for (int g = warp; g < nseg && ok; g += kProjUnits) {
             const float4 t = lane < kProjUnits ? mine[g * kProjUnits + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
             const DF A = warp_sum_df(DF{t.x, t.y}), B = warp_sum_df(DF{t.z, t.w});
@@ -878,7 +887,7 @@ __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, 
                 segtot[g][1] = (double)B.hi + (double)B.lo;
             }
         }
-        __syncthreads();
+        if (!__syncthreads_and(ok)) return false;
         if (threadIdx.x == 0) {
             double t[2] = {0.0, 0.0};
             for (int g = 0; g < nseg; g++) {
@@ -888,14 +897,25 @@ __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, 
             tot[0] = t[0];
             tot[1] = t[1];
         }
+        return true;
+    };
+    // Leaving after a wait that ran out: a peer may still be sending to this CTA's
+    // shared memory, so the CTAs meet first (one that received everything may have
+    // left; it counts as arrived), and what is on its way gets 100 us to land. Without
+    // a failure nothing is on its way to a CTA that leaves: it has received every total.
+    auto give_up = [&]() {
+        cluster.sync();
+        const unsigned long long t0 = tc::globaltimer();
+        while (tc::globaltimer() - t0 < 100000ull) {
+        }
     };
     // pass 1: mass
     double M = 0.0;
-    if (init || (flags & 1u))
-        reduce(0, [&](int q, int k, float& a, float& b) {
+    if ((init || (flags & 1u)) && !reduce(0, [&](int q, int k, float& a, float& b) {
             a = H[q][k];
             b = 0.f;
-        });
+        }))
+        return give_up();
     if (threadIdx.x == 0) {
         if (init || (flags & 1u)) M = tot[0];
         bc = (flags & 1u) ? (float)(mass0 - M / (double)n) : 0.0f;
@@ -903,10 +923,11 @@ __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, 
     __syncthreads();
     // pass 2: mass shift, then potential and kinetic energy
     const float delta = bc;
-    reduce(1, [&](int q, int k, float& pot, float& kin) {
-        if (flags & 1u) H[q][k] = __fadd_rn(H[q][k], delta);
-        pk_terms(d, H[q][k], U[q][k], V[q][k], pot, kin);
-    });
+    if (!reduce(1, [&](int q, int k, float& pot, float& kin) {
+            if (flags & 1u) H[q][k] = __fadd_rn(H[q][k], delta);
+            pk_terms(d, H[q][k], U[q][k], V[q][k], pot, kin);
+        }))
+        return give_up();
     if (flags & 2u) {
         // pass 3: energy scale of (u, v), then the energy of the stored state
         double sc = 1.0;
@@ -923,15 +944,16 @@ __global__ void __launch_bounds__(kProjThreads) projection_units_kernel(Dims d, 
         }
         __syncthreads();
         const float s32 = bc;
-        reduce(2, [&](int q, int k, float& pot, float& kin) {
-            float u = __fadd_rn(__fmul_rn(U[q][k], d.norm_std[1]), d.norm_mean[1]);
-            float v = __fadd_rn(__fmul_rn(V[q][k], d.norm_std[2]), d.norm_mean[2]);
-            u = __fdiv_rn(__fsub_rn(__fmul_rn(u, s32), d.norm_mean[1]), d.norm_std[1]);
-            v = __fdiv_rn(__fsub_rn(__fmul_rn(v, s32), d.norm_mean[2]), d.norm_std[2]);
-            U[q][k] = u;
-            V[q][k] = v;
-            pk_terms(d, H[q][k], u, v, pot, kin);
-        });
+        if (!reduce(2, [&](int q, int k, float& pot, float& kin) {
+                float u = __fadd_rn(__fmul_rn(U[q][k], d.norm_std[1]), d.norm_mean[1]);
+                float v = __fadd_rn(__fmul_rn(V[q][k], d.norm_std[2]), d.norm_mean[2]);
+                u = __fdiv_rn(__fsub_rn(__fmul_rn(u, s32), d.norm_mean[1]), d.norm_std[1]);
+                v = __fdiv_rn(__fsub_rn(__fmul_rn(v, s32), d.norm_mean[2]), d.norm_std[2]);
+                U[q][k] = u;
+                V[q][k] = v;
+                pk_terms(d, H[q][k], u, v, pot, kin);
+            }))
+            return give_up();
         if (rank == 0 && threadIdx.x == 0) S.last_scale = sc;
     }
 #pragma unroll
@@ -1081,8 +1103,19 @@ template <int NV>
 static void projection_units(const Dims& d, const Pack& p, int init, int cs, int nseg, cudaStream_t s) {
     const size_t smem = (size_t)3 * nseg * f32k::kProjUnits * sizeof(float4);
     cuda_check_attr(launch_pdl(f32k::projection_units_kernel<NV>, dim3((unsigned)(p.n_inst * cs)), dim3(f32k::kProjThreads),
-                               smem, s, (unsigned)cs, d, (const InstDev*)p.inst, p.proj, init, nseg, p.err));
+                               smem, s, (unsigned)cs, d, (const InstDev*)p.inst, p.proj, init, nseg, p.err,
+                               f32k::ProjTest{}));
     check_launch("projection");
+}
+
+void projection_selftest(const Dims& d, const Pack& p, int pass, int one, unsigned long long limit_ns, cudaStream_t s) {
+    const int nseg = (int)((p.max_inst_cells + f32k::kProjSeg - 1) / f32k::kProjSeg), cs = f32k::kProjCluster;
+    if (nseg > cs) throw std::runtime_error("projection self-test: too many cells");
+    cuda_check_attr(launch_pdl(f32k::projection_units_kernel<1, true>, dim3((unsigned)(p.n_inst * cs)),
+                               dim3(f32k::kProjThreads), (size_t)3 * nseg * f32k::kProjUnits * sizeof(float4), s,
+                               (unsigned)cs, d, (const InstDev*)p.inst, p.proj, 0, nseg, p.err,
+                               f32k::ProjTest{limit_ns, pass, one}));
+    check_launch("projection self-test");
 }
 
 void projection(const Dims& d, const Pack& p, int init, cudaStream_t s) {

@@ -95,6 +95,8 @@ void check_wait_flag(int* flag, cudaStream_t s);
 // with a limit of limit_us microseconds; with satisfy = 0 nothing ever
 // arrives, so the wait gives up and the call reports JC_DEVICE_TIMEOUT.
 void selftest_device_wait(int satisfy, unsigned limit_us);
+// The projection with a sum that is never sent (selftest.cu).
+void selftest_projection_wait(int pass, int one_peer, unsigned limit_us);
 
 // Tile counts of one instance's grids.
 int cell_tiles(int nx, int ny);   // 16x16 cells
