@@ -168,7 +168,11 @@ __global__ void __launch_bounds__(32 * kSwWarps) sw_rows_kernel(SwDev p, const f
     const int lo = strip > 0 ? c0 + A : 0, hi = strip + 1 < strips ? c0 + 64 - A : nx;
     const bool s0 = x >= lo && x < hi && x < nx, s1 = x + 1 >= lo && x + 1 < hi && x + 1 < nx;
     const bool wall_l = x == 0, wall_r0 = x == nx - 1, wall_r1 = x + 1 == nx - 1;
-    const int xa = min(x, nx - 1), xb = min(x + 1, nx - 1), xv = min(x, nx - 2);
+    // Lanes past the last column copy some other column, each its own: copies of one
+    // address by many lanes are taken one after another. (86 states of 187 x 97, whose
+    // last strip has 19 columns, took 39 us a pass of two steps and 41 us of one with
+    // the last column for all of them, 25 and 14 this way.)
+    const int xa = x % nx, xb = (x + 1) % nx;  // xa is even where nx is
     const float* H = src + off;
     // rows ahead in flight, each lane's own part (nothing to wait for but its own copies)
     constexpr int kRing = 8, kAhead = 6;
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(32 * kSwWarps) sw_rows_kernel(SwDev p, const f
         for (int a = 0; a < 3; a++, q += n) {
             float2* to = &rg[r & (kRing - 1)][a][lane];
             if (vec) {
-                cp_async8(to, q + xv);
+                cp_async8(to, q + xa);
             } else {
                 cp_async4(&to->x, q + xa, true);
                 cp_async4(&to->y, q + xb, true);
