@@ -76,6 +76,9 @@ struct Pack {
     long long bc_plane[kCellBufs];  // bytes between the 8-channel planes of a plane-major cell buffer
 };
 
+// SMs of the current device.
+int sm_count();
+
 enum TickMode { kWriteIncrement = 0, kWriteNextState = 1 };
 
 // FP32 forward of every instance of `p`; writes the increment or the next

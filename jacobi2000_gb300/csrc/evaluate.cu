@@ -146,7 +146,7 @@ struct SwStage {
 // 2 STEPS that a step's result reaches on each side that is not a wall. Two
 // steps a pass halve the memory traffic of a step (24 bytes a cell); the rows
 // in registers take a third of the shared-memory tile's instructions. 96 states
-// of 256 x 256: a step took 46 us with 64 x 32 shared-memory tiles, 39 us in
+// of 256 x 256: a step takes 50 us with 64 x 32 shared-memory tiles, 39 us in
 // passes of one step and 34 us in passes of two (2.2 TB/s: what bounds it now is
 // instruction issue, 64% of the cycles; unrolled by 3, as many as the rows that
 // rotate through the registers, 570 us for 16 steps against 620 by 2).
@@ -228,35 +228,222 @@ __global__ void __launch_bounds__(32 * kSwWarps) sw_rows_kernel(SwDev p, const f
     }
 }
 
-template <int STEPS>
-static void sw_pass(const SwDev& p, const float* src, float* dst, int count, cudaStream_t s) {
-    KScope k("sw_step", s);
-    constexpr int A = 2 * STEPS;
-    const int strips = p.nx <= 64 ? 1 : (p.nx - 2 * A + (64 - 2 * A) - 1) / (64 - 2 * A);
-    // Rows of a band: a band computes about 2 A rows more than it stores, and the
-    // launch lasts as many rounds of bands as its warps fill the SMs (152, with 14
-    // or 20 warps by their registers): the height with the fewest rows in all.
-    const long long slots = 152LL * (STEPS == 2 ? 14 : 20);
-    int band_rows = p.ny;
-    long long least = -1;
-    for (int rows = 8; rows <= 256; rows += 4) {
-        const int nb = (p.ny + rows - 1) / rows, even = (p.ny + nb - 1) / nb;
-        const long long rounds = ((long long)count * strips * nb + slots - 1) / slots, cost = rounds * (even + 2 * A + 6);
-        if (least < 0 || cost < least) {
-            least = cost;
-            band_rows = even;
+constexpr int kSwTX = 64, kSwTY = 32;     // output tile
+constexpr int kSwThreads = 512;           // 4 cells per thread
+constexpr int kSwPX = kSwTX + 4, kSwPY = kSwTY + 4;  // inputs with a 2-cell apron
+constexpr int kSwNX = kSwTX + 2, kSwNY = kSwTY + 2;  // new depth with a 1-cell apron
+
+__device__ __forceinline__ float face_flux1(float ha, float hb, float qa, float qb) {
+    return __fmul_rn(__fmul_rn(__fmul_rn(0.5f, __fadd_rn(ha, hb)), 0.5f), __fadd_rn(qa, qb));
+}
+
+struct SwSmem {
+    float h[kSwPY][kSwPX + 1], u[kSwPY][kSwPX + 1], v[kSwPY][kSwPX + 1];
+    float hn[kSwNY][kSwNX + 1];
+};
+
+// One step of every state by 64 x 32 tiles in shared memory: grid (x tiles, y
+// tiles, states), the same arithmetic as SwStage's in scalar form. Its chain is
+// shorter (loads, continuity, momentum, where a warp of sw_rows_kernel walks its band
+// row after row): the faster single step of a few rows, and of launches that leave an
+// SM a tile or so; sw_plan has the rule and the times.
+__global__ void __launch_bounds__(kSwThreads)
+sw_tile_kernel(SwDev p, const float* __restrict__ src, float* __restrict__ dst) {
+    __shared__ SwSmem sm;
+    const int nx = p.nx, ny = p.ny;
+    const long long n = (long long)nx * ny;
+    const float* H = src + (long long)blockIdx.z * 3 * n;
+    const float* U = H + n;
+    const float* V = U + n;
+    const int x0 = blockIdx.x * kSwTX, y0 = blockIdx.y * kSwTY;
+    const int tid = threadIdx.x;
+    // inputs on [y0-2, y0+TY+2) x [x0-2, x0+TX+2); apron positions outside
+    // the grid hold a clamped neighbour and are never read below. Thread t
+    // keeps column t % kSwPX and walks rows t / kSwPX, + kLoadRows, ...
+    constexpr int kLoadRows = kSwThreads / kSwPX;  // 7 rows per pass
+    if (tid < kLoadRows * kSwPX) {
+        const int lx = tid % kSwPX;
+        const int gx = min(max(x0 - 2 + lx, 0), nx - 1);
+#pragma unroll
+        for (int ly = tid / kSwPX; ly < kSwPY; ly += kLoadRows) {
+            const int gy = min(max(y0 - 2 + ly, 0), ny - 1);
+            const long long o = (long long)gy * nx + gx;
+            sm.h[ly][lx] = __ldg(H + o);
+            sm.u[ly][lx] = __ldg(U + o);
+            sm.v[ly][lx] = __ldg(V + o);
         }
     }
-    const int bands = (p.ny + band_rows - 1) / band_rows;
-    const long long units = (long long)count * strips * bands;
+    __syncthreads();
+    // continuity on the tile and its 1-cell apron (cells inside the grid);
+    // thread t keeps column t % kSwNX
+    constexpr int kContRows = kSwThreads / kSwNX;  // 7 rows per pass
+    if (tid < kContRows * kSwNX) {
+        const int lx = tid % kSwNX;
+        const int gx = x0 - 1 + lx;
+        const bool xin = gx >= 0 && gx < nx;
+        const bool wl = gx == 0, wr = gx == nx - 1;
+        const int sx = lx + 1;
+        for (int ly = tid / kSwNX; ly < kSwNY; ly += kContRows) {
+            const int gy = y0 - 1 + ly;
+            if (!xin || gy < 0 || gy >= ny) continue;
+            const int sy = ly + 1;
+            const float h = sm.h[sy][sx];
+            const float fxl = wl ? 0.f : face_flux1(sm.h[sy][sx - 1], h, sm.u[sy][sx - 1], sm.u[sy][sx]);
+            const float fxr = wr ? 0.f : face_flux1(h, sm.h[sy][sx + 1], sm.u[sy][sx], sm.u[sy][sx + 1]);
+            const float fyl = gy == 0 ? 0.f : face_flux1(sm.h[sy - 1][sx], h, sm.v[sy - 1][sx], sm.v[sy][sx]);
+            const float fyr = gy == ny - 1 ? 0.f : face_flux1(h, sm.h[sy + 1][sx], sm.v[sy][sx], sm.v[sy + 1][sx]);
+            sm.hn[ly][lx] = __fsub_rn(h, __fmul_rn(p.r, __fadd_rn(__fsub_rn(fxr, fxl), __fsub_rn(fyr, fyl))));
+        }
+    }
+    __syncthreads();
+    float* D = dst + (long long)blockIdx.z * 3 * n;
+    // momentum, centred differences on the new surface (:188-232); thread t
+    // keeps column t % kSwTX and takes rows t / kSwTX, + 8, ...
+    const int tx = tid % kSwTX;
+    const int gx = x0 + tx;
+    const int sx = tx + 2, qx = tx + 1;  // in h, u, v / in hn
+    const int dxm = gx == 0 ? 0 : -1, dxp = gx == nx - 1 ? 0 : 1;
+    const float sxm = gx == 0 ? -1.f : 1.f, sxp = gx == nx - 1 ? -1.f : 1.f;
+#pragma unroll
+    for (int c = 0; c < (kSwTX * kSwTY) / kSwThreads; c++) {
+        const int ty = tid / kSwTX + c * (kSwThreads / kSwTX);
+        const int gy = y0 + ty;
+        if (gx >= nx || gy >= ny) continue;
+        const int sy = ty + 2, qy = ty + 1;
+        const int dym = gy == 0 ? 0 : -1, dyp = gy == ny - 1 ? 0 : 1;
+        const float sym = gy == 0 ? -1.f : 1.f, syp = gy == ny - 1 ? -1.f : 1.f;
+        const float hl = sm.hn[qy][qx + dxm], hr = sm.hn[qy][qx + dxp];
+        const float hd = sm.hn[qy + dym][qx], hu = sm.hn[qy + dyp][qx];
+        const float ul = __fmul_rn(sxm, sm.u[sy][sx + dxm]), ur = __fmul_rn(sxp, sm.u[sy][sx + dxp]);
+        const float ud = sm.u[sy + dym][sx], uu = sm.u[sy + dyp][sx];
+        const float vl = sm.v[sy][sx + dxm], vr = sm.v[sy][sx + dxp];
+        const float vd = __fmul_rn(sym, sm.v[sy + dym][sx]), vu = __fmul_rn(syp, sm.v[sy + dyp][sx]);
+        const float u0 = sm.u[sy][sx], v0 = sm.v[sy][sx];
+        const float dudx = __fmul_rn(__fsub_rn(ur, ul), p.inv2dx), dudy = __fmul_rn(__fsub_rn(uu, ud), p.inv2dx);
+        const float dvdx = __fmul_rn(__fsub_rn(vr, vl), p.inv2dx), dvdy = __fmul_rn(__fsub_rn(vu, vd), p.inv2dx);
+        const float dhdx = __fmul_rn(__fsub_rn(hr, hl), p.inv2dx), dhdy = __fmul_rn(__fsub_rn(hu, hd), p.inv2dx);
+        const float lap_u =
+            __fmul_rn(__fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(ul, ur), ud), uu), __fmul_rn(4.0f, u0)), p.invdx2);
+        const float lap_v =
+            __fmul_rn(__fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(vl, vr), vd), vu), __fmul_rn(4.0f, v0)), p.invdx2);
+        const float tu = __fadd_rn(
+            __fsub_rn(__fsub_rn(__fmul_rn(-u0, dudx), __fmul_rn(v0, dudy)), __fmul_rn(p.g, dhdx)),
+            __fmul_rn(p.nu, lap_u));
+        const float tv = __fadd_rn(
+            __fsub_rn(__fsub_rn(__fmul_rn(-u0, dvdx), __fmul_rn(v0, dvdy)), __fmul_rn(p.g, dhdy)),
+            __fmul_rn(p.nu, lap_v));
+        const long long o = (long long)gy * nx + gx;
+        D[o] = sm.hn[qy][qx];
+        D[n + o] = __fadd_rn(u0, __fmul_rn(p.dt, tu));
+        D[2 * n + o] = __fadd_rn(v0, __fmul_rn(p.dt, tv));
+    }
+}
+
+// How a launch of row passes cuts its states, and about how long it takes.
+struct SwCut {
+    int strips, bands, band_rows;
+    long long units;
+    double us;
+};
+
+template <int STEPS>
+static SwCut sw_cut(const SwDev& p, int count, int sms) {
+    constexpr int A = 2 * STEPS;
+    SwCut c;
+    c.strips = p.nx <= 64 ? 1 : (p.nx - 2 * A + (64 - 2 * A) - 1) / (64 - 2 * A);
+    // Rows of a band: a band computes about 2 A rows more than it stores, and the
+    // launch lasts as many rounds of bands as its warps fill the SMs: the height with
+    // the fewest rows in all, at 14 or 20 warps an SM a round. (Their registers allow 21
+    // and 25; other counts move single sizes: with 8 and two steps 96 states of 256 x 256
+    // take 57 us, not 68, but 451 of 46 x 86 take 29, not 25.)
+    const long long slots = (long long)sms * (STEPS == 2 ? 14 : 20);
+    c.band_rows = p.ny;
+    long long least = -1;
+    for (int rows = 8; rows <= 256 && rows < p.ny + 4; rows += 4) {
+        const int nb = (p.ny + rows - 1) / rows, even = (p.ny + nb - 1) / nb;
+        const long long rounds = ((long long)count * c.strips * nb + slots - 1) / slots, cost = rounds * (even + 2 * A + 6);
+        if (least < 0 || cost < least) {
+            least = cost;
+            c.band_rows = even;
+        }
+        if (rounds == 1) break;  // higher bands only last longer
+    }
+    c.bands = (p.ny + c.band_rows - 1) / c.band_rows;
+    c.units = (long long)count * c.strips * c.bands;
+    const double load = (double)c.units * (c.band_rows + (STEPS == 2 ? 9 : 4)) / sms;  // an SM's row iterations
+    c.us = STEPS == 2 ? std::max(8.3, 7.0 + 0.052 * load) : std::max(6.2, 5.0 + 0.036 * load);
+    return c;
+}
+
+template <int STEPS>
+static void sw_rows(const SwDev& p, const SwCut& c, const float* src, float* dst, cudaStream_t s) {
+    KScope k("sw_step", s);
     const int vec = p.nx % 2 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 7) == 0;
-    sw_rows_kernel<STEPS><<<(unsigned)((units + kSwWarps - 1) / kSwWarps), 32 * kSwWarps, 0, s>>>(p, src, dst, strips, bands,
-                                                                                             band_rows, units, vec);
+    sw_rows_kernel<STEPS><<<(unsigned)((c.units + kSwWarps - 1) / kSwWarps), 32 * kSwWarps, 0, s>>>(
+        p, src, dst, c.strips, c.bands, c.band_rows, c.units, vec);
     cuda_check(cudaGetLastError(), "sw_step launch");
 }
 
+static void sw_tiles(const SwDev& p, const float* src, float* dst, int count, cudaStream_t s) {
+    KScope k("sw_step", s);
+    const int gx = (p.nx + kSwTX - 1) / kSwTX, gy = (p.ny + kSwTY - 1) / kSwTY;
+    const long long stride = 3LL * p.nx * p.ny;
+    for (int c0 = 0; c0 < count; c0 += 65535) {
+        const int c = std::min(65535, count - c0);
+        sw_tile_kernel<<<dim3(gx, gy, c), kSwThreads, 0, s>>>(p, src + c0 * stride, dst + c0 * stride);
+    }
+    cuda_check(cudaGetLastError(), "sw_step launch");
+}
+
+// The schedule of a run: `twos` passes of two steps, the rest passes of one, by
+// tiles or rows, and a copy back when the number of passes is odd. By estimated times,
+// in us, fitted to launches of 8 x 8 to 2048 x 2048 cells and 1 to 10,000 states (to
+// 5-7% each, the copy to 20%):
+//   tiles  4.8 + (1.1 tiles + 1.1 full tiles' worth of cells) / SMs, at least 6.1;
+//          4.1 for one wave of up to 14 rows
+//   rows   sw_cut's
+//   copy   4.1 + 0.31 a MB of states
+// As measured, a step by tiles, a step by rows, two steps, the copy: one state of 64 x
+// 64 6.1, 6.1, 8.2 and 4.1; 16 of 128 x 128 6.1, 8.2, 12.3 and 4.1; 48 of 97 x 255 16.4,
+// 14.3, 22.5 and 10.2; 96 of 256 x 256 50, 39, 68 and 27. Over 379 sizes and 1 to 8 and
+// 16 steps the schedule comes within 0.3% (in the mean) of the best by the measured
+// times, none is slower than tiles alone, and the mean is 0.76 of their time.
+struct SwPlan {
+    bool tiles;
+    int twos;
+    SwCut one, two;
+};
+
+static SwPlan sw_plan(const SwDev& p, int count, int steps) {
+    const int sms = sm_count();
+    const double cells = (double)p.nx * p.ny * count;
+    const double tiles = (double)((p.nx + kSwTX - 1) / kSwTX) * ((p.ny + kSwTY - 1) / kSwTY) * count;
+    const double tile_us = p.ny <= 14 && tiles <= sms ? 4.1 : std::max(6.1, 4.8 + 1.1 * (tiles + cells / (kSwTX * kSwTY)) / sms);
+    const double copy_us = 4.1 + 0.31 * 12e-6 * cells;
+    SwPlan plan{false, 0, sw_cut<1>(p, count, sms), SwCut{}};
+    if (steps > 1) plan.two = sw_cut<2>(p, count, sms);
+    // (0.95: the estimates' error; a launch has 65,535 rows of tiles at most)
+    plan.tiles = plan.one.us > 0.95 * tile_us && (p.ny + kSwTY - 1) / kSwTY <= 65535;
+    const double one_us = plan.tiles ? tile_us : plan.one.us;
+    double least = -1.0;
+    // linear in `twos` but for the copy: the best is at one of the ends or next to it
+    for (int twos : {0, 1, steps / 2 - 1, steps / 2}) {
+        if (twos < 0 || twos > steps / 2) continue;
+        const double us = twos * plan.two.us + (steps - 2.0 * twos) * one_us + ((steps - twos) % 2 ? copy_us : 0.0);
+        if (least < 0.0 || us < least) {
+            least = us;
+            plan.twos = twos;
+        }
+    }
+    return plan;
+}
+
+// One step, src to dst.
 void sw_step(const SwDev& p, const float* src, float* dst, int count, cudaStream_t s) {
-    if (count > 0) sw_pass<1>(p, src, dst, count, s);
+    if (count <= 0) return;
+    const SwPlan plan = sw_plan(p, count, 1);
+    if (plan.tiles) sw_tiles(p, src, dst, count, s);
+    else sw_rows<1>(p, plan.one, src, dst, s);
 }
 
 void check_params(const jc_sw_params& p) {
@@ -272,15 +459,11 @@ void check_params(const jc_sw_params& p) {
 void sw_run(const SwDev& d, float* states, float* scratch, int count, int steps, cudaStream_t s) {
     float* a = states;
     float* b = scratch;
-    // passes of two steps, and an even number of passes where that can be (the
-    // result is then in place: a copy costs more than a pass of one step)
-    int passes = (steps + 1) / 2;
-    if (passes % 2 && steps > 1) passes++;
-    for (int left = steps; left > 0; passes--) {
-        const bool two = left > passes;
-        if (two) sw_pass<2>(d, a, b, count, s);
-        else sw_pass<1>(d, a, b, count, s);
-        left -= two ? 2 : 1;
+    const SwPlan plan = sw_plan(d, count, steps);
+    for (int k = 0; k < steps - plan.twos; k++) {
+        if (k < plan.twos) sw_rows<2>(d, plan.two, a, b, s);
+        else if (plan.tiles) sw_tiles(d, a, b, count, s);
+        else sw_rows<1>(d, plan.one, a, b, s);
         std::swap(a, b);
     }
     if (a != states)

@@ -87,6 +87,16 @@ static void set_smem_per_device(K kernel, int bytes, std::atomic<unsigned long l
     done.fetch_or(bit);
 }
 
+int sm_count() {
+    static std::atomic<int> known[64];  // by device
+    int dev = 0, n = 0;
+    cuda_check_attr(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && (n = known[dev].load()) > 0) return n;
+    cuda_check_attr(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    if (dev >= 0 && dev < 64) known[dev].store(n);
+    return n;
+}
+
 static void check_launch(const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
