@@ -465,6 +465,12 @@ jc_status jc_roundtrip_run(jc_roundtrip* r, const jc_drop* drops, int32_t n, con
  * with satisfy = 1 the barrier completes and the call returns JC_OK. */
 jc_status jc_selftest_device_wait(int32_t satisfy, uint32_t limit_us);
 
+/* The wait runs out on m's own error flag and stream, as it would in a kernel of
+ * jc_forward_device or jc_rollout_device. The call itself returns JC_OK at once;
+ * m's next call that reads results on the host returns JC_DEVICE_TIMEOUT and
+ * clears the flag. */
+jc_status jc_selftest_model_wait(jc_model* m, uint32_t limit_us);
+
 /* The same for the projection, whose CTAs wait for one another's sums: one sum
  * of pass 0 (mass), 1 (energies) or 2 (energies after the scale) is not sent, to
  * every CTA or (one_peer != 0) to the one that records the instance's energy.

@@ -164,6 +164,11 @@ jc_status jc_selftest_device_wait(int32_t satisfy, uint32_t limit_us) {
     return guard([&] { jc::selftest_device_wait(satisfy, limit_us); });
 }
 
+jc_status jc_selftest_model_wait(jc_model* m, uint32_t limit_us) {
+    if (!m) return fail(JC_BAD_ARGUMENT, "model is null");
+    return guard([&] { jc::selftest_model_wait(*m->m, limit_us); });
+}
+
 jc_status jc_selftest_projection_wait(int32_t pass, int32_t one_peer, uint32_t limit_us) {
     return guard([&] { jc::selftest_projection_wait(pass, one_peer, limit_us); });
 }

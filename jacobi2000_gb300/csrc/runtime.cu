@@ -677,12 +677,14 @@ void Model::finish_init() {
     d_inc_ = arena.alloc_n<float>(state_len);
     cuda_check(cudaMallocHost(&h_pinned_, (2 * state_len + 128) * sizeof(float)), "cudaMallocHost", JC_OVER_BUDGET);
     // host calls: their own descriptor (never rewritten), input (state | meta) and
-    // output (state | wait flag) buffers, one copy each way
+    // output (state | wait flag) buffers, one copy each way. The flag is the
+    // workspace's too, so that a host call also reports a wait that ran out in a
+    // device call before it, which reads nothing back.
     d_host_in_ = arena.alloc_n<float>(state_len + 64);
     d_host_out_ = arena.alloc_n<float>(state_len + 64);
+    ws_.base.err = pack_.err = reinterpret_cast<int*>(d_host_out_ + state_len);
     host_pack_ = pack_;
     host_pack_.inst = arena.alloc_n<InstDev>(1);
-    host_pack_.err = reinterpret_cast<int*>(d_host_out_ + state_len);
     InstDev hi = inst_;
     hi.state = d_host_in_;
     hi.out = d_host_out_;

@@ -95,6 +95,9 @@ void check_wait_flag(int* flag, cudaStream_t s);
 // with a limit of limit_us microseconds; with satisfy = 0 nothing ever
 // arrives, so the wait gives up and the call reports JC_DEVICE_TIMEOUT.
 void selftest_device_wait(int satisfy, unsigned limit_us);
+// The wait running out on a model's own flag (selftest.cu).
+class Model;
+void selftest_model_wait(Model& m, unsigned limit_us);
 // The projection with a sum that is never sent (selftest.cu).
 void selftest_projection_wait(int pass, int one_peer, unsigned limit_us);
 
@@ -145,6 +148,8 @@ class Model {
 
     // Forward of every instance of a pack with this model's weights.
     void forward_pack(const Pack& p, int mode, cudaStream_t s) const;
+    // The device flag that a kernel of this model sets when a wait runs out.
+    int* wait_flag() const { return pack_.err; }
 
    private:
     std::vector<uint64_t> slot_off_;  // weight slots' offsets into the device image

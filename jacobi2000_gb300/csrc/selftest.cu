@@ -46,6 +46,14 @@ void selftest_device_wait(int satisfy, unsigned limit_us) {
     check_wait_flag(flag, nullptr);
 }
 
+// The same wait running out in a device call of `m`, as far as the model can tell: it
+// sets the model's flag, on the model's stream, and nothing is read back.
+void selftest_model_wait(Model& m, unsigned limit_us) {
+    if (limit_us < 1 || limit_us > 2000000u) throw Error(JC_BAD_ARGUMENT, "limit_us must be in [1, 2000000]");
+    wait_selftest_kernel<<<1, 64, 0, m.stream>>>(0, (unsigned long long)limit_us * 1000ull, m.wait_flag());
+    cuda_check(cudaGetLastError(), "wait self-test launch");
+}
+
 // The projection of one 100 x 60 state by a cluster of eight CTAs, one unit's total
 // of pass `pass` unsent (to the cluster's first CTA alone when one_peer). CTAs whose
 // sums are not whole must store nothing: that is all of them, or in the last pass the

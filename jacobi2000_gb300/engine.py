@@ -276,7 +276,8 @@ def _declare_batch(L):
 
 
 EXPORTED += ["jc_batch_create", "jc_batch_destroy", "jc_batch_rollout", "jc_batch_profile",
-             "jc_forward_device_noalloc", "jc_selftest_device_wait", "jc_selftest_projection_wait"]
+             "jc_forward_device_noalloc", "jc_selftest_device_wait", "jc_selftest_model_wait",
+             "jc_selftest_projection_wait"]
 
 
 class Batch:
