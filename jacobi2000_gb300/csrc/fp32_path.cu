@@ -1005,22 +1005,28 @@ static void gemm_tile(const char* name, const AL& a, const float* W, const float
     check_launch(name);
 }
 
-// The tile by the CTAs it gives: the smallest tiles while they find an SM each
-// (152), the middle ones while there are at most four to an SM, then the large
-// ones. Back to back launches, us (32x16 | 32x32 | 64x32 tiles): R = 256, N =
-// 128, K = 512: 5.0 | 6.9 | 9.7; R = 1024, the same: 6.9 | 7.0 | 9.9; R = 2048,
-// N = 512, K = 128: 10.7 | 9.8 | 10.4; R = 160 K, N = 128, K = 512: 32x32 486,
-// 64x32 461 (45 TFLOP/s).
+// The tile by the CTAs it gives: the smallest tiles while they find an SM each, the
+// middle ones after that; the large ones for plain rows from 12 middle tiles an SM on,
+// where their fewer shared-memory reads pay. Loaders that gather (convolutions,
+// patches) are faster with the middle ones at every size measured, and take the large
+// ones only where a launch has not rows of tiles enough (65,535). us a launch between
+// events, 32x16 | 32x32 | 64x32 tiles (middle ones an SM):
+//   plain, R = 512, N = 128, K = 512 (0.4): 10.6 | 12.2 | 14.9; R = 2048, the same (1.7): 16.7 | 14.7 | 16.0;
+//     R = 8192, K = 128 (6.7): 16.4 | 14.4 | 15.8; R = 12 K, K = 512 (10): 55.7 | 49.5 | 48.6;
+//     R = 16 K (13): 70 | 60 | 56; R = 41 K (34): 164 | 137 | 125; R = 25 K, N = 512, K = 128 (81): 113 | 99 | 99
+//   3x3 convolution, R = 8192, N = 128, K = 1152 (6.7): 117 | 84 | 103; R = 41 K (34): 522 | 366 | 405;
+//     R = 131 K, N = 32, K = 324 (27): 152 | 109 | 125
+//   patches, R = 41 K, N = 128, K = 48 (34): 50 | 45 | 55
 template <class AL, class EP>
 static void gemm(const char* name, const AL& a, const float* W, const float* b, int R, int N, int K, const EP& e,
                  cudaStream_t s) {
     using namespace f32k;
     KScope k(name, s);
-    constexpr long long kSms = 152;
-    const long long rows32 = (R + 31) / 32;
-    if (rows32 * ((N + 15) / 16) <= kSms) gemm_tile<Tile<4, 1, 1, 1, 4>>(name, a, W, b, R, N, K, e, s);
-    else if (rows32 * ((N + 31) / 32) <= 4 * kSms) gemm_tile<Tile<4, 2, 1, 1, 3>>(name, a, W, b, R, N, K, e, s);
-    else gemm_tile<Tile<8, 2, 1, 1, 3>>(name, a, W, b, R, N, K, e, s);
+    const long long sms = sm_count(), rows32 = (R + 31) / 32;
+    if (rows32 * ((N + 15) / 16) <= sms) return gemm_tile<Tile<4, 1, 1, 1, 4>>(name, a, W, b, R, N, K, e, s);
+    if (rows32 > 65535 || (!AL::kCtx && rows32 * ((N + 31) / 32) > 12 * sms))
+        return gemm_tile<Tile<8, 2, 1, 1, 3>>(name, a, W, b, R, N, K, e, s);
+    gemm_tile<Tile<4, 2, 1, 1, 3>>(name, a, W, b, R, N, K, e, s);
 }
 
 static void layernorm(const char* name, const float* x, const float* g, const float* b, int R, int D, float* y,
@@ -1137,7 +1143,7 @@ void projection(const Dims& d, const Pack& p, int init, cudaStream_t s) {
     // CTA's own work is what a pass waits for.
     if (nseg <= 2 * f32k::kProjCluster && p.err) {
         int cs = 2;  // never one: a launch without clusters has no peers for st.async to send to (an illegal instruction)
-        while (cs < f32k::kProjCluster && ((long long)p.n_inst * cs <= 152 || nseg > 2 * cs)) cs *= 2;
+        while (cs < f32k::kProjCluster && ((long long)p.n_inst * cs <= sm_count() || nseg > 2 * cs)) cs *= 2;
         if (nseg <= cs) projection_units<1>(d, p, init, cs, (int)nseg, s);
         else projection_units<2>(d, p, init, cs, (int)nseg, s);
         return;
@@ -1145,11 +1151,11 @@ void projection(const Dims& d, const Pack& p, int init, cudaStream_t s) {
     static std::atomic<unsigned long long> attr{0};
     set_smem_per_device(f32k::projection_kernel, 200 * 1024, attr);
     // cluster size: the smallest whose slices fit in shared memory, and about
-    // one CTA per SM (152 here) when the instances are few; the sums do not
+    // one CTA per SM when the instances are few; the sums do not
     // depend on it (segment totals in segment order)
     int cs = 1;
     while (cs < f32k::kProjCluster && (nseg + cs - 1) / cs * f32k::kProjSeg > f32k::kProjSmemCells) cs *= 2;
-    while (cs < f32k::kProjCluster && (long long)p.n_inst * cs < 152 && nseg >= 2LL * cs) cs *= 2;
+    while (cs < f32k::kProjCluster && (long long)p.n_inst * cs < sm_count() && nseg >= 2LL * cs) cs *= 2;
     const long long seg_cap = (nseg + cs - 1) / cs;
     // staged in shared memory when a CTA's cells fit, else passes run in place
     const int cap = seg_cap * f32k::kProjSeg <= f32k::kProjSmemCells ? (int)(seg_cap * f32k::kProjSeg) : 1;
