@@ -3389,7 +3389,14 @@ static void launch_attention(const Dims& d, const bf16* qkv, const InstDev* inst
     JC_ATTN_HEAD(32)
     JC_ATTN_HEAD(64)
 #undef JC_ATTN_HEAD
-    throw Error(JC_LIMIT, "the BF16 attention supports head widths 8, 16, 32 and 64");
+}
+
+// Before anything is launched: with the other widths the dim is one that no kernel
+// here is made for (96 has 288 q/k/v columns, more than an MMA or the tensor memory takes).
+static void check_head_width(const Dims& d) {
+    const int hd = d.D / d.heads;
+    if (hd != 8 && hd != 16 && hd != 32 && hd != 64)
+        throw Error(JC_LIMIT, "the BF16 attention supports head widths 8, 16, 32 and 64");
 }
 
 static int initial_autotune() {
@@ -3478,6 +3485,7 @@ static float time_launches(F&& launch, int reps, cudaStream_t s) {
 
 void BF16Path::tune(const Dims& d, const WeightsF32& w, const Pack& p, cudaStream_t s) const {
     if (!g_autotune.load() || p.R == 0) return;
+    check_head_width(d);
     const int bucket = row_bucket(p.R);
     {
         std::lock_guard<std::mutex> lk(tune_mu_);
@@ -3614,6 +3622,7 @@ void BF16Path::prepare(const Dims& d, const Pack& p, const InstDev* hinst, cudaS
 void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mode, cudaStream_t s) const {
     const int R = p.R, D = d.D, n = p.n_inst;
     if (R == 0) return;
+    check_head_width(d);
     bf16* ln = reinterpret_cast<bf16*>(p.bt[0]);
     bf16* qkv = reinterpret_cast<bf16*>(p.bt[1]);
     bf16* attn = reinterpret_cast<bf16*>(p.bt[2]);
