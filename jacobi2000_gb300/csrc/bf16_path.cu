@@ -7,15 +7,18 @@
 //     attention (CUDA cores) stencil-masked softmax over <= (2r+1)^2 keys -> attn (bf16)
 //     proj  (tcgen05 GEMM)  x += attn @ Wp + b; LN2(x)             -> x (f32), LN2(x) (bf16)
 //     mlp   (tcgen05, fused) x += gelu(LN2(x) @ W1 + b1) @ W2 + b2; LN(x) for the next step
+//                           (at dim 128 one kernel with proj)
 //   token_mix (tcgen05 conv) t1 = xn + gelu(conv3x3(xn) + b)        (bf16)
-//   to_cells (tcgen05 GEMM) z0 = t1 @ Wtc + b                      (f32)
-//   upsample (CUDA cores)   zc = [upsample(z0), state]             (bf16, 48 channels)
-//   conv1 (tcgen05 conv)    c1 = gelu(conv3x3(zc) + b)             (bf16)
-//   conv2 + step (CUDA cores) next = state + conv3x3(c1) + b       (f32)
-// The two 3x3 convolutions are implicit GEMMs without an im2col copy: a
-// halo tile (10 x 18 positions, all channels) is loaded once by TMA in the
-// no-swizzle core-matrix layout and each of the 9 taps is the same tile
-// addressed through a shifted shared-memory descriptor.
+//   to_cells (tcgen05 GEMM) z0 = t1 @ Wtc + b                      (f32; one kernel
+//                           with token_mix at dims up to 128)
+//   upsample (CUDA cores)   zc = [upsample(z0), state]             (f16, 48 channels)
+//   conv1 (tcgen05 conv)    c1 = gelu(conv3x3(zc) + b)             (f16)
+//   conv2 + step (tcgen05 conv) next = state + conv3x3(c1) + b     (f32)
+// The 3x3 convolutions are implicit GEMMs without an im2col copy: a halo tile
+// (10 x 18 positions, all channels) is loaded once in the no-swizzle core-matrix
+// layout and each of the 9 taps is the same tile addressed through a shifted
+// shared-memory descriptor (conv2, with 3 outputs, is one GEMM over the halo whose
+// 27 columns are then added up).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -147,9 +150,7 @@ static CUtensorMap tile_store_map(const void* base, int C, int nx, int ny, bool 
 // each) and a box of a conv tile moves in a few long rows instead of one
 // 16-byte row per position. Halo loads: 10 x 18 positions of every plane
 // from element (x0 - 1) * 8 (a 16-byte boundary; the fill covers the grid's
-// edges), landing as [planes][18][10][8]; tile stores: 8 x 16 positions of
-// every plane from [planes][16][8][8] (positions outside the grid are not
-// written).
+// edges), landing as [planes][18][10][8].
 static CUtensorMap cell_plane_map(const void* base, int planes, long long plane, int nx, int ny) {
     uint64_t dims[3] = {(uint64_t)nx * 8, (uint64_t)ny, (uint64_t)planes};
     uint64_t strides[2] = {(uint64_t)nx * 16, (uint64_t)plane};
@@ -842,36 +843,16 @@ __device__ __forceinline__ uint32_t lane_addr(uint32_t tmem) {
     return tmem + (((threadIdx.x >> 5) & 3u) * 32u << 16);
 }
 
-__device__ __forceinline__ void store_bf16x16(bf16* p, const float* v) {
-    BfVec<8>::store(p, v);
-    BfVec<8>::store(p + 8, v + 8);
-}
-
-// GELU, x Phi(x) (cpu.rs:67-74), as x * sigmoid(2 u) with the odd
-// polynomial u = x (c1 + c3 x^2 + c5 x^4): the tanh form of Hendrycks &
+// GELU of v + b for two values, x Phi(x) (cpu.rs:67-74), as x * sigmoid(2 u) with
+// the odd polynomial u = x (c1 + c3 x^2 + c5 x^4): the tanh form of Hendrycks &
 // Gimpel (2016) with its coefficients refitted (minimax of the absolute GELU
 // error on |x| <= 9; |x| is clamped to 9, where Phi is 0 or 1 to f32
 // precision). Maximum absolute error 2.6e-5 against the exact erf form, far
-// below the bf16 rounding of the values it feeds. Two MUFU operations
-// (ex2, rcp) and seven FMA-pipe instructions.
-__device__ __forceinline__ float gelu_fast(float x) {
-    // coefficients of u, times -2 log2(e), so sigmoid(2u) = 1 / (1 + 2^t)
-    constexpr float k1 = -2.0f * 1.4426950408889634f * 7.97506042e-01f;
-    constexpr float k3 = -2.0f * 1.4426950408889634f * 3.70071725e-02f;
-    constexpr float k5 = -2.0f * 1.4426950408889634f * -3.51557324e-04f;
-    const float xc = fminf(fmaxf(x, -9.0f), 9.0f);
-    const float x2 = xc * xc;
-    const float t = xc * fmaf(x2, fmaf(x2, k5, k3), k1);
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return x * r;
-}
-
-// gelu_fast(v + b) of two values with the adds, multiplies and multiply-adds
-// paired (add/mul/fma.rn.f32x2: each lane is the scalar operation with the
-// same rounding), so both results are gelu_fast's bits in fewer instructions.
+// below the bf16 rounding of the values it feeds. Two MUFU operations a value
+// (ex2, rcp); the adds, multiplies and multiply-adds are paired (add/mul/fma.rn.f32x2:
+// each lane is the scalar operation with the same rounding).
 __device__ __forceinline__ void gelu_fast_pair(float& v0, float& v1, float b0, float b1) {
+    // coefficients of u, times -2 log2(e), so sigmoid(2u) = 1 / (1 + 2^t)
     constexpr float k1 = -2.0f * 1.4426950408889634f * 7.97506042e-01f;
     constexpr float k3 = -2.0f * 1.4426950408889634f * 3.70071725e-02f;
     constexpr float k5 = -2.0f * 1.4426950408889634f * -3.51557324e-04f;
@@ -1110,7 +1091,6 @@ __device__ __forceinline__ void rows_resid_ln_any(const float* tile, int D, int 
                                   const XRows* xin = nullptr) {
     if (D == 256) rows_resid_ln_t<2, true>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows);
     else if (D == 128) rows_resid_ln_t<1, true, PRE>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows, xin);
-    else if (D > 128) rows_resid_ln_t<2, false>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows);
     else rows_resid_ln_t<1, false, PRE>(tile, D, m0, R, bias, x, g, b, ln, warp, nwarps, nrows);
 }
 
@@ -1256,7 +1236,7 @@ __device__ __forceinline__ float4* xrow_chunk(uint8_t* sX, int r, int q) {
 // shared-memory reads of a pass are all in flight at once); DT = 0: D.
 template <int DT>
 __device__ void row_resid_ln_t(uint32_t ta, int r, int D_, uint8_t* sX, const float* sbias, const float* sg,
-                               const float* sb, uint8_t* sLn, bf16* lnrow) {
+                               const float* sb, bf16* lnrow) {
     const int D = DT > 0 ? DT : D_;
     // D <= 128: slot q is lane q's only slot, so lane partial q = 0 + sum4
     const int nq = D / 4;
@@ -1286,19 +1266,14 @@ __device__ void row_resid_ln_t(uint32_t ta, int r, int D_, uint8_t* sX, const fl
         float o[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) o[i] = ln1(in[i], mean, rstd, sg[c + i], sb[c + i]);
-        if (sLn) {
-            const int j = (c & 63) >> 3;
-            BfVec<8>::store(reinterpret_cast<bf16*>(sLn + (size_t)(c >> 6) * 16384 + (size_t)r * 128 + ((j ^ (r & 7)) << 4)), o);
-        } else if (lnrow) {
-            BfVec<8>::store(lnrow + c, o);
-        }
+        if (lnrow) BfVec<8>::store(lnrow + c, o);
     }
 }
 
 __device__ __forceinline__ void row_resid_ln(uint32_t ta, int r, int D, uint8_t* sX, const float* sbias,
-                                             const float* sg, const float* sb, uint8_t* sLn, bf16* lnrow) {
-    if (D == 128) row_resid_ln_t<128>(ta, r, D, sX, sbias, sg, sb, sLn, lnrow);
-    else row_resid_ln_t<0>(ta, r, D, sX, sbias, sg, sb, sLn, lnrow);
+                                             const float* sg, const float* sb, bf16* lnrow) {
+    if (D == 128) row_resid_ln_t<128>(ta, r, D, sX, sbias, sg, sb, lnrow);
+    else row_resid_ln_t<0>(ta, r, D, sX, sbias, sg, sb, lnrow);
 }
 
 constexpr int kLnMaxD = 128;  // widest row the row-per-thread LayerNorm serves
@@ -2295,7 +2270,7 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
             tc::tc_fence_after();
             const int m0 = ((int)blockIdx.x + it * (int)gridDim.x) * 128;
             const int row = m0 + r;
-            row_resid_ln(lane_addr(tmem + (uint32_t)s * D), r, D, sX + s * x_bytes, sbias, sg, sb, nullptr,
+            row_resid_ln(lane_addr(tmem + (uint32_t)s * D), r, D, sX + s * x_bytes, sbias, sg, sb,
                          row < R ? ln + (size_t)row * D : nullptr);
             tc::tc_fence_before();
             tc::mbar_arrive(&acc_empty[s]);
@@ -2324,8 +2299,12 @@ __global__ void __launch_bounds__(kPLThreads, 1) tc_projln_persistent_kernel(
 //              of two TMEM accumulators;
 //   warps 2-5  add the bias, round to bf16 into a 128-byte swizzled staging
 //              area and store it with TMA.
-// Two CTAs per SM, each with one buffer of a kind: the other CTA's work covers
-// what a CTA waits for, and few tiles still spread over three times the CTAs.
+// Two CTAs per SM, each with one buffer of rows and one of staged output: the other
+// CTA's work covers what a CTA waits for, and few tiles still spread over three times
+// the CTAs. (At dim 64, one N block of 192 columns, a CTA's two accumulators take all of
+// an SM's tensor memory: the second CTA waits in its allocation until the first has
+// walked its tiles. With one CTA per SM instead a launch of 1024 tiles alone takes 21 us,
+// not 23, but a tick of 64 x 128 x 128 cells, 2 layers, 592 us and not 584.)
 // SW (D a multiple of 64): the rows arrive as 128-byte swizzled boxes of 64
 // columns, not as 16-byte columns (2048 pieces a tile, which the TMA unit took
 // longer over than the rest of the tile). At 64 K rows: 19 us a launch with all
@@ -2477,37 +2456,33 @@ __global__ void __launch_bounds__(kQKVPThreads, 2) tc_qkv_kernel(
 // offset (ky*10 + kx)*16 bytes. B per tap: [C/8][BN][8] (the N block `nb`).
 // Epilogue (token_mix): out = xn + gelu(acc + b) (cpu.rs:326-328), bf16. The
 // cell-head convolutions have their own persistent kernel (tc_cellconv_kernel).
-enum { CONV_TOKMIX = 0 };
 
-// Shared memory of tc_conv3_kernel: the halo planes, then NS tap weight
-// blocks; with NS = 9 every tap is resident and loaded once.
-static __host__ __device__ size_t conv3_smem(int C, int BN, int NS) {
-    return (size_t)(C / 8) * kHaloPlane + (size_t)NS * C * BN * 2;
+// Shared memory of tc_conv3_kernel: the halo planes, then the weight blocks of
+// the taps in flight.
+constexpr int kConvTaps = 2;
+static __host__ __device__ size_t conv3_smem(int C, int BN) {
+    return (size_t)(C / 8) * kHaloPlane + (size_t)kConvTaps * C * BN * 2;
 }
-// Where the epilogue stages its output boxes: after the halo (1024-aligned,
-// for the 128-byte swizzle) when the halo is still read (token mix), else at
-// the start.
-static __host__ __device__ size_t conv3_stage_offset(int C, bool after_halo) {
-    return after_halo ? ((size_t)(C / 8) * kHaloPlane + 1023) / 1024 * 1024 : 0;
+// Where the epilogue stages its output boxes: after the halo, which it still
+// reads (1024-aligned, for the 128-byte swizzle).
+static __host__ __device__ size_t conv3_stage_offset(int C) {
+    return ((size_t)(C / 8) * kHaloPlane + 1023) / 1024 * 1024;
 }
 // Dynamic shared memory of a launch: operands, or the staged output boxes
-// (128 bytes of channels each, eb bytes per element) if those need more.
-static size_t conv3_launch_smem(int C, int BN, int NS, int eb) {
-    const size_t boxes = (size_t)((BN * eb + 127) / 128);
-    return std::max(conv3_smem(C, BN, NS), conv3_stage_offset(C, eb == 2) + boxes * 16384);
+// (64 channels each) if those need more.
+static size_t conv3_launch_smem(int C, int BN) {
+    return std::max(conv3_smem(C, BN), conv3_stage_offset(C) + (size_t)((BN + 63) / 64) * 16384);
 }
 
-template <int KIND>
 __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __restrict__ maps, int map_slot,
                                                        int store_slot, const bf16* __restrict__ Wt,
-                                                       const float* __restrict__ bias, int C, int BN, int NS,
+                                                       const float* __restrict__ bias, int C, int BN,
                                                        const InstDev* inst, int n_inst, int* err) {
-    static_assert(KIND == CONV_TOKMIX, "token_mix only");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sHalo = smem;                                   // [C/8][18][10][8]
     uint8_t* sB = smem + (size_t)(C / 8) * kHaloPlane;       // NS x [C/8][BN][8]
-    constexpr int kMaxNS = 9;
-    __shared__ uint64_t bar_h, bar_b[kMaxNS], bar_m[kMaxNS], bar_done;
+    constexpr int NS = kConvTaps;
+    __shared__ uint64_t bar_h, bar_b[NS], bar_m[NS], bar_done;
     __shared__ __align__(16) float sbias[256];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
@@ -2528,13 +2503,13 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
     if (threadIdx.x == 0) {
         tc::mbar_init(&bar_h, 1);
         tc::mbar_init(&bar_done, 1);
-        for (int i = 0; i < kMaxNS; i++) {
+        for (int i = 0; i < NS; i++) {
             tc::mbar_init(&bar_b[i], 1);
             tc::mbar_init(&bar_m[i], 1);
         }
         tc::fence_barrier_init();
         failed = 0;
-        if ((tc::smem_u32(smem) & 1023u) || NS < 2 || NS > kMaxNS) {  // aligned operand tiles
+        if (tc::smem_u32(smem) & 1023u) {  // aligned operand tiles
             failed = 1;
             atomicExch(err, 2);
         }
@@ -2554,7 +2529,7 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
         tc::mbar_expect_tx(&bar_h, (uint32_t)(C / 8) * (kHaloW * kHaloH * 16));
         for (int kc = 0; kc < C / 8; kc++)
             tc::tma_load_3d(sHalo + kc * kHaloPlane, map, kc * 8, x0 - 1, y0 - 1, &bar_h);
-        for (int t = 0; t < NS && t < 9; t++) {
+        for (int t = 0; t < NS; t++) {
             tc::mbar_expect_tx(&bar_b[t], wtap);
             tc::bulk_load(sB + t * wtap, Wn + (size_t)t * C * BN, wtap, &bar_b[t]);
         }
@@ -2594,7 +2569,7 @@ __global__ void __launch_bounds__(128) tc_conv3_kernel(const CUtensorMap* __rest
         constexpr int EB = 2;        // bytes per output element (bf16)
         constexpr int PB = 128 / EB;  // elements per box row
         // the epilogue still reads the halo centre, so it stages after the halo
-        uint8_t* stage = smem + conv3_stage_offset(C, true);
+        uint8_t* stage = smem + conv3_stage_offset(C);
         for (int c = 0; c < BN; c += 16) {
             float a[16];
             tc::tmem_ld16(ta + c, a);
@@ -3322,7 +3297,7 @@ void BF16Path::set_kernel_attributes() {
     set_smem(tc_cellconv_kernel<kCellConv2>, 200 * 1024);
     set_smem(bf_attn_tile_kernel<32>, 200 * 1024);
     set_smem(bf_attn_tile_kernel<64>, 200 * 1024);
-    set_smem(tc_conv3_kernel<CONV_TOKMIX>, 200 * 1024);
+    set_smem(tc_conv3_kernel, 200 * 1024);
     set_smem(tc_mix_cells_kernel, 225 * 1024);
     set_smem(bf_embed_kernel<1, 2>, 100 * 1024);
     set_smem(bf_embed_kernel<1, 8>, 100 * 1024);
@@ -3441,9 +3416,9 @@ void BF16Path::launch_mlp(const Dims& d, const WeightsF32& w, int l, const Tunin
     bf16* ln = reinterpret_cast<bf16*>(p.bt[0]);
     if (m_attn) {
         if (!proj_fuses(tu)) throw Error(JC_LIMIT, "the fused projection needs dim 128 and 64-column MLP chunks");
-        // While half of the SMs would stand idle two CTAs share a tile: 3 tiles
-        // took 16 us a launch with one CTA each and take 13, 32 tiles 16.5 and 13.5.
-        // From there on a second CTA would wait for an SM.
+        // While half of the SMs would stand idle two CTAs share a tile (one CTA | two, us a
+        // launch between events: 8 tiles 19.2 | 15.9, 32 tiles 19.6 | 16.4, 72 tiles 19.7 |
+        // 16.3); from there on a second CTA waits for an SM (80 tiles 20.2 | 26.6).
         const int tiles = (R + 127) / 128;
         const bool split = 2 * tiles <= n_sms_;
         cuda_check(launch_pdl(split ? tc_proj_mlp_kernel<true> : tc_proj_mlp_kernel<false>,
@@ -3729,9 +3704,8 @@ void BF16Path::forward(const Dims& d, const WeightsF32& w, const Pack& p, int mo
         {
             KScope k("tc_token_mix", s);
             const int BN = bn_tm;
-            const int NS = conv3_smem(D, BN, 9) <= 100 * 1024 ? 9 : 2;
-            cuda_check(launch_pdl(tc_conv3_kernel<CONV_TOKMIX>, dim3(p.n_ttiles, D / BN), 128, conv3_launch_smem(D, BN, NS, 2), s, 1u, 
-                reinterpret_cast<const CUtensorMap*>(p.tmaps), 0, 2, wtm, w.tm_b, D, BN, NS, p.inst, n, p.err), "launch");
+            cuda_check(launch_pdl(tc_conv3_kernel, dim3(p.n_ttiles, D / BN), 128, conv3_launch_smem(D, BN), s, 1u,
+                reinterpret_cast<const CUtensorMap*>(p.tmaps), 0, 2, wtm, w.tm_b, D, BN, p.inst, n, p.err), "launch");
             check_launch("tc_token_mix");
         }
         {

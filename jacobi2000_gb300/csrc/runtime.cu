@@ -738,8 +738,9 @@ void Model::enqueue_host(int mode) {
 }
 
 // A model's first call launches its kernels one by one; the second captures
-// them as a graph, which the calls after it replay (a 32 x 32 FP32 step is 38
-// launches: 185 us one by one, 144 us replayed; capturing costs about two calls).
+// them as a graph, which the calls after it replay (a 32 x 32 FP32 step of four layers
+// is 35 launches and two copies: 185 us one by one, 144 us replayed; capturing costs
+// about two calls). The modes share the count: the first call of either is eager.
 void Model::host_call(const float* state, const float* meta, float* out, int mode) {
     if (!state || !meta || !out) throw Error(JC_BAD_ARGUMENT, "null buffer");
     std::memcpy(h_pinned_, state, state_len * 4);
